@@ -2,12 +2,12 @@
 //
 // One warp solves one N x N problem.  The reference runs the same
 // shortest-augmenting-path Kuhn-Munkres on ONE thread per problem
-// (lap_batch.py:62-165); here the N columns are spread over the 32 lanes
-// (column j lives in lane j % 32, slot j / 32) so each Dijkstra step is a
-// parallel slack update plus a warp argmin.  Every per-element float
-// operation is the reference's, in the same order, and the argmin keeps the
-// lowest column among equal slacks (the reference's strict '<' scan), so
-// the assignment and the total are bit-identical to the sequential kernel.
+// (lap_batch.py:62-165); here the N columns are spread over the 32 lanes so
+// each Dijkstra step is a parallel slack update plus a warp argmin.  Every
+// per-element float operation is the reference's, in the same order, and the
+// argmin keeps the lowest column among equal slacks (the reference's strict
+// '<' scan), so the assignment and the total are bit-identical to the
+// sequential kernel.
 #pragma once
 #include "common.cuh"
 
@@ -15,134 +15,204 @@
 // dynamic shared memory one CTA may hold on sm_100a (227 KB)
 #define PK_LAP_SMEM_MAX ((size_t)227 * 1024)
 
-// Warp-cooperative Hungarian for problem b.  u and rm are this warp's shared
-// arrays of N entries.  costfn(row, col) returns C[row][col] for this
-// problem (called for the lane's own columns only).  Returns false (and
-// leaves rm at -1 for unmatched rows) if a step finds no finite slack.
-// PREFETCH: load the next step's cost row as soon as the argmin names it,
-// before the step's dual updates, so that an L2 load latency overlaps them
-// (2048 x 100^2 from L2: 1.76 -> 1.27 ms).  Costs read from shared memory or
-// computed in registers are fetched at the start of their step instead
-// (earlier loads measured slower there).  Same operations, same results.
-template <int CPL, bool PREFETCH, typename CostFn>
-__device__ __forceinline__ bool pk_hungarian_warp(int N, float* u, int* rm, CostFn costfn)
+// Column of slot k of this lane.  VEC: four consecutive columns per lane, so a
+// row is read with one 16-byte load per four slots; otherwise column j lives in
+// lane j % 32.  Either way a lane's columns ascend with k.
+template <bool VEC>
+__device__ __forceinline__ int pk_lap_col(int lane, int k)
+{
+    return VEC ? 128 * (k >> 2) + 4 * lane + (k & 3) : lane + 32 * k;
+}
+template <bool VEC>
+__device__ __forceinline__ int pk_lap_lane(int j) { return VEC ? (j >> 2) & 31 : j & 31; }
+template <bool VEC>
+__device__ __forceinline__ int pk_lap_slot(int j) { return VEC ? ((j >> 7) << 2) | (j & 3) : j >> 5; }
+
+// Minimum of a float over the warp (redux.sync takes floats on sm_100a).
+__device__ __forceinline__ float pk_redux_min(float v)
+{
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// a[slot] of an array held in registers.
+template <int CPL, typename T>
+__device__ __forceinline__ T pk_lap_pick(const T (&a)[CPL], int slot)
+{
+    T r = a[0];
+#pragma unroll
+    for (int k = 1; k < CPL; ++k) r = slot == k ? a[k] : r;
+    return r;
+}
+
+// Reads this lane's columns of one cost row (columns beyond N are left alone).
+template <int CPL, bool VEC>
+__device__ __forceinline__ void pk_lap_row(const float* row, int N, int lane, float (&c)[CPL])
+{
+    if (VEC) {   // N is a multiple of 4 and the row 16-byte aligned
+#pragma unroll
+        for (int q = 0; q < CPL / 4; ++q)
+            if (128 * q + 4 * lane < N) {
+                const float4 v = *(const float4*)(row + 128 * q + 4 * lane);
+                c[4 * q] = v.x; c[4 * q + 1] = v.y; c[4 * q + 2] = v.z; c[4 * q + 3] = v.w;
+            }
+    } else {
+#pragma unroll
+        for (int k = 0; k < CPL; ++k)
+            if (lane + 32 * k < N) c[k] = row[lane + 32 * k];
+    }
+}
+
+// Warp-cooperative Hungarian.  rowfn(row, c) reads this lane's columns of a
+// cost row into c.  On success cm[k] is the row matched to the lane's k-th
+// column; false if a step finds no finite slack.
+//
+// One problem is a chain of dependent Dijkstra steps (about 900 at N = 100,
+// 2 000 in the slowest of 2048), so a step's latency and its instructions are
+// what it costs.  All state is in registers: the dual of a matched row lives
+// with its column (it moves when the column is rematched), the dual of row i
+// in every lane, and a column's parent is the column scanned before it, so a
+// step has no shared memory and no barrier: the slacks, two redux.sync minima
+// (the smallest slack, then the lowest column that has it together with the
+// row matched to it) and a shuffle for that row's dual.  The next row's dual
+// needs no update before it is used: its column was not yet in the tree.
+// PREFETCH: the next row is read as soon as it is known, before the dual
+// updates, which then overlap an L2 load's latency.
+template <int CPL, bool VEC, bool PREFETCH, typename RowFn>
+__device__ __forceinline__ bool pk_hungarian_warp(int N, RowFn rowfn, int (&cm)[CPL])
 {
     const int lane = threadIdx.x & 31;
-    float v[CPL], minv[CPL];
-    int p[CPL], cm[CPL];
-    unsigned used = 0;
+    float v[CPL], uc[CPL], minv[CPL], c[CPL];
+    int p[CPL];
+    unsigned invalid = 0;
 #pragma unroll
-    for (int k = 0; k < CPL; ++k) { v[k] = 0.f; cm[k] = -1; }
-    for (int r = lane; r < N; r += 32) { u[r] = 0.f; rm[r] = -1; }
-    __syncwarp();
+    for (int k = 0; k < CPL; ++k) {
+        v[k] = 0.f; uc[k] = 0.f; cm[k] = -1; c[k] = 0.f;
+        if (pk_lap_col<VEC>(lane, k) >= N) invalid |= 1u << k;
+    }
+    if (PREFETCH) rowfn(0, c);
     for (int i = 0; i < N; ++i) {
+        unsigned used = invalid;
+        float ui = 0.f, urow = 0.f;
+        int cur_row = i, cur_col = -1;
 #pragma unroll
         for (int k = 0; k < CPL; ++k) { minv[k] = 1e30f; p[k] = -1; }
-        used = 0;
-        int cur_row = i, cur_col = -1;
-        float crow[CPL];   // the lane's costs in the row this step scans
-#pragma unroll
-        for (int k = 0; k < CPL; ++k) {
-            const int j = lane + 32 * k;
-            crow[k] = (PREFETCH && j < N) ? costfn(cur_row, j) : 0.f;
-        }
-        for (int step = 0; step < N; ++step) {
-            if (!PREFETCH) {
-#pragma unroll
-                for (int k = 0; k < CPL; ++k) {
-                    const int j = lane + 32 * k;
-                    if (j < N && !((used >> k) & 1u)) crow[k] = costfn(cur_row, j);
-                }
-            }
-            const float urow = u[cur_row];
-            float lbv = 1e30f;
-            int lbj = 0x7fffffff;
+        for (;;) {   // each turn adds a column to the tree, so at most N turns
+            if (!PREFETCH) rowfn(cur_row, c);
+            // the lane's smallest slack: selects, no branches, pairs before
+            // pairs of pairs; the left one keeps a tie
+            float sl[CPL], su[CPL];
+            unsigned ss[CPL];   // column << 16 | row matched to it (0xffff: none)
 #pragma unroll
             for (int k = 0; k < CPL; ++k) {
-                const int j = lane + 32 * k;
-                if (j < N && !((used >> k) & 1u)) {
-                    float red = crow[k] - urow;
-                    red = red - v[k];
-                    if (red < minv[k]) { minv[k] = red; p[k] = cur_row; }
-                    if (minv[k] < lbv) { lbv = minv[k]; lbj = j; }
-                }
+                const bool open = !((used >> k) & 1u);
+                const float red = (c[k] - urow) - v[k];
+                const bool better = open && red < minv[k];
+                minv[k] = better ? red : minv[k];
+                p[k] = better ? cur_col : p[k];
+                sl[k] = open ? minv[k] : 1e30f;
+                su[k] = uc[k];
+                ss[k] = ((unsigned)pk_lap_col<VEC>(lane, k) << 16) | (unsigned)(cm[k] & 0xffff);
             }
-            // Warp argmin in two redux.sync steps: the smallest slack as an
-            // order-preserving unsigned key (-0 folded into +0, so equal
-            // floats give equal keys), then the lowest column among the
-            // lanes holding it.  Slacks are never NaN: a NaN cost fails the
-            // '<' above and leaves minv untouched.
-            {
-                const unsigned bits = __float_as_uint(__fadd_rn(lbv, 0.f));
-                const unsigned key = (bits & 0x80000000u) ? ~bits : (bits | 0x80000000u);
-                const unsigned kmin = __reduce_min_sync(PK_FULL_MASK, key);
-                lbj = (int)__reduce_min_sync(PK_FULL_MASK, key == kmin ? (unsigned)lbj : 0xffffffffu);
-            }
-            if (lbj == 0x7fffffff) return false;   // no finite slack: infeasible input
-            // the winning lane's own slack, bit for bit
-            const float delta = __shfl_sync(PK_FULL_MASK, lbv, lbj & 31);
-            // the row matched to the chosen column is the next step's row
-            const int owner = lbj & 31, slot = lbj >> 5;
-            int nxt = -1;
 #pragma unroll
-            for (int k = 0; k < CPL; ++k)
-                if (k == slot && lane == owner) nxt = cm[k];
-            const int next_row = __shfl_sync(PK_FULL_MASK, nxt, owner);
-            const unsigned used_next = used | (lane == owner ? 1u << slot : 0u);
-            if (PREFETCH && next_row >= 0) {
+            for (int o = 1; o < CPL; o <<= 1)
 #pragma unroll
-                for (int k = 0; k < CPL; ++k) {
-                    const int j = lane + 32 * k;
-                    if (j < N && !((used_next >> k) & 1u)) crow[k] = costfn(next_row, j);
+                for (int k = 0; k + o < CPL; k += 2 * o) {
+                    const bool right = sl[k + o] < sl[k];
+                    sl[k] = right ? sl[k + o] : sl[k];
+                    su[k] = right ? su[k + o] : su[k];
+                    ss[k] = right ? ss[k + o] : ss[k];
                 }
+            // slacks are never NaN: a NaN cost fails the '<' above and leaves minv untouched
+            const float delta = pk_redux_min(sl[0]);
+            if (!(delta < 1e30f)) return false;   // no finite slack: infeasible input
+            const unsigned sel = __reduce_min_sync(PK_FULL_MASK, sl[0] == delta ? ss[0] : 0xffffffffu);
+            cur_row = (int)(sel & 0xffffu);
+            cur_col = (int)(sel >> 16);
+            const bool free_col = cur_row == 0xffff;
+            const int owner = pk_lap_lane<VEC>(cur_col);
+            if (PREFETCH) {
+                const int nr = free_col ? i + 1 : cur_row;
+                if (nr < N) rowfn(nr, c);
             }
+            urow = __shfl_sync(PK_FULL_MASK, su[0], owner);
 #pragma unroll
             for (int k = 0; k < CPL; ++k) {
-                const int j = lane + 32 * k;
-                if (j < N) {
-                    if ((used >> k) & 1u) {
-                        u[cm[k]] += delta;
-                        v[k] -= delta;
-                    } else {
-                        minv[k] -= delta;
-                    }
-                }
+                const bool in = (used >> k) & 1u;
+                uc[k] = in ? uc[k] + delta : uc[k];
+                v[k] = in ? v[k] - delta : v[k];
+                minv[k] = in ? minv[k] : minv[k] - delta;
             }
-            __syncwarp();
-            if (lane == 0) u[i] += delta;
-            __syncwarp();
-            used = used_next;
-            cur_col = lbj;
-            cur_row = next_row;
-            if (cur_row < 0) break;
+            ui += delta;
+            if (free_col) break;
+            used |= lane == owner ? 1u << pk_lap_slot<VEC>(cur_col) : 0u;
         }
-        // flip the alternating path (lap_batch.py:157-163)
-        for (int guard = 0; cur_col >= 0 && guard <= N; ++guard) {
-            const int owner = cur_col & 31, slot = cur_col >> 5;
-            int prow = 0;
+        // flip the alternating path (lap_batch.py:157-163): every column on it
+        // takes the row (and that row's dual) of its parent column, the first
+        // one row i
+        for (int guard = 0; guard <= N; ++guard) {
+            const int owner = pk_lap_lane<VEC>(cur_col), slot = pk_lap_slot<VEC>(cur_col);
+            const int par = __shfl_sync(PK_FULL_MASK, pk_lap_pick<CPL>(p, slot), owner);
+            int row = i;
+            float du = ui;
+            if (par >= 0) {
+                const int pl = pk_lap_lane<VEC>(par), ps = pk_lap_slot<VEC>(par);
+                row = __shfl_sync(PK_FULL_MASK, pk_lap_pick<CPL>(cm, ps), pl);
+                du = __shfl_sync(PK_FULL_MASK, pk_lap_pick<CPL>(uc, ps), pl);
+            }
 #pragma unroll
             for (int k = 0; k < CPL; ++k)
-                if (k == slot && lane == owner) prow = p[k];
-            prow = __shfl_sync(PK_FULL_MASK, prow, owner);
-            const int pcol = rm[prow];
-            __syncwarp();
-#pragma unroll
-            for (int k = 0; k < CPL; ++k)
-                if (k == slot && lane == owner) cm[k] = prow;
-            if (lane == 0) rm[prow] = cur_col;
-            __syncwarp();
-            cur_col = pcol;
+                if (k == slot && lane == owner) { cm[k] = row; uc[k] = du; }
+            if (par < 0) break;
+            cur_col = par;
         }
     }
     return true;
 }
 
-// One warp per problem, PK_LAP_WARPS problems per CTA.  The minimum of one
-// CTA per SM in the launch bounds lets ptxas give every CPL the registers it
-// needs (up to 88, no spills); without it, it capped CPL = 5..7 at 64 with
-// spills and scheduled the rest tighter (2048 x 100^2: 1.28 -> 1.04 ms with
-// it, 512 x 200^2: 3.56 -> 2.55 ms).
-template <int CPL>
+// The matched costs added in row order (compute_costs, lap_batch.py:173-196):
+// every lane places its columns' costs at their rows of s (N floats of this
+// warp), and lane 0 adds them.  Returns lane 0's sum.
+template <int CPL, bool VEC, typename CostFn>
+__device__ __forceinline__ float pk_lap_total(int N, const int (&cm)[CPL], float* s, CostFn costfn)
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 0; k < CPL; ++k) {
+        const int j = pk_lap_col<VEC>(lane, k);
+        if (j < N) s[cm[k]] = costfn(cm[k], j, k);
+    }
+    __syncwarp();
+    float t = 0.f;
+    if (lane == 0)
+        for (int r = 0; r < N; ++r) t += s[r];
+    return t;
+}
+
+// Results of problem b: row matches (-1 everywhere if infeasible), total, status.
+template <int CPL, bool VEC>
+__device__ __forceinline__ void pk_lap_store(bool ok, const int (&cm)[CPL], float tot, int b, int N,
+                                             int* __restrict__ row_match, float* __restrict__ total,
+                                             int* __restrict__ status)
+{
+    const int lane = threadIdx.x & 31;
+    int* rm = row_match + (size_t)b * N;
+#pragma unroll
+    for (int k = 0; k < CPL; ++k) {
+        const int j = pk_lap_col<VEC>(lane, k);
+        if (j < N) rm[ok ? cm[k] : j] = ok ? j : -1;
+    }
+    if (lane == 0) {
+        total[b] = ok ? tot : __int_as_float(0x7fc00000);
+        if (status) status[b] = ok ? 0 : 1;
+    }
+}
+
+// One warp per problem, PK_LAP_WARPS problems per CTA, cost rows read from L2.
+// The minimum of one CTA per SM in the launch bounds lets ptxas give every CPL
+// the registers it needs.
+template <int CPL, bool VEC>
 __global__ void __launch_bounds__(32 * PK_LAP_WARPS, 1)
 pk_hungarian_kernel(const float* __restrict__ C, int B, int N, int* __restrict__ row_match,
                     float* __restrict__ total, int* __restrict__ status)
@@ -151,35 +221,23 @@ pk_hungarian_kernel(const float* __restrict__ C, int B, int N, int* __restrict__
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int b = blockIdx.x * PK_LAP_WARPS + warp;
     if (b >= B) return;
-    float* u = (float*)pk_smem + (size_t)warp * 2 * N;
-    int* rm = (int*)(u + N);
     const float* Cb = C + (size_t)b * N * N;
-    const bool ok = pk_hungarian_warp<CPL, true>(N, u, rm, [&](int r, int j) { return __ldg(Cb + (size_t)r * N + j); });
-    __syncwarp();
-    for (int r = lane; r < N; r += 32) row_match[(size_t)b * N + r] = ok ? rm[r] : -1;
-    if (lane == 0) {
-        // compute_costs (lap_batch.py:173-196): sequential float sum over rows
-        float t = 0.f;
-        if (ok) {
-            for (int r = 0; r < N; ++r) {
-                const int col = rm[r];
-                if (col >= 0 && col < N) t += __ldg(Cb + (size_t)r * N + col);
-            }
-        } else {
-            t = __int_as_float(0x7fc00000);
-        }
-        total[b] = t;
-        if (status) status[b] = ok ? 0 : 1;
-    }
+    int cm[CPL];
+    const bool ok = pk_hungarian_warp<CPL, VEC, true>(
+        N, [&](int r, float (&c)[CPL]) { pk_lap_row<CPL, VEC>(Cb + (size_t)r * N, N, lane, c); }, cm);
+    float t = 0.f;
+    if (ok)
+        t = pk_lap_total<CPL, VEC>(N, cm, (float*)pk_smem + (size_t)warp * N,
+                                   [&](int r, int j, int) { return Cb[(size_t)r * N + j]; });
+    pk_lap_store<CPL, VEC>(ok, cm, t, b, N, row_match, total, status);
 }
 
 // The same solver with the problem's N x N costs copied into shared memory
-// first.  Each Dijkstra step reads one cost row, and which row is only known
-// when the previous step ends, so every step waits a full load latency: from
-// shared memory that wait is a few tens of cycles instead of an L2 round trip.
-// One warp per CTA; the CTAs beyond those resident start as others finish,
-// which balances problems of very different step counts.
-template <int CPL>
+// first: which row a step reads is only known when the previous step ends, so
+// from L2 every step waits most of a round trip, from shared memory a few tens
+// of cycles.  One warp per CTA; the CTAs beyond those resident start as others
+// finish, which balances problems of very different step counts.
+template <int CPL, bool VEC>
 __global__ void __launch_bounds__(32)
 pk_hungarian_smem_kernel(const float* __restrict__ C, int B, int N, int* __restrict__ row_match,
                          float* __restrict__ total, int* __restrict__ status)
@@ -190,8 +248,7 @@ pk_hungarian_smem_kernel(const float* __restrict__ C, int B, int N, int* __restr
     if (b >= B) return;
     const size_t nn = (size_t)N * N;
     float* Cs = (float*)pk_smem;
-    float* u = Cs + ((nn + 3) & ~(size_t)3);
-    int* rm = (int*)(u + N);
+    float* s = Cs + ((nn + 3) & ~(size_t)3);
     const float* Cb = C + (size_t)b * nn;
     if ((((uintptr_t)Cb) & 15) == 0) {
         const size_t n4 = nn >> 2;
@@ -204,75 +261,71 @@ pk_hungarian_smem_kernel(const float* __restrict__ C, int B, int N, int* __restr
         for (size_t k = lane; k < nn; k += 32) Cs[k] = __ldg(Cb + k);
     }
     __syncwarp();
-    const bool ok = pk_hungarian_warp<CPL, false>(N, u, rm, [&](int r, int j) { return Cs[r * N + j]; });
-    __syncwarp();
-    for (int r = lane; r < N; r += 32) row_match[(size_t)b * N + r] = ok ? rm[r] : -1;
-    if (lane == 0) {
-        float t = 0.f;
-        if (ok) {
-            for (int r = 0; r < N; ++r) {
-                const int col = rm[r];
-                if (col >= 0 && col < N) t += Cs[r * N + col];
-            }
-        } else {
-            t = __int_as_float(0x7fc00000);
-        }
-        total[b] = t;
-        if (status) status[b] = ok ? 0 : 1;
-    }
+    int cm[CPL];
+    const bool ok = pk_hungarian_warp<CPL, VEC, false>(
+        N, [&](int r, float (&c)[CPL]) { pk_lap_row<CPL, VEC>(Cs + r * N, N, lane, c); }, cm);
+    float t = 0.f;
+    if (ok) t = pk_lap_total<CPL, VEC>(N, cm, s, [&](int r, int j, int) { return Cs[r * N + j]; });
+    pk_lap_store<CPL, VEC>(ok, cm, t, b, N, row_match, total, status);
 }
 
 // Shared memory of the staged solver for N: the matrix (rounded up to whole
-// float4s), u and the row matches.
+// float4s) and the matched costs.
 static size_t pk_lap_smem_bytes(int N)
 {
-    return (((size_t)N * N + 3) & ~(size_t)3) * 4 + (size_t)N * 8;
+    return (((size_t)N * N + 3) & ~(size_t)3) * 4 + (size_t)N * 4;
 }
 
-// Launches the staged solver when every problem can be resident at once
-// (staging trades concurrency for latency: with fewer problems in flight
-// than the SMs could hold from L2, the L2 form finishes first).  Returns 1
-// if launched, 0 if the L2 form should run, or a status on failure.
-template <int CPL>
-static int pk_lap_try_smem(const float* C, int B, int N, int* rm, float* tot, int* status, cudaStream_t st)
+// Problems of the staged solver that the GPU can hold at once (0: N does not fit).
+template <int CPL, bool VEC>
+static cudaError_t pk_lap_staged_slots(int N, long long* slots)
 {
+    *slots = 0;
     const size_t ssm = pk_lap_smem_bytes(N);
-    if (ssm > PK_LAP_SMEM_MAX) return 0;
-    cudaError_t err = cudaFuncSetAttribute(pk_hungarian_smem_kernel<CPL>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm);
+    if (ssm > PK_LAP_SMEM_MAX) return cudaSuccess;
     int dev = 0, sms = 0, per_sm = 0;
+    cudaError_t err = cudaFuncSetAttribute(pk_hungarian_smem_kernel<CPL, VEC>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm);
     if (err == cudaSuccess) err = cudaGetDevice(&dev);
     if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (err == cudaSuccess)
-        err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pk_hungarian_smem_kernel<CPL>, 32, ssm);
-    if (err != cudaSuccess) return pk_cuda_check(err, "pk_lap_solve occupancy");
-    if ((long long)per_sm * sms < (long long)B) return 0;
-    pk_hungarian_smem_kernel<CPL><<<B, 32, ssm, st>>>(C, B, N, rm, tot, status);
-    const int rc = pk_cuda_check(cudaGetLastError(), "pk_lap_solve launch");
-    return rc == PK_OK ? 1 : rc;
+        err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pk_hungarian_smem_kernel<CPL, VEC>, 32, ssm);
+    if (err == cudaSuccess) *slots = (long long)per_sm * sms;
+    return err;
 }
 
-static int pk_lap_dispatch(const float* C, int B, int N, int* rm, float* tot, int* status, cudaStream_t st)
+// The staged solver runs when every problem can be resident at once: staging
+// trades concurrency for latency.  100 x 100: 600 problems (740 fit) 269 us
+// staged against 322 from L2, 1000 problems 391 against 371, 2048 616 against
+// 517.
+template <int CPL, bool VEC>
+static int pk_lap_launch(const float* C, int B, int N, int* rm, float* tot, int* status, cudaStream_t st)
 {
-    const int cpl = (N + 31) / 32;
-    int staged = 0;
-    switch (cpl) {
-#define PK_L(K) case K: staged = pk_lap_try_smem<K>(C, B, N, rm, tot, status, st); break;
-        PK_L(1) PK_L(2) PK_L(3) PK_L(4) PK_L(5) PK_L(6) PK_L(7) PK_L(8)
-#undef PK_L
-        default: return pk_fail(PK_ERANGE, "pk_lap_solve: N beyond 256%s");
-    }
-    if (staged == 1) return PK_OK;
-    if (staged != 0) return staged;
-    const dim3 grid((B + PK_LAP_WARPS - 1) / PK_LAP_WARPS), block(32 * PK_LAP_WARPS);
-    const size_t smem = (size_t)PK_LAP_WARPS * 2 * N * 4;
-    switch (cpl) {
-#define PK_L(K) case K: pk_hungarian_kernel<K><<<grid, block, smem, st>>>(C, B, N, rm, tot, status); break;
-        PK_L(1) PK_L(2) PK_L(3) PK_L(4) PK_L(5) PK_L(6) PK_L(7) PK_L(8)
-#undef PK_L
-        default: return pk_fail(PK_ERANGE, "pk_lap_solve: N beyond 256%s");
+    long long slots = 0;
+    const cudaError_t err = pk_lap_staged_slots<CPL, VEC>(N, &slots);
+    if (err != cudaSuccess) return pk_cuda_check(err, "pk_lap_solve occupancy");
+    if (slots >= B) {
+        pk_hungarian_smem_kernel<CPL, VEC><<<B, 32, pk_lap_smem_bytes(N), st>>>(C, B, N, rm, tot, status);
+    } else {
+        const dim3 grid((B + PK_LAP_WARPS - 1) / PK_LAP_WARPS), block(32 * PK_LAP_WARPS);
+        pk_hungarian_kernel<CPL, VEC><<<grid, block, (size_t)PK_LAP_WARPS * N * 4, st>>>(C, B, N, rm, tot, status);
     }
     return pk_cuda_check(cudaGetLastError(), "pk_lap_solve launch");
+}
+
+// VEC needs 16-byte aligned rows; below four columns per lane its rounding up
+// to a multiple of four would idle lanes.
+static int pk_lap_dispatch(const float* C, int B, int N, int* rm, float* tot, int* status, cudaStream_t st)
+{
+    const bool vec = N > 96 && (N & 3) == 0 && (((uintptr_t)C) & 15) == 0;
+    if (vec && N <= 128) return pk_lap_launch<4, true>(C, B, N, rm, tot, status, st);
+    if (vec && N <= 256) return pk_lap_launch<8, true>(C, B, N, rm, tot, status, st);
+    switch ((N + 31) / 32) {
+#define PK_L(K) case K: return pk_lap_launch<K, false>(C, B, N, rm, tot, status, st);
+        PK_L(1) PK_L(2) PK_L(3) PK_L(4) PK_L(5) PK_L(6) PK_L(7) PK_L(8)
+#undef PK_L
+    }
+    return pk_fail(PK_ERANGE, "pk_lap_solve: N beyond 256%s");
 }
 
 extern "C" int pk_lap_solve(const float* C, int B, int N, int* row_match, float* total, int* status,
@@ -380,8 +433,7 @@ pk_diversity_lap_kernel(const float* __restrict__ pop, const float* __restrict__
     for (int k = threadIdx.x; k < 3 * n; k += blockDim.x) s_pop[k] = P[k];
     __syncthreads();
     if (warp < ntf) {
-        float* u = base + (size_t)warp * 2 * n;
-        int* rm = (int*)(u + n);
+        float* s_cost = base + (size_t)warp * n;
         // this lane's transformed reference columns
         float3 rc[CPL];
         const float* R = ref + (size_t)r * n * 3;
@@ -390,25 +442,18 @@ pk_diversity_lap_kernel(const float* __restrict__ pop, const float* __restrict__
             const int j = lane + 32 * k;
             rc[k] = j < n ? pk_div_transform(R[3 * j], R[3 * j + 1], R[3 * j + 2], warp) : make_float3(0, 0, 0);
         }
-        const bool ok = pk_hungarian_warp<CPL, false>(n, u, rm, [&](int row, int j) {
-            float3 c = rc[0];
+        int cm[CPL];
+        const bool ok = pk_hungarian_warp<CPL, false, false>(n, [&](int row, float (&c)[CPL]) {
+            const float px = s_pop[3 * row], py = s_pop[3 * row + 1], pt = s_pop[3 * row + 2];
 #pragma unroll
-            for (int k = 1; k < CPL; ++k)
-                if ((j >> 5) == k) c = rc[k];
-            return pk_div_cost(s_pop[3 * row], s_pop[3 * row + 1], s_pop[3 * row + 2], c);
-        });
-        __syncwarp();
+            for (int k = 0; k < CPL; ++k) c[k] = pk_div_cost(px, py, pt, rc[k]);
+        }, cm);
+        float t = __int_as_float(0x7fc00000);
+        if (ok)
+            t = pk_lap_total<CPL, false>(n, cm, s_cost, [&](int row, int, int k) {
+                return pk_div_cost(s_pop[3 * row], s_pop[3 * row + 1], s_pop[3 * row + 2], rc[k]);
+            });
         if (lane == 0) {
-            float t = 0.f;
-            if (ok) {
-                for (int row = 0; row < n; ++row) {
-                    const int col = rm[row];
-                    const float3 c = pk_div_transform(R[3 * col], R[3 * col + 1], R[3 * col + 2], warp);
-                    t += pk_div_cost(s_pop[3 * row], s_pop[3 * row + 1], s_pop[3 * row + 2], c);
-                }
-            } else {
-                t = __int_as_float(0x7fc00000);
-            }
             s_tot[warp] = t;
         }
     }
@@ -466,7 +511,7 @@ extern "C" int pk_diversity_matrix(const float* pop, const float* ref, int Np, i
                                      "pk_diversity_matrix memset");
     const int ntf = transform ? 8 : 1;
     const int cpl = (n + 31) / 32;
-    const size_t smem = 8 * 4 + (size_t)3 * n * 4 + (size_t)8 * 2 * n * 4;
+    const size_t smem = 8 * 4 + (size_t)3 * n * 4 + (size_t)8 * n * 4;
     cudaStream_t st = (cudaStream_t)stream;
     cudaError_t err = cudaSuccess;
     switch (cpl) {

@@ -220,3 +220,29 @@ def test_matched_crossover_generation(cuda):
     orm, _ = O.hungarian(matching_costs(x, x[partners]).cpu().numpy())
     assert np.array_equal(rm, orm)
     assert torch.isfinite(out).all() and torch.isfinite(loss).all()
+
+
+@pytest.mark.parametrize("N", [96, 97, 100, 124, 128, 132, 164, 252])
+def test_column_layouts_bitexact(cuda, N):
+    """Above 96 columns an aligned matrix whose side is a multiple of 4 is read
+    four columns per lane, any other one column per lane: both sides of that
+    rule, the tile edges at 128 and 256, equal slacks across lanes, and entries
+    that are infinite or NaN (never matched while a finite choice is left)."""
+    from packing_b200.lap_batch import solve_lap_batch
+    rng = np.random.default_rng(N)
+    C = np.concatenate([rng.random((4, N, N)), rng.integers(0, 4, size=(4, N, N)), rng.normal(size=(4, N, N)) * 1e3,
+                        rng.random((2, N, N))]).astype(np.float32)
+    C[12][rng.random((N, N)) < 0.1] = np.inf
+    C[13][rng.random((N, N)) < 0.1] = np.nan
+    orm, otot = O.hungarian(C)
+    flat = torch.empty(1 + C.size, device=cuda)
+    flat[1:] = torch.from_numpy(C).to(cuda).reshape(-1)
+    for M in (torch.from_numpy(C).to(cuda), flat[1:].view(C.shape)):
+        rm, tot = solve_lap_batch(M)
+        assert np.array_equal(rm.cpu().numpy(), orm)
+        assert np.array_equal(tot.cpu().numpy(), otot)
+    # more problems than fit shared memory at once: the L2 form, the same answers
+    k = 60 if N < 130 else 20
+    rm, tot = solve_lap_batch(torch.from_numpy(C).to(cuda).repeat(k, 1, 1))
+    assert np.array_equal(rm.cpu().numpy(), np.tile(orm, (k, 1)))
+    assert np.array_equal(tot.cpu().numpy(), np.tile(otot, k))
