@@ -136,6 +136,8 @@ SIGNATURES = {
     "pk_move_draws": [ctypes.c_uint64, ctypes.c_uint64, _I, _I, _I, _P, _P],
     "pk_lap_solve": [_P, _I, _I, _P, _P, _P, _P],
     "pk_diversity_matrix": [_P, _P, _I, _I, _I, _I, _P, _P],
+    "pk_diversity_matrix_work": [_P, _P, _I, _I, _I, _I, _P, _P, ctypes.c_size_t, _P],
+    "pk_diversity_work_floats": [_I, _I, _I, _I],
     "pk_diversity_costs": [_P, _P, _I, _I, _I, _I, _P, _P],
     "pk_diversity_shortcut": [_P, _P, _I, _I, _I, _F, _F, _I, _P, _P],
     "pk_lbfgs_phase": [_I, _I, _P, _I, _I, _I, _I, _D, _D, _D, _D, _I, _I, _P],
@@ -154,7 +156,8 @@ SIGNATURES = {
     "pk_relax_noalloc": [_P, _P, _I, _I, ctypes.POINTER(PkCostSpec), ctypes.POINTER(PkRelaxParams), _P, _P, _P, _P,
                          _P],
 }
-RESTYPES = {"pk_last_error": ctypes.c_char_p, "pk_relax_workspace_floats": ctypes.c_size_t}
+RESTYPES = {"pk_last_error": ctypes.c_char_p, "pk_relax_workspace_floats": ctypes.c_size_t,
+            "pk_diversity_work_floats": ctypes.c_size_t}
 
 
 def lib_path() -> str:

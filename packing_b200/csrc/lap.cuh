@@ -348,9 +348,11 @@ extern "C" int pk_lap_solve(const float* C, int B, int N, int* row_match, float*
 // (kaggle_support.py:2061-2071), cost sqrt(dx^2 + dy^2 + wrap(dtheta)^2)
 // (:2105-2112), one LAP per transform, minimum over transforms (:2126).
 // The reference materialises a (8 * N_pop * N_ref, N, N) tensor and calls
-// solve_lap_batch; here each CTA of 8 warps handles one (pop, ref) pair,
-// warp t solving transform t with its cost rows generated on the fly, and
-// the minimum is taken in shared memory.  No intermediate tensor.
+// solve_lap_batch; here every problem's matrix lives only while its warp solves
+// it, in shared memory or in a slab of a caller's scratch
+// (pk_diversity_matrix_work).  Without scratch (pk_diversity_matrix) a CTA of 8
+// warps handles one (pop, ref) pair, warp t solving transform t with its cost
+// rows generated in the steps that read them.
 // ---------------------------------------------------------------------------
 
 // Transformed reference pose (kaggle_support.py:2080-2099), FP32.
@@ -465,6 +467,91 @@ pk_diversity_lap_kernel(const float* __restrict__ pop, const float* __restrict__
     }
 }
 
+// One (pair, transform) problem solved by a warp from a cost matrix it generates
+// once into Cs: n^2 costs (a square root and an angle remainder each) instead of
+// a row of them in every Dijkstra step, about 9 n steps at n = 100.  The steps
+// then read finished rows, like the assignment solver's.  out holds the minimum
+// over the transforms: totals are never negative, so their bits order as
+// integers, below the NaN of an infeasible problem and the initial 0x7fffffff.
+template <int CPL, bool VEC, bool PREFETCH>
+__device__ __forceinline__ void pk_diversity_problem(const float* __restrict__ pop, const float* __restrict__ ref,
+                                                     int Nr, int n, int ntf, int prob, float* Cs, float* s,
+                                                     int* __restrict__ out)
+{
+    const int lane = threadIdx.x & 31;
+    const int pr = prob / ntf, tf = prob - pr * ntf;
+    const float* P = pop + (size_t)(pr / Nr) * n * 3;
+    const float* R = ref + (size_t)(pr % Nr) * n * 3;
+    float3 rc[CPL];   // this lane's transformed reference columns
+#pragma unroll
+    for (int k = 0; k < CPL; ++k) {
+        const int j = pk_lap_col<VEC>(lane, k);
+        rc[k] = j < n ? pk_div_transform(R[3 * j], R[3 * j + 1], R[3 * j + 2], tf) : make_float3(0, 0, 0);
+    }
+    // every lane writes, and later reads, its own columns only: no barrier
+    for (int r = 0; r < n; ++r) {
+        const float px = __ldg(P + 3 * r), py = __ldg(P + 3 * r + 1), pt = __ldg(P + 3 * r + 2);
+        float c[CPL];
+#pragma unroll
+        for (int k = 0; k < CPL; ++k) c[k] = pk_div_cost(px, py, pt, rc[k]);
+        float* row = Cs + r * n;
+#pragma unroll
+        for (int k = 0; k < CPL; k += VEC ? 4 : 1) {
+            const int j = pk_lap_col<VEC>(lane, k);
+            if (VEC) { if (j < n) *(float4*)(row + j) = make_float4(c[k], c[k + 1], c[k + 2], c[k + 3]); }
+            else if (j < n) row[j] = c[k];
+        }
+    }
+    int cm[CPL];
+    const bool ok = pk_hungarian_warp<CPL, VEC, PREFETCH>(
+        n, [&](int r, float (&c)[CPL]) { pk_lap_row<CPL, VEC>(Cs + r * n, n, lane, c); }, cm);
+    float t = __int_as_float(0x7fc00000);
+    if (ok) t = pk_lap_total<CPL, VEC>(n, cm, s, [&](int r, int j, int) { return Cs[r * n + j]; });
+    if (lane == 0) atomicMin(out + pr, __float_as_int(t));
+}
+
+// The matrix in shared memory, one problem per CTA of one warp: the lowest
+// latency, while every problem can be resident at once.
+template <int CPL, bool VEC>
+__global__ void __launch_bounds__(32)
+pk_diversity_staged_kernel(const float* __restrict__ pop, const float* __restrict__ ref, int Nr, int n, int ntf,
+                           int* __restrict__ out)
+{
+    extern __shared__ __align__(16) unsigned char pk_smem[];
+    float* Cs = (float*)pk_smem;
+    pk_diversity_problem<CPL, VEC, false>(pop, ref, Nr, n, ntf, blockIdx.x, Cs, Cs + ((n * n + 3) & ~3), out);
+}
+
+// The matrix in the warp's own slab of a caller's scratch (slab floats apart),
+// which stays in L2: many more problems in flight than shared memory holds.
+// Warps take problems from a counter, so unequal problems even out.  128 x 8
+// pairs of 100 trees: 2.11 ms with rows generated in the steps, 2.29 staged in
+// shared memory, 1.43 from the scratch (16 warps per SM; 8: 1.86, 24: 1.42).
+template <int CPL, bool VEC>
+__global__ void __launch_bounds__(32 * PK_LAP_WARPS, 1)
+pk_diversity_work_kernel(const float* __restrict__ pop, const float* __restrict__ ref, int Nr, int n, int ntf,
+                         int problems, float* work, size_t slab, int* next, int* __restrict__ out)
+{
+    extern __shared__ __align__(16) unsigned char pk_smem[];
+    const int warp = threadIdx.x >> 5;
+    float* Cs = work + ((size_t)blockIdx.x * PK_LAP_WARPS + warp) * slab;
+    float* s = (float*)pk_smem + (size_t)warp * n;
+    for (;;) {
+        int prob = (threadIdx.x & 31) == 0 ? atomicAdd(next, 1) : 0;
+        prob = __shfl_sync(PK_FULL_MASK, prob, 0);
+        if (prob >= problems) return;
+        pk_diversity_problem<CPL, VEC, true>(pop, ref, Nr, n, ntf, prob, Cs, s, out);
+        __syncwarp();
+    }
+}
+
+// out and the problem counter before a launch of the two kernels above.
+__global__ void pk_diversity_init_kernel(int* __restrict__ out, int count, int* next)
+{
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) out[k] = 0x7fffffff;
+    if (next && blockIdx.x == 0 && threadIdx.x == 0) *next = 0;
+}
+
 // Shared argument checks of the diversity entry points: sizes, the (pop, ref)
 // pair count of a one-CTA-per-pair grid (computed in 64 bits), and the
 // pointers of a launch that has work.
@@ -527,6 +614,99 @@ extern "C" int pk_diversity_matrix(const float* pop, const float* ref, int Np, i
     }
     if (err != cudaSuccess) return pk_cuda_check(err, "pk_diversity_matrix attribute");
     return pk_cuda_check(cudaGetLastError(), "pk_diversity_matrix launch");
+}
+
+// Scratch of pk_diversity_matrix_work: a header for the problem counter and one
+// matrix slab per warp.  As many warps per SM, between 16 and 32, as keep the
+// slabs within the 126 MB L2 (n <= 78: 32; 96: 20; from 108: 16), and no more
+// than there are problems.
+#define PK_DIV_HEADER 32   // floats; keeps the slabs 128-byte aligned
+static size_t pk_div_slab(int n) { return ((size_t)n * n + 31) & ~(size_t)31; }
+
+static cudaError_t pk_div_warps(int n, long long problems, long long* warps)
+{
+    int dev = 0, sms = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (err != cudaSuccess) return err;
+    long long per_sm = (long long)(126e6 / (4.0 * (double)pk_div_slab(n) * sms)) & ~3LL;
+    per_sm = per_sm < 16 ? 16 : (per_sm > 32 ? 32 : per_sm);
+    long long w = per_sm * sms;
+    if (w > problems) w = (problems + PK_LAP_WARPS - 1) / PK_LAP_WARPS * PK_LAP_WARPS;
+    *warps = w;
+    return cudaSuccess;
+}
+
+// Floats of scratch pk_diversity_matrix_work needs (0: none, or no device).
+extern "C" size_t pk_diversity_work_floats(int Np, int Nr, int n, int transform)
+{
+    if (Np <= 0 || Nr <= 0 || n <= 0 || n > PK_MAX_LAP_N) return 0;
+    long long warps = 0;
+    if (pk_div_warps(n, (long long)Np * Nr * (transform ? 8 : 1), &warps) != cudaSuccess) return 0;
+    return PK_DIV_HEADER + (size_t)warps * pk_div_slab(n);
+}
+
+template <int CPL, bool VEC>
+static int pk_diversity_launch(const float* pop, const float* ref, int Np, int Nr, int n, int ntf, float* out,
+                               float* work, size_t work_floats, cudaStream_t st)
+{
+    const long long problems = (long long)Np * Nr * ntf;
+    const int pairs = Np * Nr;
+    // Shared memory when it holds every problem at once and the matrices are
+    // large: 8 pairs of 200 trees 0.95 ms against 1.44 from the scratch, but
+    // 64 problems of 100 trees 0.25 against 0.23.
+    cudaError_t err = cudaSuccess;
+    long long slots = 0;
+    const size_t ssm = pk_lap_smem_bytes(n);
+    if (n > 128 && ssm <= PK_LAP_SMEM_MAX) {
+        int dev = 0, sms = 0, per_sm = 0;
+        err = cudaFuncSetAttribute(pk_diversity_staged_kernel<CPL, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)ssm);
+        if (err == cudaSuccess) err = cudaGetDevice(&dev);
+        if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (err == cudaSuccess)
+            err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pk_diversity_staged_kernel<CPL, VEC>, 32, ssm);
+        slots = (long long)per_sm * sms;
+    }
+    long long warps = 0;
+    if (err == cudaSuccess && slots < problems) err = pk_div_warps(n, problems, &warps);
+    if (err != cudaSuccess) return pk_cuda_check(err, "pk_diversity_matrix_work occupancy");
+    const size_t slab = pk_div_slab(n);
+    if (slots < problems && work_floats < PK_DIV_HEADER + (size_t)warps * slab)
+        return pk_fail(PK_EINVAL, "pk_diversity_matrix_work: work holds fewer floats than pk_diversity_work_floats%s");
+    int* next = slots < problems ? (int*)work : nullptr;
+    pk_diversity_init_kernel<<<(pairs + 255) / 256 < 592 ? (pairs + 255) / 256 : 592, 256, 0, st>>>((int*)out, pairs,
+                                                                                                    next);
+    if (slots >= problems)
+        pk_diversity_staged_kernel<CPL, VEC><<<(int)problems, 32, ssm, st>>>(pop, ref, Nr, n, ntf, (int*)out);
+    else
+        pk_diversity_work_kernel<CPL, VEC><<<(int)(warps / PK_LAP_WARPS), 32 * PK_LAP_WARPS,
+                                             (size_t)PK_LAP_WARPS * n * 4, st>>>(
+            pop, ref, Nr, n, ntf, (int)problems, work + PK_DIV_HEADER, slab, next, (int*)out);
+    return pk_cuda_check(cudaGetLastError(), "pk_diversity_matrix_work launch");
+}
+
+extern "C" int pk_diversity_matrix_work(const float* pop, const float* ref, int Np, int Nr, int n, int transform,
+                                        float* out, float* work, size_t work_floats, void* stream)
+{
+    int rc = pk_diversity_args("pk_diversity_matrix_work", pop, ref, Np, Nr, n, out);
+    if (rc) return rc;
+    if (n > PK_MAX_LAP_N) return pk_fail(PK_ERANGE, "pk_diversity_matrix_work: more than 256 trees%s");
+    const int ntf = transform ? 8 : 1;
+    cudaStream_t st = (cudaStream_t)stream;
+    // a 31-bit problem counter; beyond it (and for empty packings) the form without scratch
+    if (Np == 0 || Nr == 0 || n == 0 || (long long)Np * Nr * ntf > 0x7fff0000LL)
+        return pk_diversity_matrix(pop, ref, Np, Nr, n, transform, out, stream);
+    if (!work || ((uintptr_t)work & 127)) return pk_fail(PK_EINVAL, "pk_diversity_matrix_work: work must be 128-byte aligned%s");
+    if (n > 96 && (n & 3) == 0)
+        return n <= 128 ? pk_diversity_launch<4, true>(pop, ref, Np, Nr, n, ntf, out, work, work_floats, st)
+                        : pk_diversity_launch<8, true>(pop, ref, Np, Nr, n, ntf, out, work, work_floats, st);
+    switch ((n + 31) / 32) {
+#define PK_D(K) case K: return pk_diversity_launch<K, false>(pop, ref, Np, Nr, n, ntf, out, work, work_floats, st);
+        PK_D(1) PK_D(2) PK_D(3) PK_D(4) PK_D(5) PK_D(6) PK_D(7) PK_D(8)
+#undef PK_D
+    }
+    return pk_fail(PK_ERANGE, "pk_diversity_matrix_work: more than 256 trees%s");
 }
 
 // diversity_shortcut_kernel (lap_batch.py:216-331): transform of the

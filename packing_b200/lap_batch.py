@@ -9,8 +9,9 @@ the summed row / column minima.  N <= 256 (the reference stops at 200).
 
 ``compute_diversity_shortcut_kernel`` follows ``lap_batch.py:537-607``.
 ``genetic_diversity_matrix`` is the B200 form of
-``kaggle_support.compute_genetic_diversity_matrix`` (``:2014-2129``): cost
-rows are generated inside the assignment kernel, no 5-D temporary.
+``kaggle_support.compute_genetic_diversity_matrix`` (``:2014-2129``): every
+running warp generates its problem's costs into a slab of a scratch sized by
+the GPU, no 5-D temporary.
 """
 from __future__ import annotations
 
@@ -97,9 +98,19 @@ def genetic_diversity_matrix(population_xyt, reference_xyt, transform: bool = Tr
     assert n == n2, f"Number of trees mismatch: population has {n}, reference has {n2}"
     out = torch.empty((Np, Nr), dtype=torch.float32, device=P.device)
     if Np * Nr > 0:
+        L, tf = _lib.load(), int(bool(transform))
         with torch.cuda.device(P.device):
-            rc = _lib.load().pk_diversity_matrix(_lib.ptr(P), _lib.ptr(R), Np, Nr, n, int(bool(transform)),
-                                                 _lib.ptr(out), ctypes.c_void_p(_lib.stream_handle(None, P.device)))
+            stream = ctypes.c_void_p(_lib.stream_handle(None, P.device))
+            floats = L.pk_diversity_work_floats(Np, Nr, n, tf)
+            try:
+                work = torch.empty(floats, dtype=torch.float32, device=P.device) if floats else None
+            except torch.OutOfMemoryError:
+                work = None   # no room for the cost matrices: generate their rows as they are read
+            if work is None:
+                rc = L.pk_diversity_matrix(_lib.ptr(P), _lib.ptr(R), Np, Nr, n, tf, _lib.ptr(out), stream)
+            else:
+                rc = L.pk_diversity_matrix_work(_lib.ptr(P), _lib.ptr(R), Np, Nr, n, tf, _lib.ptr(out),
+                                                _lib.ptr(work), floats, stream)
         _lib.check(rc, "genetic_diversity_matrix")
     return out
 

@@ -246,3 +246,31 @@ def test_column_layouts_bitexact(cuda, N):
     rm, tot = solve_lap_batch(torch.from_numpy(C).to(cuda).repeat(k, 1, 1))
     assert np.array_equal(rm.cpu().numpy(), np.tile(orm, (k, 1)))
     assert np.array_equal(tot.cpu().numpy(), np.tile(otot, k))
+
+
+@pytest.mark.parametrize("Np,Nr,n,transform", [(1, 1, 1, True), (3, 2, 33, False), (40, 3, 20, True), (7, 2, 96, True),
+                                               (60, 2, 100, True), (5, 2, 129, True), (2, 2, 160, False),
+                                               (20, 1, 132, True)])
+def test_diversity_forms_agree(cuda, Np, Nr, n, transform):
+    """The scratch form, the staged form (large n, few problems) and the form
+    without scratch give the same matrix bit for bit, and it is the minimum of
+    the materialised problems' totals; a NaN pose makes its pairs NaN."""
+    import ctypes
+
+    from packing_b200 import _lib
+    from packing_b200.lap_batch import genetic_diversity_cost_matrices, genetic_diversity_matrix, solve_lap_batch
+    pop = torch.from_numpy(poses(Np, n, seed=n)).to(cuda)
+    ref = torch.from_numpy(poses(Nr, n, seed=n + 1)).to(cuda)
+    if Np > 2:
+        pop[1, n // 2, 0] = float("nan")
+    D = genetic_diversity_matrix(pop, ref, transform)
+    plain = torch.empty_like(D)
+    rc = _lib.load().pk_diversity_matrix(_lib.ptr(pop), _lib.ptr(ref), Np, Nr, n, int(transform), _lib.ptr(plain),
+                                         ctypes.c_void_p(_lib.stream_handle(None, cuda)))
+    assert rc == 0
+    _, tot = solve_lap_batch(genetic_diversity_cost_matrices(pop, ref, transform))
+    want = tot.reshape(-1, Np, Nr).amin(0)
+    for got in (D, plain):
+        assert torch.equal(torch.isnan(got), torch.isnan(want))
+        assert torch.equal(got.nan_to_num(-1.0), want.nan_to_num(-1.0))
+    assert bool(torch.isnan(D[1]).all()) == (Np > 2) if Np > 1 else True
