@@ -36,18 +36,62 @@ __device__ __forceinline__ bool pk_pieces_overlap64(const double2 (&P)[4], bool 
     return true;
 }
 
+// Block-wide maximum of four doubles (one round trip through shared memory);
+// red needs 4 * warps doubles.  All threads get the result.
+__device__ __forceinline__ void pk_block_max4d(double (&v)[4], double* red)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[k] = fmax(v[k], __shfl_xor_sync(PK_FULL_MASK, v[k], o));
+    if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) red[4 * warp + k] = v[k];
+    __syncthreads();
+    for (int w = 0; w < nw; ++w)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = fmax(v[k], red[4 * w + k]);
+}
+
+// Shared memory of the validator: near pairs (an index into which, with two
+// piece numbers, is an item: 12 + 2 + 2 bits) and the items of T near pairs.
+#define PK_VAL_NEAR 4096
+static size_t pk_validate_smem(int n, int T)
+{
+    return (size_t)n * (32 + 64 + 8) + 32 * 8 + 16 + (size_t)PK_VAL_NEAR * 4 + (size_t)16 * T * 2;
+}
+
+// One CTA per packing.  Bound by FP64 issue in the separating-axis tests, so
+// the work before them only narrows what reaches them, in FP32 with margins
+// that never drop a pair whose exact test could say "overlap":
+//   - centres farther apart than two radii (thread per tree, offsets 1 .. n/2:
+//     no index division, conflict-free reads);
+//   - of a near pair's 16 piece pairs, those whose boxes are apart by more than
+//     the margin: some edge normal then separates the pieces by more than FP64
+//     rounding (each piece corner is wider than 30 degrees).
+// The piece pairs left over are listed and tested one per thread, so a warp's
+// lanes do the same work (one thread per near pair ran its 16 tests, each with
+// its pieces placed again, beside lanes with none).  4096 x n = 200: 0.97 ms
+// before.
 template <typename T>
-__global__ void pk_validate_kernel(const T* __restrict__ xyt, int E, int n, int* __restrict__ overlaps,
-                                   double* __restrict__ side)
+__global__ void __launch_bounds__(256, 3)
+pk_validate_kernel(const T* __restrict__ xyt, int E, int n, int* __restrict__ overlaps, double* __restrict__ side)
 {
     extern __shared__ __align__(16) unsigned char pk_smem[];
-    double4* pose = (double4*)pk_smem;            // x, y, cos, sin
-    double* red = (double*)(pose + n);            // 32
-    int* redi = (int*)(red + 32);                 // 32
+    double4* pose = (double4*)pk_smem;            // [n] x, y, cos, sin
+    float4* box = (float4*)(pose + n);            // [4][n] per piece: minx, maxx, miny, maxy about the centre
+    double* red = (double*)(box + 4 * n);         // [32]
+    int* cnt = (int*)(red + 32);                  // near pairs, items, overlapping pairs
+    uint32_t* near = (uint32_t*)(cnt + 4);        // [PK_VAL_NEAR] i | j << 11 | overlap << 31
+    float2* pos = (float2*)(near + PK_VAL_NEAR);  // [n] FP32 centres about the bounding box's corner
+    uint16_t* items = (uint16_t*)(pos + n);       // [16 * blockDim.x] near index | p << 12 | q << 14
     const int e = blockIdx.x;
     if (e >= E) return;
     const T* X = xyt + (size_t)e * n * 3;
-    double bx0 = 1e300, bx1 = -1e300, by0 = 1e300, by1 = -1e300;
+    const int lane = threadIdx.x & 31;
+    double bb[4] = {-1e300, -1e300, -1e300, -1e300};   // -min x, max x, -min y, max y
+    if (threadIdx.x < 3) cnt[threadIdx.x] = 0;
     for (int t = threadIdx.x; t < n; t += blockDim.x) {
         const double x = (double)X[3 * t], y = (double)X[3 * t + 1], th = (double)X[3 * t + 2];
         double s, c;
@@ -56,49 +100,118 @@ __global__ void pk_validate_kernel(const T* __restrict__ xyt, int E, int n, int*
         for (int v = 0; v < c_geom64.n_tree; ++v) {
             const double2 l = c_geom64.legal_tree[v];
             const double vx = c * l.x - s * l.y + x, vy = s * l.x + c * l.y + y;
-            bx0 = fmin(bx0, vx); bx1 = fmax(bx1, vx);
-            by0 = fmin(by0, vy); by1 = fmax(by1, vy);
+            bb[0] = fmax(bb[0], -vx); bb[1] = fmax(bb[1], vx);
+            bb[2] = fmax(bb[2], -vy); bb[3] = fmax(bb[3], vy);
         }
-    }
-    bx0 = -pk_block_max<double>(-bx0, red);
-    bx1 = pk_block_max<double>(bx1, red);
-    by0 = -pk_block_max<double>(-by0, red);
-    by1 = pk_block_max<double>(by1, red);
-    const double cut = 4.0 * c_geom64.legal_radius * c_geom64.legal_radius * (1.0 + 1e-12);
-    int count = 0;
-    const long long npairs = (long long)n * (n - 1) / 2;
-    for (long long k = threadIdx.x; k < npairs; k += blockDim.x) {
-        const int dd = (int)(k / n);
-        const int i = (int)(k - (long long)dd * n);
-        int j = i + dd + 1;
-        if (j >= n) j -= n;
-        const double4 A = pose[i], B = pose[j];
-        const double dx = B.x - A.x, dy = B.y - A.y;
-        if (dx * dx + dy * dy > cut) continue;
-        bool ov = false;
-        for (int p = 0; p < 4 && !ov; ++p) {
-            double2 P[4];
+        const float cf = (float)c, sf = (float)s;
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            float4 b = make_float4(1e30f, -1e30f, 1e30f, -1e30f);
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
-                const double2 l = c_geom64.legal_piece[p][v];
-                P[v] = make_double2(A.z * l.x - A.w * l.y + A.x, A.w * l.x + A.z * l.y + A.y);
+                const float lx = (float)c_geom64.legal_piece[p][v].x, ly = (float)c_geom64.legal_piece[p][v].y;
+                const float vx = cf * lx - sf * ly, vy = sf * lx + cf * ly;
+                b.x = fminf(b.x, vx); b.y = fmaxf(b.y, vx);
+                b.z = fminf(b.z, vy); b.w = fmaxf(b.w, vy);
             }
-            for (int q = 0; q < 4 && !ov; ++q) {
-                double2 Q[4];
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const double2 l = c_geom64.legal_piece[q][v];
-                    Q[v] = make_double2(B.z * l.x - B.w * l.y + B.x, B.w * l.x + B.z * l.y + B.y);
-                }
-                ov = pk_pieces_overlap64(P, c_geom64.piece_nv[p] == 3, Q, c_geom64.piece_nv[q] == 3);
+            box[p * n + t] = b;
+        }
+    }
+    pk_block_max4d(bb, red);
+    // FP32 rounding of centres and boxes is below 1e-6 of the extent
+    const double ext = fmax(fmax(fabs(bb[0]), fabs(bb[1])), fmax(fabs(bb[2]), fabs(bb[3])));
+    const float margin = (float)(1e-5 + 1e-6 * ext);
+    const float reach = 2.0f * (float)c_geom64.legal_radius + 2.0f * margin;
+    const float reach2 = reach * reach;
+    for (int t = threadIdx.x; t < n; t += blockDim.x) {
+        const double4 A = pose[t];
+        pos[t] = make_float2((float)(A.x + bb[0]), (float)(A.y + bb[2]));
+    }
+    __syncthreads();
+    const double cut = 4.0 * c_geom64.legal_radius * c_geom64.legal_radius * (1.0 + 1e-12);
+    const int half = n >> 1;
+    const int group = max(1, PK_VAL_NEAR / (2 * max(n, 1)));   // offsets between looks at the list
+    for (int d0 = 1; d0 <= half; d0 += group) {
+        const int d1 = min(half, d0 + group - 1);
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            const float2 a = pos[i];
+            for (int d = d0; d <= d1; ++d) {
+                if (2 * d == n && i >= d) break;   // the offset n / 2 meets each pair twice
+                int j = i + d;
+                if (j >= n) j -= n;
+                const float dx = pos[j].x - a.x, dy = pos[j].y - a.y;
+                if (dx * dx + dy * dy > reach2) continue;
+                near[atomicAdd(&cnt[0], 1)] = (uint32_t)i | ((uint32_t)j << 11);
             }
         }
-        count += ov ? 1 : 0;
+        __syncthreads();
+        const int cn = cnt[0];
+        __syncthreads();   // everyone has read it before anyone appends again
+        if (d1 < half && cn + group * n <= PK_VAL_NEAR) continue;   // uniform: the next group fits
+        for (int c0 = 0; c0 < cn; c0 += blockDim.x) {
+            const int w = c0 + threadIdx.x;
+            uint32_t mask = 0;
+            if (w < cn) {
+                const int i = near[w] & 2047, j = (near[w] >> 11) & 2047;
+                const double4 A = pose[i], B = pose[j];
+                const double dx = B.x - A.x, dy = B.y - A.y;
+                if (!(dx * dx + dy * dy > cut)) {
+                    const float fx = (float)dx, fy = (float)dy;
+#pragma unroll
+                    for (int p = 0; p < 4; ++p) {
+                        const float4 a = box[p * n + i];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const float4 b = box[q * n + j];
+                            const bool apart = a.y + margin < b.x + fx || b.y + fx + margin < a.x ||
+                                               a.w + margin < b.z + fy || b.w + fy + margin < a.z;
+                            mask |= (uint32_t)!apart << (4 * p + q);
+                        }
+                    }
+                }
+            }
+            const int k = __popc(mask);
+            int incl = k;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(PK_FULL_MASK, incl, o);
+                if (lane >= o) incl += u;
+            }
+            int base = 0;
+            if (lane == 31 && incl) base = atomicAdd(&cnt[1], incl);
+            int at = __shfl_sync(PK_FULL_MASK, base, 31) + incl - k;
+            while (mask) {
+                const int b = __ffs(mask) - 1;
+                mask &= mask - 1;
+                items[at++] = (uint16_t)(w | ((b >> 2) << 12) | ((b & 3) << 14));
+            }
+            __syncthreads();
+            const int ni = cnt[1];
+            for (int it = threadIdx.x; it < ni; it += blockDim.x) {
+                const int v = items[it], wn = v & (PK_VAL_NEAR - 1), p = (v >> 12) & 3, q = v >> 14;
+                const uint32_t ij = near[wn];
+                if (ij >> 31) continue;   // another piece pair of these trees has been found to overlap
+                const double4 A = pose[ij & 2047], B = pose[(ij >> 11) & 2047];
+                double2 P[4], Q[4];
+#pragma unroll
+                for (int k2 = 0; k2 < 4; ++k2) {
+                    const double2 l = c_geom64.legal_piece[p][k2], m = c_geom64.legal_piece[q][k2];
+                    P[k2] = make_double2(A.z * l.x - A.w * l.y + A.x, A.w * l.x + A.z * l.y + A.y);
+                    Q[k2] = make_double2(B.z * m.x - B.w * m.y + B.x, B.w * m.x + B.z * m.y + B.y);
+                }
+                if (pk_pieces_overlap64(P, c_geom64.piece_nv[p] == 3, Q, c_geom64.piece_nv[q] == 3))
+                    if (!(atomicOr(&near[wn], 0x80000000u) >> 31)) atomicAdd(&cnt[2], 1);
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) cnt[1] = 0;
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) cnt[0] = 0;
+        __syncthreads();
     }
-    count = pk_block_sum<int>(count, redi);
     if (threadIdx.x == 0) {
-        overlaps[e] = count;
-        side[e] = n > 0 ? fmax(bx1 - bx0, by1 - by0) : 0.0;
+        overlaps[e] = n > 1 ? cnt[2] : 0;
+        side[e] = n > 0 ? fmax(bb[1] + bb[0], bb[3] + bb[2]) : 0.0;
     }
 }
 
@@ -112,7 +225,7 @@ extern "C" int pk_validate_fp64(const void* xyt, int dtype_bytes, int E, int n, 
     if (E == 0) return PK_OK;
     if ((!xyt && n > 0) || !overlaps || !side) return pk_fail(PK_EINVAL, "pk_validate_fp64: NULL pointer%s");
     const int T = n <= 64 ? 64 : (n <= 128 ? 128 : 256);
-    const size_t smem = (size_t)n * 32 + 32 * 8 + 32 * 4;
+    const size_t smem = pk_validate_smem(n, T);
     cudaStream_t st = (cudaStream_t)stream;
     cudaError_t err;
     if (dtype_bytes == 4) {

@@ -63,3 +63,39 @@ def test_relaxed_packings_become_legal(cuda):
     assert np.array_equal(ov, oov)
     np.testing.assert_allclose(side, oside, rtol=1e-12)
     assert (ov == 0).mean() > 0.9
+
+
+@pytest.mark.parametrize("n,kind", [(1, "rows"), (2, "pile"), (3, "pile"), (64, "rows"), (65, "pile"), (129, "far"),
+                                    (200, "rows"), (301, "pile"), (1024, "pile"), (1023, "rows")])
+def test_list_edges_match_oracle(cuda, n, kind):
+    """Sizes around the CTA's and the list's limits: rows of nearly touching
+    trees, piles whose near pairs overflow the list many times, and clusters a
+    million units apart (where the FP32 culls must keep their margin)."""
+    rng = np.random.default_rng(n)
+    E = 3 if n < 1000 else 1
+    th = rng.uniform(0, 2 * np.pi, size=(E, n, 1))
+    if kind == "rows":
+        k = np.arange(n)
+        cols = max(1, int(np.sqrt(2.2 * n)))
+        xy = np.stack([(k % cols) * 0.46, (k // cols) * 1.02 + 0.06 * (k % cols % 2)], 1)[None] + rng.normal(
+            scale=0.01, size=(E, n, 2))
+        th = (k % cols % 2 * np.pi)[None, :, None] + rng.normal(scale=0.03, size=(E, n, 1))
+    elif kind == "pile":
+        s = 1.5 if n < 1000 else 6.0
+        xy = rng.uniform(-s, s, size=(E, n, 2))
+    else:
+        c = rng.uniform(-1e6, 1e6, size=(E, n // 3 + 1, 1, 2))
+        xy = (c + rng.uniform(-0.6, 0.6, size=(E, n // 3 + 1, 3, 2))).reshape(E, -1, 2)[:, :n]
+    x = np.concatenate([xy, th], 2)
+    for dtype in (torch.float64, torch.float32):
+        xs = x if dtype == torch.float64 else x.astype(np.float32).astype(np.float64)
+        ov, side = _val(xs, cuda, dtype)
+        oov, oside = O.validate(xs)
+        if kind == "far":
+            # the oracle's clipped areas lose 1e-4 to cancellation out there: take
+            # its count cluster by cluster, each moved (exactly) to the origin
+            move = np.round(c)
+            oov = sum(O.validate(np.concatenate([xs[:, 3 * k:3 * k + 3, :2] - move[:, k], xs[:, 3 * k:3 * k + 3, 2:]],
+                                                2))[0] for k in range(n // 3))
+        assert np.array_equal(ov, oov)
+        np.testing.assert_allclose(side, oside, rtol=1e-12)
