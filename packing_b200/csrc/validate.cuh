@@ -54,26 +54,63 @@ __device__ __forceinline__ void pk_block_max4d(double (&v)[4], double* red)
         for (int k = 0; k < 4; ++k) v[k] = fmax(v[k], red[4 * w + k]);
 }
 
+// The same test in FP32 on coordinates about one tree's centre, decided only
+// where rounding cannot matter: -1 if some edge normal separates the pieces by
+// more than margin, 1 if every normal has them overlap by more than margin, 0
+// if FP64 has to say.  (The normals are not unit vectors but shorter than 1, so
+// the margin in distance is larger still.)
+__device__ __forceinline__ int pk_pieces_overlap32(const float2 (&P)[4], bool pt, const float2 (&Q)[4], bool qt,
+                                                   float margin)
+{
+    float least = 1e30f;   // smallest overlap along a normal so far
+#pragma unroll
+    for (int pass = 0; pass < 2; ++pass) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const bool tri = pass == 0 ? pt : qt;
+            const float2 a = pass == 0 ? P[k] : Q[k];
+            const float2 b = pass == 0 ? P[(k + 1) & 3] : Q[(k + 1) & 3];
+            const float nx = -(b.y - a.y), ny = b.x - a.x;
+            float mn1 = 1e30f, mx1 = -1e30f, mn2 = 1e30f, mx2 = -1e30f;
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                const float p1 = P[v].x * nx + P[v].y * ny, p2 = Q[v].x * nx + Q[v].y * ny;
+                mn1 = fminf(mn1, p1); mx1 = fmaxf(mx1, p1);
+                mn2 = fminf(mn2, p2); mx2 = fmaxf(mx2, p2);
+            }
+            const float ov = fminf(mx1 - mn2, mx2 - mn1);
+            if (!(k == 3 && tri)) least = fminf(least, ov);   // a triangle's fourth edge has no length
+        }
+    }
+    return least < -margin ? -1 : (least > margin ? 1 : 0);
+}
+
 // Shared memory of the validator: near pairs (an index into which, with two
-// piece numbers, is an item: 12 + 2 + 2 bits) and the items of T near pairs.
+// piece numbers, is an item: 12 + 2 + 2 bits), the items of T near pairs and
+// those of them that FP32 cannot decide.
 #define PK_VAL_NEAR 4096
 static size_t pk_validate_smem(int n, int T)
 {
-    return (size_t)n * (32 + 64 + 8) + 32 * 8 + 16 + (size_t)PK_VAL_NEAR * 4 + (size_t)16 * T * 2;
+    return (size_t)n * (32 + 64) + 32 * 8 + 16 + 16 * 8 + (size_t)PK_VAL_NEAR * 4 + ((size_t)n + n / 2 + 16) * 8 +
+           (size_t)2 * 16 * T * 2;
 }
 
-// One CTA per packing.  Bound by FP64 issue in the separating-axis tests, so
-// the work before them only narrows what reaches them, in FP32 with margins
-// that never drop a pair whose exact test could say "overlap":
-//   - centres farther apart than two radii (thread per tree, offsets 1 .. n/2:
-//     no index division, conflict-free reads);
+// One CTA per packing.  Nearly every decision can be made in FP32 with a margin
+// that covers its rounding; only what lies within the margin goes to the exact
+// FP64 test:
+//   - centres farther apart than two radii (thread per tree, offsets 1 .. n/2
+//     read from an array that runs on past n: no index division, no wrap,
+//     conflict-free);
 //   - of a near pair's 16 piece pairs, those whose boxes are apart by more than
 //     the margin: some edge normal then separates the pieces by more than FP64
-//     rounding (each piece corner is wider than 30 degrees).
-// The piece pairs left over are listed and tested one per thread, so a warp's
-// lanes do the same work (one thread per near pair ran its 16 tests, each with
-// its pieces placed again, beside lanes with none).  4096 x n = 200: 0.97 ms
-// before.
+//     rounding (each piece corner is wider than 30 degrees);
+//   - piece pairs that a normal separates, or all normals have overlap, by more
+//     than the margin.
+// Each narrowing step lists what is left, one entry per thread in the next, so a
+// warp's lanes do the same work.  (Before: one thread per near pair ran its 16
+// FP64 tests beside lanes with none, 4096 x n = 200 in 0.97 ms; with lists but
+// every listed test in FP64, whose minima and maxima are three instructions
+// each, 0.38 ms.)
 template <typename T>
 __global__ void __launch_bounds__(256, 3)
 pk_validate_kernel(const T* __restrict__ xyt, int E, int n, int* __restrict__ overlaps, double* __restrict__ side)
@@ -82,16 +119,23 @@ pk_validate_kernel(const T* __restrict__ xyt, int E, int n, int* __restrict__ ov
     double4* pose = (double4*)pk_smem;            // [n] x, y, cos, sin
     float4* box = (float4*)(pose + n);            // [4][n] per piece: minx, maxx, miny, maxy about the centre
     double* red = (double*)(box + 4 * n);         // [32]
-    int* cnt = (int*)(red + 32);                  // near pairs, items, overlapping pairs
-    uint32_t* near = (uint32_t*)(cnt + 4);        // [PK_VAL_NEAR] i | j << 11 | overlap << 31
-    float2* pos = (float2*)(near + PK_VAL_NEAR);  // [n] FP32 centres about the bounding box's corner
-    uint16_t* items = (uint16_t*)(pos + n);       // [16 * blockDim.x] near index | p << 12 | q << 14
+    int* cnt = (int*)(red + 32);                  // near pairs, items, overlapping pairs, undecided items
+    float2* piece = (float2*)(cnt + 4);           // [16] the legality tree's pieces in FP32
+    uint32_t* near = (uint32_t*)(piece + 16);     // [PK_VAL_NEAR] i | j << 11 | overlap << 31
+    float2* pos = (float2*)(near + PK_VAL_NEAR);  // [n + n/2 + 16] FP32 centres about the bounding box's corner
+    uint16_t* items = (uint16_t*)(pos + n + n / 2 + 16);   // [16 T] near index | p << 12 | q << 14
+    uint16_t* undecided = items + 16 * blockDim.x;         // [16 T]
     const int e = blockIdx.x;
     if (e >= E) return;
     const T* X = xyt + (size_t)e * n * 3;
     const int lane = threadIdx.x & 31;
     double bb[4] = {-1e300, -1e300, -1e300, -1e300};   // -min x, max x, -min y, max y
-    if (threadIdx.x < 3) cnt[threadIdx.x] = 0;
+    if (threadIdx.x < 4) cnt[threadIdx.x] = 0;
+    if (threadIdx.x < 16) {
+        const double2 l = c_geom64.legal_piece[threadIdx.x >> 2][threadIdx.x & 3];
+        piece[threadIdx.x] = make_float2((float)l.x, (float)l.y);
+    }
+    __syncthreads();
     for (int t = threadIdx.x; t < n; t += blockDim.x) {
         const double x = (double)X[3 * t], y = (double)X[3 * t + 1], th = (double)X[3 * t + 2];
         double s, c;
@@ -109,8 +153,8 @@ pk_validate_kernel(const T* __restrict__ xyt, int E, int n, int* __restrict__ ov
             float4 b = make_float4(1e30f, -1e30f, 1e30f, -1e30f);
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
-                const float lx = (float)c_geom64.legal_piece[p][v].x, ly = (float)c_geom64.legal_piece[p][v].y;
-                const float vx = cf * lx - sf * ly, vy = sf * lx + cf * ly;
+                const float2 l = piece[4 * p + v];
+                const float vx = cf * l.x - sf * l.y, vy = sf * l.x + cf * l.y;
                 b.x = fminf(b.x, vx); b.y = fmaxf(b.y, vx);
                 b.z = fminf(b.z, vy); b.w = fmaxf(b.w, vy);
             }
@@ -123,31 +167,54 @@ pk_validate_kernel(const T* __restrict__ xyt, int E, int n, int* __restrict__ ov
     const float margin = (float)(1e-5 + 1e-6 * ext);
     const float reach = 2.0f * (float)c_geom64.legal_radius + 2.0f * margin;
     const float reach2 = reach * reach;
-    for (int t = threadIdx.x; t < n; t += blockDim.x) {
-        const double4 A = pose[t];
+    const int half = n >> 1;
+    for (int t = threadIdx.x; t < n + half; t += blockDim.x) {
+        const double4 A = pose[t < n ? t : t - n];
         pos[t] = make_float2((float)(A.x + bb[0]), (float)(A.y + bb[2]));
     }
     __syncthreads();
     const double cut = 4.0 * c_geom64.legal_radius * c_geom64.legal_radius * (1.0 + 1e-12);
-    const int half = n >> 1;
-    const int group = max(1, PK_VAL_NEAR / (2 * max(n, 1)));   // offsets between looks at the list
+    // offsets between looks at the list: a group always fits an empty one
+    const int group = max(4, min(16, (PK_VAL_NEAR / max(n, 1)) & ~3));
     for (int d0 = 1; d0 <= half; d0 += group) {
-        const int d1 = min(half, d0 + group - 1);
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            const float2 a = pos[i];
-            for (int d = d0; d <= d1; ++d) {
-                if (2 * d == n && i >= d) break;   // the offset n / 2 meets each pair twice
-                int j = i + d;
+        const int nd = min(group, half - d0 + 1);
+        for (int i0 = 0; i0 < n; i0 += blockDim.x) {
+            const int i = i0 + threadIdx.x;
+            uint32_t hit = 0;
+            if (i < n) {
+                const float2 a = pos[i];
+                for (int b = 0; b < nd; b += 4)
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {   // up to 3 past half: inside the array, masked below
+                        const float2 o = pos[i + d0 + b + u];
+                        const float dx = o.x - a.x, dy = o.y - a.y;
+                        hit |= (uint32_t)!(dx * dx + dy * dy > reach2) << (b + u);
+                    }
+                hit &= (1u << nd) - 1u;
+                if (2 * (d0 + nd - 1) == n && i >= half) hit &= ~(1u << (nd - 1));   // offset n/2 meets a pair twice
+            }
+            const int k = __popc(hit);
+            int incl = k;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(PK_FULL_MASK, incl, o);
+                if (lane >= o) incl += u;
+            }
+            int base = 0;
+            if (lane == 31 && incl) base = atomicAdd(&cnt[0], incl);
+            int at = __shfl_sync(PK_FULL_MASK, base, 31) + incl - k;
+            while (hit) {
+                const int b = __ffs(hit) - 1;
+                hit &= hit - 1;
+                int j = i + d0 + b;
                 if (j >= n) j -= n;
-                const float dx = pos[j].x - a.x, dy = pos[j].y - a.y;
-                if (dx * dx + dy * dy > reach2) continue;
-                near[atomicAdd(&cnt[0], 1)] = (uint32_t)i | ((uint32_t)j << 11);
+                near[at++] = (uint32_t)i | ((uint32_t)j << 11);
             }
         }
         __syncthreads();
         const int cn = cnt[0];
         __syncthreads();   // everyone has read it before anyone appends again
-        if (d1 < half && cn + group * n <= PK_VAL_NEAR) continue;   // uniform: the next group fits
+        if (d0 + group <= half && cn + group * n <= PK_VAL_NEAR) continue;   // uniform: the next group fits
         for (int c0 = 0; c0 < cn; c0 += blockDim.x) {
             const int w = c0 + threadIdx.x;
             uint32_t mask = 0;
@@ -160,11 +227,11 @@ pk_validate_kernel(const T* __restrict__ xyt, int E, int n, int* __restrict__ ov
 #pragma unroll
                     for (int p = 0; p < 4; ++p) {
                         const float4 a = box[p * n + i];
+                        const float4 am = make_float4(a.x - margin, a.y + margin, a.z - margin, a.w + margin);
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
                             const float4 b = box[q * n + j];
-                            const bool apart = a.y + margin < b.x + fx || b.y + fx + margin < a.x ||
-                                               a.w + margin < b.z + fy || b.w + fy + margin < a.z;
+                            const bool apart = am.y < b.x + fx || b.y + fx < am.x || am.w < b.z + fy || b.w + fy < am.z;
                             mask |= (uint32_t)!apart << (4 * p + q);
                         }
                     }
@@ -192,6 +259,29 @@ pk_validate_kernel(const T* __restrict__ xyt, int E, int n, int* __restrict__ ov
                 const uint32_t ij = near[wn];
                 if (ij >> 31) continue;   // another piece pair of these trees has been found to overlap
                 const double4 A = pose[ij & 2047], B = pose[(ij >> 11) & 2047];
+                const float ac = (float)A.z, as = (float)A.w, bc = (float)B.z, bs = (float)B.w;
+                const float fx = (float)(B.x - A.x), fy = (float)(B.y - A.y);
+                float2 P[4], Q[4];
+#pragma unroll
+                for (int k2 = 0; k2 < 4; ++k2) {
+                    const float2 l = piece[4 * p + k2], m = piece[4 * q + k2];
+                    P[k2] = make_float2(ac * l.x - as * l.y, as * l.x + ac * l.y);
+                    Q[k2] = make_float2(bc * m.x - bs * m.y + fx, bs * m.x + bc * m.y + fy);
+                }
+                const int r = pk_pieces_overlap32(P, c_geom64.piece_nv[p] == 3, Q, c_geom64.piece_nv[q] == 3, margin);
+                if (r > 0) {
+                    if (!(atomicOr(&near[wn], 0x80000000u) >> 31)) atomicAdd(&cnt[2], 1);
+                } else if (r == 0) {
+                    undecided[atomicAdd(&cnt[3], 1)] = (uint16_t)v;
+                }
+            }
+            __syncthreads();
+            const int nu = cnt[3];
+            for (int it = threadIdx.x; it < nu; it += blockDim.x) {
+                const int v = undecided[it], wn = v & (PK_VAL_NEAR - 1), p = (v >> 12) & 3, q = v >> 14;
+                const uint32_t ij = near[wn];
+                if (ij >> 31) continue;
+                const double4 A = pose[ij & 2047], B = pose[(ij >> 11) & 2047];
                 double2 P[4], Q[4];
 #pragma unroll
                 for (int k2 = 0; k2 < 4; ++k2) {
@@ -203,7 +293,7 @@ pk_validate_kernel(const T* __restrict__ xyt, int E, int n, int* __restrict__ ov
                     if (!(atomicOr(&near[wn], 0x80000000u) >> 31)) atomicAdd(&cnt[2], 1);
             }
             __syncthreads();
-            if (threadIdx.x == 0) cnt[1] = 0;
+            if (threadIdx.x == 0) { cnt[1] = 0; cnt[3] = 0; }
             __syncthreads();
         }
         if (threadIdx.x == 0) cnt[0] = 0;
