@@ -25,7 +25,7 @@ struct PkCostSmem {
     unsigned* acc_lo;   // [3*n_max] fixed-point gradient, low words
     unsigned* acc_hi;   // [3*n_max] fixed-point gradient, high words
     float4* bnd;        // [n_max] boundary: cost, dh0, dh1, dh2 (unweighted)
-    uint32_t* items;    // [cap_items] piece pairs: i | j << 11 | pi << 22 | pj << 24
+    uint16_t* items;    // [cap_items] piece pairs: near list index | pi << 11 | pj << 13
     uint32_t* near;     // [cap_near] centre-culled pairs: i | j << 11
     int* count;         // items in the list
     double* red;        // [32]
@@ -49,15 +49,17 @@ struct PkCostSmem {
 // wide): two per tree, at least 64, at most 1024.
 __host__ __device__ inline int pk_grid_cap(int n_max) { return n_max < 32 ? 64 : (n_max > 512 ? 1024 : 2 * n_max); }
 
-// List capacities.  The near list takes 8 T pairs, at least the n_max - 1
-// pairs of one tree for every n_max that pk_cost_threads gives T for; an
-// expansion chunk appends at most 16 T piece pairs to the item list, which is
-// flushed before the next chunk could overflow it (the LUT's items are the
-// near pairs themselves).
+// List capacities.  The near list takes 8 T pairs (2048 at most: an item names
+// its pair by an 11-bit index), at least the n_max - 1 pairs of one tree for
+// every n_max that pk_cost_threads gives T for; an expansion chunk appends at
+// most 16 T piece pairs to the item list, which is flushed before the next
+// chunk could overflow it: above 20 T items, so that the about 7 T of a packing
+// of n = T trees are evaluated in one go (the LUT's items are the near pairs
+// themselves).
 __host__ __device__ inline void pk_caps(int T, int mode, int* cap_near, int* cap_items)
 {
     *cap_near = 8 * T;
-    *cap_items = mode == PK_PAIR_LUT ? 0 : 20 * T;
+    *cap_items = mode == PK_PAIR_LUT ? 0 : 36 * T;
 }
 
 // keep: room for the kept near list's state (the fused relaxation only; a
@@ -71,10 +73,10 @@ __host__ __device__ inline size_t pk_cost_smem_bytes(int n_max, int cap_near, in
     b += (size_t)n_max * 64;        // aabb
     b += (size_t)n_max * 24;        // acc
     b += (size_t)n_max * 4;         // theta
-    b += (size_t)cap_items * 4;     // items
+    b += (size_t)cap_items * 2;     // items
     b += (size_t)cap_near * 4;      // near pairs
     b += (size_t)(2 * pk_grid_cap(n_max) + 1) * 4 + (size_t)n_max * 16 + 4;   // grid
-    b += 32 * 8 + 32 * 8 + 16 * 8 + 4 * 4 + 16 + 16 + 16 + 16 + 128;
+    b += 8 * 16 + 16 * 8 + 16 + 16 + 16 + 32 * 8 + 32 * 8;   // piece tables, counters, reductions
     if (keep) b += 16 + 32 * 4;   // pk_nlist, pk_disp
     return (b + 15) & ~(size_t)15;   // whatever follows starts 16-byte aligned
 }
@@ -84,24 +86,24 @@ __device__ inline PkCostSmem pk_cost_carve(unsigned char* base, int n_max, int c
 {
     PkCostSmem s;
     unsigned char* p = base;
-    s.pose = (float4*)p; p += (size_t)n_max * 16;
-    s.bnd = (float4*)p; p += (size_t)n_max * 16;
-    s.aabb = (float4*)p; p += (size_t)n_max * 64;
-    s.piece4 = (float4*)p; p += 8 * 16;   // 16-byte aligned: every offset so far is a multiple of 16
-    // 8-byte arrays next: every offset up to here is a multiple of 16
-    s.red = (double*)p; p += 32 * 8;
-    s.redl = (long long*)p; p += 32 * 8;
-    if (keep) p += 32 * 4;   // pk_disp
-    s.acc_lo = (unsigned*)p; p += (size_t)n_max * 12;
-    s.acc_hi = (unsigned*)p; p += (size_t)n_max * 12;
+    // fixed sizes first: their addresses, and the poses', are constants
+    s.piece4 = (float4*)p; p += 8 * 16;
     s.piece = (float2*)p; p += 16 * 8;
-    s.theta = (float*)p; p += (size_t)n_max * 4;
-    s.items = (uint32_t*)p; p += (size_t)cap_items * 4;
-    s.near = (uint32_t*)p; p += (size_t)cap_near * 4;
     s.piece_nv = (int*)p; p += 16;
     s.count = (int*)p; p += 16;
     s.cnt = (unsigned int*)p; p += 16;
     if (keep) p += 16;   // pk_nlist
+    s.red = (double*)p; p += 32 * 8;
+    s.redl = (long long*)p; p += 32 * 8;
+    if (keep) p += 32 * 4;   // pk_disp
+    s.pose = (float4*)p; p += (size_t)n_max * 16;
+    s.bnd = (float4*)p; p += (size_t)n_max * 16;
+    s.aabb = (float4*)p; p += (size_t)n_max * 64;
+    s.near = (uint32_t*)p; p += (size_t)cap_near * 4;
+    s.items = (uint16_t*)p; p += (size_t)cap_items * 2;
+    s.acc_lo = (unsigned*)p; p += (size_t)n_max * 12;
+    s.acc_hi = (unsigned*)p; p += (size_t)n_max * 12;
+    s.theta = (float*)p; p += (size_t)n_max * 4;
     s.grid_cap = pk_grid_cap(n_max);
     s.cell_start = (int*)p; p += (size_t)(s.grid_cap + 1) * 4;
     s.cell_fill = (int*)p; p += (size_t)s.grid_cap * 4;
@@ -109,7 +111,6 @@ __device__ inline PkCostSmem pk_cost_carve(unsigned char* base, int n_max, int c
     s.tcell = (int*)p; p += (size_t)n_max * 4;
     s.near_cnt = (int*)p; p += (size_t)n_max * 4;
     s.near_start = (int*)p; p += (size_t)n_max * 4 + 4;
-    p += 16;
     s.cap_items = cap_items;
     s.cap_near = cap_near;
     s.n_cap = n_max;
@@ -264,30 +265,27 @@ __device__ __forceinline__ bool pk_clip_pass(const float2 (&X)[4], bool x_tri, c
                 }
             }
         }
+        // the part [tin, tout] of the edge, by selects: a warp's lanes cross
+        // different lines, so nearly every branch here would be taken by some
         const unsigned oa = out[v] & ~skip, ob = out[vb] & ~skip;
-        if (empty || (oa & ob)) continue;
-        const unsigned crossm = oa | ob;
         float tin = 0.f, tout = 1.f;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            if ((crossm >> k) & 1u) {
-                const float fa = f[k][v], fb = f[k][vb];
-                const float t = __fdividef(fa, fa - fb);
-                if ((oa >> k) & 1u) tin = fmaxf(tin, t);    // entering
-                else tout = fminf(tout, t);                 // leaving
-            }
+            const float fa = f[k][v], fb = f[k][vb];
+            const float t = __fdividef(fa, fa - fb);    // meaningful where the edge crosses line k
+            tin = fmaxf(tin, (oa >> k) & 1u ? t : 0.f);     // entering
+            tout = fminf(tout, (ob >> k) & 1u ? t : 1.f);   // leaving
         }
-        if (tin < tout) {
-            const float dt = tout - tin;
-            const float2 e = make_float2(b.x - a.x, b.y - a.y);
-            A2 += dt * pk_cross(a, b);
-            const float2 N = make_float2(dt * e.y, -dt * e.x);
-            const float tm = 0.5f * (tin + tout);
-            const float2 m = make_float2(a.x + tm * e.x - ctr.x, a.y + tm * e.y - ctr.y);
-            g.x += N.x;
-            g.y += N.y;
-            g.z += pk_cross(m, N);
-        }
+        const bool part = !empty && !(oa & ob) && tin < tout;
+        const float dt = part ? tout - tin : 0.f;
+        const float2 e = make_float2(b.x - a.x, b.y - a.y);
+        A2 += dt * pk_cross(a, b);
+        const float2 N = make_float2(dt * e.y, -dt * e.x);
+        const float tm = part ? 0.5f * (tin + tout) : 0.f;   // finite, so an empty part adds zeros
+        const float2 m = make_float2(a.x + tm * e.x - ctr.x, a.y + tm * e.y - ctr.y);
+        g.x += N.x;
+        g.y += N.y;
+        g.z += pk_cross(m, N);
     }
     return true;
 }
@@ -531,80 +529,136 @@ __device__ __forceinline__ int pk_is_near(float4 A, float4 B, float cutoff)
     return __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)) <= cutoff;
 }
 
-// Phase B: evaluate every listed item; returns this thread's fixed-point
-// pair total.  Items: i (11 bits) | j (11 bits) | pi (2) | pj (2).
-// filter (LUT only): the list is a kept near list, so a pair is looked up only
-// if it passes the centre cull now; the kept pairs are counted.
-template <int MODE>
-__device__ __forceinline__ long long pk_process_items(const PkCostSmem& sm, const uint32_t* list, int count,
-                                                      float w_pair, const PkLut& lut, bool filter = false,
-                                                      float cutoff = 0.f)
+// Whether some line of Y has every vertex of X on its outer side, by more than
+// tol: f[k][v] < -tol for all v, with the side values pk_clip_pass sees.
+__device__ __forceinline__ bool pk_line_separates(const PkQuad& X, const PkQuad& Y, float tol)
+{
+    float f[4][4];
+    pk_side_values_q(X, Y, f);
+    float m = 3.4e38f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) m = fminf(m, fmaxf(fmaxf(f[k][0], f[k][1]), fmaxf(f[k][2], f[k][3])));
+    return m < -tol;   // the degenerate fourth line of a triangle gives 0: it separates nothing
+}
+
+// Phase B, LUT: looks up the count near pairs of the list; returns this
+// thread's fixed-point pair total.  filter: the list is a kept near list, so a
+// pair is looked up only if it passes the centre cull now; the kept pairs are
+// counted.
+__device__ __forceinline__ long long pk_process_lut(const PkCostSmem& sm, int count, float w_pair, const PkLut& lut,
+                                                    bool filter, float cutoff)
 {
     long long tot = 0;
     unsigned kept = 0;
-    const int nwarps = blockDim.x >> 5;
-    for (int base = 0; base < count; base += blockDim.x) {
-        // Analytic modes, full rounds: a warp's lanes take items nwarps apart.
-        // Consecutive items share trees (a near pair's piece pairs, a tree's
-        // near pairs), and spread over warps their accumulator atomics stop
-        // hitting the same addresses within a warp (1 % at 4096 x n = 200;
-        // the same bits).  The LUT's lookups keep the contiguous order.
-        const int w = MODE != PK_PAIR_LUT && base + (int)blockDim.x <= count
-                          ? base + (int)(threadIdx.x & 31) * nwarps + (int)(threadIdx.x >> 5)
-                          : base + (int)threadIdx.x;
-        if (w >= count) continue;
-        const uint32_t it = list[w];
+#pragma unroll 1   // one pair's eight gathers in flight per thread: two were slower
+    for (int w = threadIdx.x; w < count; w += blockDim.x) {
+        const uint32_t it = sm.near[w];
         const int i = it & 2047, j = (it >> 11) & 2047;
         const float4 A = sm.pose[i], B = sm.pose[j];
-        if (MODE == PK_PAIR_LUT && filter) {
+        if (filter) {
             if (!pk_is_near(A, B, cutoff)) continue;
             ++kept;
         }
+        // ref = lower index, as the reference's triangular loop (pack_cuda_lut.py:437)
+        const int r = i < j ? i : j, o = i < j ? j : i;
+        const float4 R = sm.pose[r], O = sm.pose[o];
+        const float dxw = O.x - R.x, dyw = O.y - R.y;
+        const float dxl = R.z * dxw + R.w * dyw;
+        const float dyl = -R.w * dxw + R.z * dyw;
+        const float dth = pk_wrap_angle(sm.theta[o] - sm.theta[r]);
+        float3 gl;
+        float val = pk_lut_lookup(lut, dxl, dyl, dth, gl);
+        if (lut.quadratic) {
+            if (val > 0.f) {
+                gl.x *= 2.0f * val; gl.y *= 2.0f * val; gl.z *= 2.0f * val;
+                val = val * val;
+            } else {
+                val = 0.f;
+                gl = make_float3(0.f, 0.f, 0.f);
+            }
+        }
+        const float3 gr = make_float3(-gl.x * R.z + gl.y * R.w, -gl.x * R.w - gl.y * R.z,
+                                      gl.x * dyl - gl.y * dxl - gl.z);
+        const float3 go = make_float3(gl.x * R.z - gl.y * R.w, gl.x * R.w + gl.y * R.z, gl.z);
+        const float3 gi = (r == i) ? gr : go, gj = (r == i) ? go : gr;
+        if (val != 0.f || gi.x != 0.f || gi.y != 0.f || gi.z != 0.f) {
+            tot += pk_to_fx(w_pair * val);
+            pk_acc_add2(sm, i, make_float3(w_pair * gi.x, w_pair * gi.y, w_pair * gi.z));
+            pk_acc_add2(sm, j, make_float3(w_pair * gj.x, w_pair * gj.y, w_pair * gj.z));
+        }
+    }
+    if (filter) {
+        kept = __reduce_add_sync(PK_FULL_MASK, kept);
+        if ((threadIdx.x & 31) == 0 && kept) { atomicAdd(&sm.cnt[1], kept); atomicAdd(&sm.cnt[2], kept); }
+    }
+    return tot;
+}
+
+// Phase B, analytic modes: evaluates the count listed piece pairs; returns this
+// thread's fixed-point pair total.
+//
+// 36 % (initial poses of a random packing) to 45 % (relaxed) of the piece pairs
+// whose boxes meet are separated by one of their lines, 80 % in a nearly legal
+// packing's separation cost, and a lane with such a pair idled through the
+// clipper beside the others.  So each warp first tests its items (side values
+// and minima only) and keeps those not separated at the front of its own part
+// of the list, then evaluates these with full warps.  A warp's part is the
+// items warp, warp + nwarps, ...: no barrier between the two passes, and
+// consecutive items, which share trees, are spread over the warps, whose
+// accumulator atomics then rarely meet.
+//
+// The area's test is the clipper's own (same side values).  The separation's
+// axes are normalised and round differently, so there a line must clear the
+// pieces by 1e-6 (side value: gap times an edge shorter than 1; coordinates are
+// within 2 units, whose rounding is 3e-7) before the pair is dropped.
+template <int MODE>
+__device__ __forceinline__ long long pk_process_items(const PkCostSmem& sm, int count, float w_pair)
+{
+    long long tot = 0;
+    const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const float tol = MODE == PK_PAIR_AREA ? 0.f : 1e-6f;
+    uint16_t* const mine = sm.items + warp;
+    const int own = count > warp ? (count - warp + nw - 1) / nw : 0;   // items of this warp
+    int kept = 0;
+    for (int b = 0; b < own; b += 32) {
+        bool keep = false;
+        uint16_t it = 0;
+        if (b + lane < own) {
+            it = mine[(b + lane) * nw];
+            const uint32_t ij = sm.near[it & 2047];
+            const float4 A = sm.pose[ij & 2047], B = sm.pose[(ij >> 11) & 2047];
+            const PkQuad PQ = pk_load_quad(sm, (it >> 11) & 3, A.z, A.w, 0.f, 0.f);
+            const PkQuad QQ = pk_load_quad(sm, it >> 13, B.z, B.w, B.x - A.x, B.y - A.y);
+            keep = !pk_line_separates(PQ, QQ, tol) && !pk_line_separates(QQ, PQ, tol);
+        }
+        const unsigned m = __ballot_sync(PK_FULL_MASK, keep);
+        if (keep) mine[(kept + __popc(m & ((1u << lane) - 1u))) * nw] = it;
+        kept += __popc(m);
+    }
+    __syncwarp();
+    for (int b = lane; b < kept; b += 32) {
+        const int it = mine[b * nw], pi = (it >> 11) & 3, pj = it >> 13;
+        const uint32_t ij = sm.near[it & 2047];
+        const int i = ij & 2047, j = (ij >> 11) & 2047;
+        const float4 A = sm.pose[i], B = sm.pose[j];
         const float2 d = make_float2(B.x - A.x, B.y - A.y);
         float val;
         float3 gi, gj;
-        if (MODE == PK_PAIR_LUT) {
-            // ref = lower index, as the reference's triangular loop (pack_cuda_lut.py:437)
-            const int r = i < j ? i : j, o = i < j ? j : i;
-            const float4 R = sm.pose[r], O = sm.pose[o];
-            const float dxw = O.x - R.x, dyw = O.y - R.y;
-            const float dxl = R.z * dxw + R.w * dyw;
-            const float dyl = -R.w * dxw + R.z * dyw;
-            const float dth = pk_wrap_angle(sm.theta[o] - sm.theta[r]);
-            float3 gl;
-            val = pk_lut_lookup(lut, dxl, dyl, dth, gl);
-            if (lut.quadratic) {
-                if (val > 0.f) {
-                    gl.x *= 2.0f * val; gl.y *= 2.0f * val; gl.z *= 2.0f * val;
-                    val = val * val;
-                } else {
-                    val = 0.f;
-                    gl = make_float3(0.f, 0.f, 0.f);
-                }
-            }
-            float3 gr = make_float3(-gl.x * R.z + gl.y * R.w, -gl.x * R.w - gl.y * R.z,
-                                    gl.x * dyl - gl.y * dxl - gl.z);
-            float3 go = make_float3(gl.x * R.z - gl.y * R.w, gl.x * R.w + gl.y * R.z, gl.z);
-            gi = (r == i) ? gr : go;
-            gj = (r == i) ? go : gr;
+        const bool pt = sm.piece_nv[pi] == 3, qt = sm.piece_nv[pj] == 3;
+        if (MODE == PK_PAIR_AREA) {
+            const PkQuad PQ = pk_load_quad(sm, pi, A.z, A.w, 0.f, 0.f);
+            const PkQuad QQ = pk_load_quad(sm, pj, B.z, B.w, d.x, d.y);
+            pk_piece_area_grad_q(PQ, pt, QQ, qt, d, val, gi, gj);
         } else {
-            const int pi = (it >> 22) & 3, pj = (it >> 24) & 3;
-            const bool pt = sm.piece_nv[pi] == 3, qt = sm.piece_nv[pj] == 3;
-            if (MODE == PK_PAIR_AREA) {
-                const PkQuad PQ = pk_load_quad(sm, pi, A.z, A.w, 0.f, 0.f);
-                const PkQuad QQ = pk_load_quad(sm, pj, B.z, B.w, d.x, d.y);
-                pk_piece_area_grad_q(PQ, pt, QQ, qt, d, val, gi, gj);
-            } else {
-                float2 P[4], Q[4];
-                pk_load_piece(sm, pi, A.z, A.w, 0.f, 0.f, P);
-                pk_load_piece(sm, pj, B.z, B.w, d.x, d.y, Q);
-                float sp;
-                pk_piece_sat_grad(P, pt, Q, qt, d, sp, gi, gj);
-                const float f = 2.0f * sp;
-                gi = make_float3(f * gi.x, f * gi.y, f * gi.z);
-                gj = make_float3(f * gj.x, f * gj.y, f * gj.z);
-                val = sp * sp;
-            }
+            float2 P[4], Q[4];
+            pk_load_piece(sm, pi, A.z, A.w, 0.f, 0.f, P);
+            pk_load_piece(sm, pj, B.z, B.w, d.x, d.y, Q);
+            float sp;
+            pk_piece_sat_grad(P, pt, Q, qt, d, sp, gi, gj);
+            const float f = 2.0f * sp;
+            gi = make_float3(f * gi.x, f * gi.y, f * gi.z);
+            gj = make_float3(f * gj.x, f * gj.y, f * gj.z);
+            val = sp * sp;
         }
         if (val != 0.f || gi.x != 0.f || gi.y != 0.f || gi.z != 0.f) {
             tot += pk_to_fx(w_pair * val);
@@ -612,11 +666,20 @@ __device__ __forceinline__ long long pk_process_items(const PkCostSmem& sm, cons
             pk_acc_add2(sm, j, make_float3(w_pair * gj.x, w_pair * gj.y, w_pair * gj.z));
         }
     }
-    if (MODE == PK_PAIR_LUT && filter) {
-        kept = __reduce_add_sync(PK_FULL_MASK, kept);
-        if ((threadIdx.x & 31) == 0 && kept) { atomicAdd(&sm.cnt[1], kept); atomicAdd(&sm.cnt[2], kept); }
-    }
     return tot;
+}
+
+// The fused relaxation evaluates its items out of line: one call per flush
+// saves the optimiser's registers once, and the clipper has the rest to itself.
+// Inlined, they were live across it and spilled per item.  Carves the shared
+// memory again, like pk_broad_phase_outlined.
+template <int MODE>
+__device__ __noinline__ long long pk_process_items_outlined(int n_cap, int cap_near, int cap_items, int count,
+                                                            float w_pair)
+{
+    extern __shared__ __align__(16) unsigned char pk_smem[];
+    const PkCostSmem sm = pk_cost_carve(pk_smem, n_cap, cap_near, cap_items, true);
+    return pk_process_items<MODE>(sm, count, w_pair);
 }
 
 // Sorted-position ranges [b0, b1) and [b2, b3) of the half neighbourhood of
@@ -653,7 +716,7 @@ __device__ __forceinline__ long long pk_flush_near(const PkCostSmem& sm, int cn,
     if (MODE == PK_PAIR_LUT) {
         const bool filter = KEEP && pk_nlist(sm)[2] != 0;
         if (threadIdx.x == 0 && !filter) sm.cnt[2] += (unsigned)cn;
-        tot += pk_process_items<MODE>(sm, sm.near, cn, spec.w_pair, spec.lut, filter, c_geom.cutoff_sq);
+        tot += pk_process_lut(sm, cn, spec.w_pair, spec.lut, filter, c_geom.cutoff_sq);
     } else {
         for (int c0 = 0; c0 < cn; c0 += T) {
             const int w = c0 + threadIdx.x;
@@ -703,13 +766,14 @@ __device__ __forceinline__ long long pk_flush_near(const PkCostSmem& sm, int cn,
             while (mask) {
                 const int b = __ffs(mask) - 1;
                 mask &= mask - 1;
-                sm.items[pos++] = ij | ((uint32_t)(b >> 2) << 22) | ((uint32_t)(b & 3) << 24);
+                sm.items[pos++] = (uint16_t)(w | ((b >> 2) << 11) | ((b & 3) << 13));
             }
             __syncthreads();
             const int ci = *sm.count;
             __syncthreads();
             if (ci > sm.cap_items - 16 * T || c0 + T >= cn) {
-                tot += pk_process_items<MODE>(sm, sm.items, ci, spec.w_pair, spec.lut);
+                tot += KEEP ? pk_process_items_outlined<MODE>(sm.n_cap, sm.cap_near, sm.cap_items, ci, spec.w_pair)
+                            : pk_process_items<MODE>(sm, ci, spec.w_pair);
                 __syncthreads();
                 if (threadIdx.x == 0) *sm.count = 0;
                 __syncthreads();
