@@ -702,7 +702,7 @@ __device__ __forceinline__ void pk_half_neighbourhood(const PkCostSmem& sm, int 
 
 // Processes the cn near pairs of the list: the LUT looks them up directly;
 // the analytic modes expand each into the piece pairs whose boxes overlap and
-// evaluate those in chunks.  With KEEP the list may be a kept near list
+// evaluate those, all in one go unless they overflow the item list.  With KEEP the list may be a kept near list
 // (pk_nlist(sm)[2] set), whose pairs were within cutoff + skin when it was
 // built: each pair is then first tested against the centre cutoff at the
 // current poses, and the pairs that pass are counted.  The flag is read where
@@ -718,69 +718,80 @@ __device__ __forceinline__ long long pk_flush_near(const PkCostSmem& sm, int cn,
         if (threadIdx.x == 0 && !filter) sm.cnt[2] += (unsigned)cn;
         tot += pk_process_lut(sm, cn, spec.w_pair, spec.lut, filter, c_geom.cutoff_sq);
     } else {
-        for (int c0 = 0; c0 < cn; c0 += T) {
-            const int w = c0 + threadIdx.x;
-            const bool filter = KEEP && pk_nlist(sm)[2] != 0;
-            uint32_t mask = 0, ij = 0;
-            bool keep = false;
-            float4 A, B;
-            if (w < cn) {
-                ij = sm.near[w];
-                A = sm.pose[ij & 2047];
-                B = sm.pose[(ij >> 11) & 2047];
-                keep = !filter || pk_is_near(A, B, c_geom.cutoff_sq);
-            }
-            if (filter) {
-                const unsigned kb = __ballot_sync(PK_FULL_MASK, keep);
-                if (lane == 0 && kb) atomicAdd(&sm.cnt[1], (unsigned)__popc(kb));
-            }
-            if (keep) {
-                const int i = ij & 2047, j = (ij >> 11) & 2047;
-                const float dx = B.x - A.x, dy = B.y - A.y;
+        // Each warp expands every nwarps-th 32 pairs and reserves room for their
+        // items; one that finds none stops, and goes on after the list is done.
+        const bool filter = KEEP && pk_nlist(sm)[2] != 0;
+        const int chunks = (cn + 31) >> 5, nw = T >> 5;
+        int ch = threadIdx.x >> 5;
+        unsigned near = 0;
+        for (;;) {
+            for (; ch < chunks; ch += nw) {
+                const int w = 32 * ch + lane;
+                uint32_t mask = 0;
+                bool keep = false;
+                if (w < cn) {
+                    const uint32_t ij = sm.near[w];
+                    const int i = ij & 2047, j = (ij >> 11) & 2047;
+                    const float4 A = sm.pose[i], B = sm.pose[j];
+                    keep = !filter || pk_is_near(A, B, c_geom.cutoff_sq);
+                    if (keep) {
+                        const float dx = B.x - A.x, dy = B.y - A.y;
+                        float4 bq[4];
 #pragma unroll
-                for (int p = 0; p < 4; ++p) {
-                    const float4 a = sm.aabb[p * sm.n_cap + i];
+                        for (int q = 0; q < 4; ++q) {
+                        }
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const float4 b = sm.aabb[q * sm.n_cap + j];
-                        const bool ov = !(a.y < b.x + dx || b.y + dx < a.x || a.w < b.z + dy || b.w + dy < a.z);
-                        mask |= (uint32_t)ov << (4 * p + q);
+                        for (int p = 0; p < 4; ++p) {
+                            const float4 a = sm.aabb[p * sm.n_cap + i];
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) {
+                                const float4 b2 = sm.aabb[q * sm.n_cap + j];
+                                const bool ov = !(a.y < b2.x + dx || b2.y + dx < a.x || a.w < b2.z + dy || b2.w + dy < a.z);
+                                mask |= (uint32_t)ov << (4 * p + q);
+                            }
+                        }
                     }
                 }
-            }
-            const int cnt = __popc(mask);
-            int incl = cnt;
+                const int cnt = __popc(mask);
+                int incl = cnt;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(PK_FULL_MASK, incl, o);
-                if (lane >= o) incl += v;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(PK_FULL_MASK, incl, o);
+                    if (lane >= o) incl += v;
+                }
+                const int wtot = __shfl_sync(PK_FULL_MASK, incl, 31);
+                int wbase = 0;
+                if (lane == 31 && wtot) {
+                    // once a reservation fails every later one does (the count
+                    // is above the capacity until it is taken back), so the
+                    // list has no gaps
+                    wbase = atomicAdd(sm.count, wtot);
+                    if (wbase + wtot > sm.cap_items) { atomicSub(sm.count, wtot); wbase = -1; }
+                }
+                wbase = __shfl_sync(PK_FULL_MASK, wbase, 31);
+                if (wbase < 0) break;
+                if (filter) near += (unsigned)__popc(__ballot_sync(PK_FULL_MASK, keep));
+                int pos = wbase + incl - cnt;
+                while (mask) {
+                    const int b = __ffs(mask) - 1;
+                    mask &= mask - 1;
+                    sm.items[pos++] = (uint16_t)(w | ((b >> 2) << 11) | ((b & 3) << 13));
+                }
             }
-            const int wtot = __shfl_sync(PK_FULL_MASK, incl, 31);
-            int wbase = 0;
-            if (lane == 31 && wtot) {
-                wbase = atomicAdd(sm.count, wtot);
-                atomicAdd(&sm.cnt[2], (unsigned)wtot);
-            }
-            wbase = __shfl_sync(PK_FULL_MASK, wbase, 31);
-            int pos = wbase + incl - cnt;
-            while (mask) {
-                const int b = __ffs(mask) - 1;
-                mask &= mask - 1;
-                sm.items[pos++] = (uint16_t)(w | ((b >> 2) << 11) | ((b & 3) << 13));
-            }
-            __syncthreads();
+            const int more = __syncthreads_or(ch < chunks);
             const int ci = *sm.count;
+            if (threadIdx.x == 0) sm.cnt[2] += (unsigned)ci;
+            tot += KEEP ? pk_process_items_outlined<MODE>(sm.n_cap, sm.cap_near, sm.cap_items, ci, spec.w_pair)
+                        : pk_process_items<MODE>(sm, ci, spec.w_pair);
+            if (!more) break;
             __syncthreads();
-            if (ci > sm.cap_items - 16 * T || c0 + T >= cn) {
-                tot += KEEP ? pk_process_items_outlined<MODE>(sm.n_cap, sm.cap_near, sm.cap_items, ci, spec.w_pair)
-                            : pk_process_items<MODE>(sm, ci, spec.w_pair);
-                __syncthreads();
-                if (threadIdx.x == 0) *sm.count = 0;
-                __syncthreads();
-            }
+            if (threadIdx.x == 0) *sm.count = 0;
+            __syncthreads();
         }
+        if (near && lane == 0) atomicAdd(&sm.cnt[1], near);
     }
     __syncthreads();
+    if (MODE != PK_PAIR_LUT && threadIdx.x == 0) *sm.count = 0;   // the next flush appends after another barrier
     return tot;
 }
 

@@ -224,3 +224,29 @@ def test_argument_errors(cuda):
     with pytest.raises(ValueError):
         pack_cuda.overlap_multi_ensemble(x, x, False, out_cost=c, crystal_axes=torch.zeros(2, 4, device=cuda),
                                          N_periodic=-1)
+
+
+@pytest.mark.parametrize("pair", ["area", "sep"])
+@pytest.mark.parametrize("n", [2, 33, 40, 120])
+def test_piled_trees_overflow_the_lists(cuda, n, pair):
+    """Trees piled on one spot: about ten box-overlapping piece pairs per pair of
+    trees, far more than a small CTA's item list.  Whatever the lists' sizes (32 to 256
+    threads) the same bits, and the oracle's cost and area gradient."""
+    from packing_b200.classes import SizeClass
+    from packing_b200.cost import CostSpec, compound_cost
+    rng = np.random.default_rng(n)
+    E = 5
+    x = np.concatenate([rng.uniform(-0.25, 0.25, size=(E, n, 2)), rng.uniform(0, 2 * np.pi, size=(E, n, 1))],
+                       2).astype(np.float32)
+    spec = CostSpec(pair=pair, w_pair=1.0, w_boundary=0.0, w_area=0.0)
+    flat = _t(x.reshape(-1, 3), cuda)
+    off = torch.arange(0, (E + 1) * n, n, dtype=torch.int32, device=cuda)
+    order = torch.arange(E, dtype=torch.int32, device=cuda)
+    got = [compound_cost(flat, None, spec, offsets=off, n_max=n, order=order, classes=[SizeClass(0, E, n, t)])[:2]
+           for t in (32, 64, 96, 256)]
+    for c, g in got[1:]:
+        assert torch.equal(c, got[0][0]) and torch.equal(g, got[0][1])
+    oc, og = O.pair_cost(x.astype(np.float64), pair == "sep")
+    np.testing.assert_allclose(got[0][0].cpu().numpy(), oc, rtol=RTOL_COST)
+    if pair == "area":   # the separation's smallest axis can differ between FP32 and FP64 where two tie
+        np.testing.assert_allclose(got[0][1].cpu().numpy().reshape(E, n, 3), og, rtol=TOL_GRAD, atol=TOL_GRAD)
