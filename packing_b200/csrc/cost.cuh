@@ -152,16 +152,9 @@ __device__ __forceinline__ float pk_cross3_rn(float2 a, float2 b, float2 c)
     return __fmaf_rn(b.x - a.x, c.y - a.y, -__fmul_rn(b.y - a.y, c.x - a.x));
 }
 
-// f[k][v] = cross(Y[k+1] - Y[k], X[v] - Y[k]): X's vertices against Y's
-// edge lines (>= 0 inside).
-__device__ __forceinline__ void pk_side_values(const float2 (&X)[4], const float2 (&Y)[4], float (&f)[4][4])
-{
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) f[k][v] = pk_cross3_rn(Y[k], Y[(k + 1) & 3], X[v]);
-}
-
+// Side values: f[k][v] = cross(Y[k+1] - Y[k], X[v] - Y[k]), X's vertices against
+// Y's edge lines (>= 0 inside).
+//
 // A convex piece's four vertices packed in pairs for the FP32x2 instructions
 // of sm_100 (FFMA2 / FMUL2: two independent FP32 operations, each rounded
 // like its scalar form): x01 = (x0, x1), x23 = (x2, x3), likewise y.
@@ -181,63 +174,98 @@ __device__ __forceinline__ PkQuad pk_quad(const float2 (&V)[4])
     return q;
 }
 
-// f[k][v] for the four lines of Y, two vertices of X per instruction, with
-// the rounding of pk_cross3_rn (the vertex is taken relative to the line's
-// first point before the cross product, which keeps small side values
-// accurate wherever the pieces lie).
+// X's four vertices against line k of Y, two per instruction: (f0, f1) in f01,
+// (f2, f3) in f23, with the rounding of pk_cross3_rn (the vertex is taken
+// relative to the line's first point before the cross product, which keeps
+// small side values accurate wherever the pieces lie).
+__device__ __forceinline__ void pk_side_line(const PkQuad& X, const PkQuad& Y, int k, float2& f01, float2& f23)
+{
+    const float2 a = pk_qv(Y, k), b = pk_qv(Y, (k + 1) & 3);
+    const float ex = b.x - a.x, ey = b.y - a.y;
+    const float2 ex2 = make_float2(ex, ex), ney2 = make_float2(-ey, -ey);
+    const float2 nax2 = make_float2(-a.x, -a.x), nay2 = make_float2(-a.y, -a.y);   // x - a = x + (-a), exactly
+    f01 = __ffma2_rn(ex2, __fadd2_rn(X.y01, nay2), __fmul2_rn(ney2, __fadd2_rn(X.x01, nax2)));
+    f23 = __ffma2_rn(ex2, __fadd2_rn(X.y23, nay2), __fmul2_rn(ney2, __fadd2_rn(X.x23, nax2)));
+}
+
+// f[k][v] for the four lines of Y.
 __device__ __forceinline__ void pk_side_values_q(const PkQuad& X, const PkQuad& Y, float (&f)[4][4])
 {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const float2 a = pk_qv(Y, k), b = pk_qv(Y, (k + 1) & 3);
-        const float ex = b.x - a.x, ey = b.y - a.y;
-        const float2 ex2 = make_float2(ex, ex), ney2 = make_float2(-ey, -ey);
-        const float2 nax2 = make_float2(-a.x, -a.x), nay2 = make_float2(-a.y, -a.y);   // x - a = x + (-a), exactly
-        const float2 f01 = __ffma2_rn(ex2, __fadd2_rn(X.y01, nay2), __fmul2_rn(ney2, __fadd2_rn(X.x01, nax2)));
-        const float2 f23 = __ffma2_rn(ex2, __fadd2_rn(X.y23, nay2), __fmul2_rn(ney2, __fadd2_rn(X.x23, nax2)));
+        float2 f01, f23;
+        pk_side_line(X, Y, k, f01, f23);
         f[k][0] = f01.x; f[k][1] = f01.y; f[k][2] = f23.x; f[k][3] = f23.y;
     }
 }
 
-// One pass of the assembly: the portions of X's edges inside Y, added to A2
-// (twice the area) and to g (gradient of X's rigid pose about centre ctr).
-// f holds X's vertices against Y's lines.  Per vertex, a 4-bit mask of the
-// lines it is outside of decides most edges without arithmetic: an edge
-// with both ends outside one line is empty, an edge with neither end
-// outside any line is whole, and only the lines it crosses get a crossing
-// parameter.  Returns false when some line of Y has every vertex of X
-// outside (separating axis: the pieces are disjoint).  KEEP_SAME_DIR: a
-// collinear edge of X is kept when it runs the same way as Y's (X = Q) or
-// always dropped (X = P).
-template <bool KEEP_SAME_DIR>
-__device__ __forceinline__ bool pk_clip_pass(const float2 (&X)[4], bool x_tri, const float2 (&Y)[4], bool y_tri,
-                                             const float (&f)[4][4], float2 ctr, float& A2, float3& g)
+// Whether some line of Y has every vertex of X on its outer side, by more than
+// tol: f[k][v] < -tol for all v, with the side values the clipper sees.
+__device__ __forceinline__ bool pk_line_separates(const PkQuad& X, const PkQuad& Y, float tol)
 {
+    float m = 3.4e38f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        float2 f01, f23;
+        pk_side_line(X, Y, k, f01, f23);
+        m = fminf(m, fmaxf(fmaxf(f01.x, f01.y), fmaxf(f23.x, f23.y)));
+    }
+    return m < -tol;   // the degenerate fourth line of a triangle gives 0: it separates nothing
+}
+
+// Approximate a / b, as __fdividef but with subnormals taken as zero: the same
+// value wherever a, b and a / b are normal, without __fdividef's scaling of
+// tiny and huge divisors (3 % of the cost kernel).  A crossing parameter below
+// 1e-38 is zero to everything computed from it.
+__device__ __forceinline__ float pk_quotient(float a, float b)
+{
+    float q;
+    asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(q) : "f"(a), "f"(b));
+    return q;
+}
+
+// Adds the part [tin, tout] of the edge a -> b to A2 (twice the area) and to g
+// (gradient of the rigid pose about centre ctr).
+__device__ __forceinline__ void pk_edge_part(float2 a, float2 b, float tin, float tout, float2 ctr, float& A2, float3& g)
+{
+    const float dt = tout - tin;
+    const float2 e = make_float2(b.x - a.x, b.y - a.y);
+    A2 += dt * pk_cross(a, b);
+    const float2 N = make_float2(dt * e.y, -dt * e.x);
+    const float tm = 0.5f * (tin + tout);
+    const float2 m = make_float2(a.x + tm * e.x - ctr.x, a.y + tm * e.y - ctr.y);
+    g.x += N.x;
+    g.y += N.y;
+    g.z += pk_cross(m, N);
+}
+
+// One pass of the assembly: the portions of X's edges inside Y, added to A2 and
+// g.  This form serves pieces with a vertex within the tolerance of a line of
+// the other (rare, so out of line): per vertex, 4-bit masks of the lines it is
+// outside of and near, from which collinear edges are found.  KEEP_SAME_DIR: a
+// collinear edge of X is kept when it runs the same way as Y's (X = Q) or always
+// dropped (X = P).  Returns (A2, g).
+template <bool KEEP_SAME_DIR>
+__device__ __noinline__ float4 pk_clip_near(const PkQuad XQ, bool x_tri, const PkQuad YQ, bool y_tri, float2 ctr,
+                                            float A2, float3 g)
+{
+    const float2 X[4] = {pk_qv(XQ, 0), pk_qv(XQ, 1), pk_qv(XQ, 2), pk_qv(XQ, 3)};
+    const float2 Y[4] = {pk_qv(YQ, 0), pk_qv(YQ, 1), pk_qv(YQ, 2), pk_qv(YQ, 3)};
+    float f[4][4];
+    pk_side_values_q(XQ, YQ, f);
     const float tiny = c_geom.coll_tiny;
     const unsigned lines = y_tri ? 0x7u : 0xFu;
-    unsigned out[4], nearm[4] = {0u, 0u, 0u, 0u};
-    float mn = 3.4e38f;   // smallest |f| against Y's real lines
+    unsigned out[4], nearm[4];   // per vertex, a bit per line: outside it, near it
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
-        unsigned o = 0;
+        unsigned o = 0, nm = 0;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             o |= (unsigned)(f[k][v] < 0.f) << k;
-            mn = fminf(mn, (k == 3 && y_tri) ? 3.4e38f : fabsf(f[k][v]));
+            nm |= (unsigned)(fabsf(f[k][v]) <= tiny) << k;
         }
         out[v] = o & lines;
-    }
-    if (out[0] & out[1] & out[2] & out[3]) return false;
-    if (mn <= tiny) {
-        // some vertex lies within the tolerance of a line: the per-vertex
-        // masks of near lines (rarely needed, so built only here)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            unsigned nm = 0;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) nm |= (unsigned)(fabsf(f[k][v]) <= tiny) << k;
-            nearm[v] = nm & lines;
-        }
+        nearm[v] = nm & lines;
     }
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
@@ -265,31 +293,74 @@ __device__ __forceinline__ bool pk_clip_pass(const float2 (&X)[4], bool x_tri, c
                 }
             }
         }
-        // the part [tin, tout] of the edge, by selects: a warp's lanes cross
-        // different lines, so nearly every branch here would be taken by some
         const unsigned oa = out[v] & ~skip, ob = out[vb] & ~skip;
         float tin = 0.f, tout = 1.f;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const float fa = f[k][v], fb = f[k][vb];
-            const float t = __fdividef(fa, fa - fb);    // meaningful where the edge crosses line k
+            const float t = pk_quotient(fa, fa - fb);    // meaningful where the edge crosses line k
             tin = fmaxf(tin, (oa >> k) & 1u ? t : 0.f);     // entering
             tout = fminf(tout, (ob >> k) & 1u ? t : 1.f);   // leaving
         }
         const bool part = !empty && !(oa & ob) && tin < tout;
-        const float dt = part ? tout - tin : 0.f;
-        const float2 e = make_float2(b.x - a.x, b.y - a.y);
-        A2 += dt * pk_cross(a, b);
-        const float2 N = make_float2(dt * e.y, -dt * e.x);
-        const float tm = part ? 0.5f * (tin + tout) : 0.f;   // finite, so an empty part adds zeros
-        const float2 m = make_float2(a.x + tm * e.x - ctr.x, a.y + tm * e.y - ctr.y);
-        g.x += N.x;
-        g.y += N.y;
-        g.z += pk_cross(m, N);
+        if (part) pk_edge_part(a, b, tin, tout, ctr, A2, g);
     }
-    return true;
+    return make_float4(A2, g.x, g.y, g.z);
 }
 
+// The pass for all other pieces.  Line by line of Y: the vertices' side values,
+// their quotients along X's four edges, and per edge the largest entering and
+// the smallest leaving parameter.  Whether a quotient counts is put in by
+// arithmetic, with s = 1 for a vertex outside the line and 0 inside: t s is t
+// or 0 (an infinite t gives NaN, which the minima and maxima ignore), t s +
+// (1 - s) is t or 1.  Compares and selects share one half-rate pipe, which was
+// the busiest (51 %) with them; multiplications have another to themselves.  An
+// edge outside one line at both ends has tin >= tout by the same quotient.
+template <bool KEEP_SAME_DIR>
+__device__ __forceinline__ void pk_clip_pass(const PkQuad& X, bool x_tri, const PkQuad& Y, bool y_tri, float2 ctr,
+                                             float& A2, float3& g)
+{
+    float tin[4] = {0.f, 0.f, 0.f, 0.f}, tout[4] = {1.f, 1.f, 1.f, 1.f};
+    float mn = 3.4e38f;   // smallest |f| against Y's real lines
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        float2 f01, f23;
+        pk_side_line(X, Y, k, f01, f23);
+        const float f[4] = {f01.x, f01.y, f23.x, f23.y};
+        float s[4], r[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            s[v] = f[v] < 0.f ? 1.f : 0.f;
+            r[v] = 1.f - s[v];
+        }
+        const float m = fminf(fminf(fabsf(f[0]), fabsf(f[1])), fminf(fabsf(f[2]), fabsf(f[3])));
+        mn = fminf(mn, k == 3 && y_tri ? 3.4e38f : m);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int n = (e + 1) & 3;
+            const float t = pk_quotient(f[e], f[e] - f[n]);
+            tin[e] = fmaxf(tin[e], t * s[e]);
+            tout[e] = fminf(tout[e], fmaf(t, s[n], r[n]));
+        }
+    }
+    if (mn <= c_geom.coll_tiny) {
+        const float4 q = pk_clip_near<KEEP_SAME_DIR>(X, x_tri, Y, y_tri, ctr, A2, g);
+        A2 = q.x;
+        g = make_float3(q.y, q.z, q.w);
+        return;
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const bool part = tin[e] < tout[e] && !(e == 3 && x_tri);
+        // an empty part becomes [0, 0]: finite, so it adds zeros
+        pk_edge_part(pk_qv(X, e), pk_qv(X, (e + 1) & 3), part ? tin[e] : 0.f, part ? tout[e] : 0.f, ctr, A2, g);
+    }
+}
+
+// CHECK: the pieces may be separated by one of their lines (then nothing
+// overlaps, and the clipper's rounding is kept from finding otherwise); without
+// it the caller has tested that.
+template <bool CHECK>
 __device__ __forceinline__ void pk_piece_area_grad_q(const PkQuad& PQ, bool p_tri, const PkQuad& QQ, bool q_tri,
                                                      float2 d, float& area, float3& gP, float3& gQ)
 {
@@ -297,16 +368,9 @@ __device__ __forceinline__ void pk_piece_area_grad_q(const PkQuad& PQ, bool p_tr
     gP = make_float3(0.f, 0.f, 0.f);
     gQ = make_float3(0.f, 0.f, 0.f);
     area = 0.f;
-    const float2 P[4] = {pk_qv(PQ, 0), pk_qv(PQ, 1), pk_qv(PQ, 2), pk_qv(PQ, 3)};
-    const float2 Q[4] = {pk_qv(QQ, 0), pk_qv(QQ, 1), pk_qv(QQ, 2), pk_qv(QQ, 3)};
-    float f[4][4];
-    pk_side_values_q(PQ, QQ, f);
-    if (!pk_clip_pass<false>(P, p_tri, Q, q_tri, f, make_float2(0.f, 0.f), A2, gP)) return;
-    pk_side_values_q(QQ, PQ, f);
-    if (!pk_clip_pass<true>(Q, q_tri, P, p_tri, f, d, A2, gQ)) {
-        gP = make_float3(0.f, 0.f, 0.f);
-        return;
-    }
+    if (CHECK && (pk_line_separates(PQ, QQ, 0.f) || pk_line_separates(QQ, PQ, 0.f))) return;
+    pk_clip_pass<false>(PQ, p_tri, QQ, q_tri, make_float2(0.f, 0.f), A2, gP);
+    pk_clip_pass<true>(QQ, q_tri, PQ, p_tri, d, A2, gQ);
     area = 0.5f * A2;
     if (!(area > 0.f)) {   // empty or numerically vanishing overlap
         area = 0.f;
@@ -319,7 +383,7 @@ __device__ __forceinline__ void pk_piece_area_grad(const float2 (&P)[4], bool p_
                                                    const float2 (&Q)[4], bool q_tri, float2 d,
                                                    float& area, float3& gP, float3& gQ)
 {
-    pk_piece_area_grad_q(pk_quad(P), p_tri, pk_quad(Q), q_tri, d, area, gP, gQ);
+    pk_piece_area_grad_q<true>(pk_quad(P), p_tri, pk_quad(Q), q_tri, d, area, gP, gQ);
 }
 
 // ---------------------------------------------------------------------------
@@ -529,18 +593,6 @@ __device__ __forceinline__ int pk_is_near(float4 A, float4 B, float cutoff)
     return __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)) <= cutoff;
 }
 
-// Whether some line of Y has every vertex of X on its outer side, by more than
-// tol: f[k][v] < -tol for all v, with the side values pk_clip_pass sees.
-__device__ __forceinline__ bool pk_line_separates(const PkQuad& X, const PkQuad& Y, float tol)
-{
-    float f[4][4];
-    pk_side_values_q(X, Y, f);
-    float m = 3.4e38f;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) m = fminf(m, fmaxf(fmaxf(f[k][0], f[k][1]), fmaxf(f[k][2], f[k][3])));
-    return m < -tol;   // the degenerate fourth line of a triangle gives 0: it separates nothing
-}
-
 // Phase B, LUT: looks up the count near pairs of the list; returns this
 // thread's fixed-point pair total.  filter: the list is a kept near list, so a
 // pair is looked up only if it passes the centre cull now; the kept pairs are
@@ -648,7 +700,7 @@ __device__ __forceinline__ long long pk_process_items(const PkCostSmem& sm, int 
         if (MODE == PK_PAIR_AREA) {
             const PkQuad PQ = pk_load_quad(sm, pi, A.z, A.w, 0.f, 0.f);
             const PkQuad QQ = pk_load_quad(sm, pj, B.z, B.w, d.x, d.y);
-            pk_piece_area_grad_q(PQ, pt, QQ, qt, d, val, gi, gj);
+            pk_piece_area_grad_q<false>(PQ, pt, QQ, qt, d, val, gi, gj);
         } else {
             float2 P[4], Q[4];
             pk_load_piece(sm, pi, A.z, A.w, 0.f, 0.f, P);
