@@ -193,24 +193,61 @@ __device__ __forceinline__ double pk_rsqrt(double a) { return __dsqrt_rn(a); }
 // next reduction.  pk_canon_sum adds each group's per-lane partial in k
 // order, then the groups in order, then a fixed shuffle tree, so the sum
 // depends on N alone, not on blockDim.  red: two buffers of 64 * ngroups
-// entries, alternated by `flip` (one barrier per reduction: a thread can only
+// + 64 entries, alternated by `flip` (one barrier per reduction: a thread can only
 // write a buffer again after the next reduction's barrier, by which time every
 // thread has finished reading it).  All threads call these and all get the
 // result.
 #define PK_CANON_GROUP 128
 #define PK_OWN_LOOP(k, N)                                                                      \
     for (int _g = (int)(threadIdx.x >> 5); _g * PK_CANON_GROUP < (N); _g += (int)(blockDim.x >> 5)) \
-        for (int k = _g * PK_CANON_GROUP + (int)(threadIdx.x & 31);                             \
-             k < min((N), (_g + 1) * PK_CANON_GROUP); k += 32)
+        _Pragma("unroll") for (int _j = 0; _j < PK_CANON_GROUP; _j += 32)                      \
+            if (const int k = _g * PK_CANON_GROUP + (int)(threadIdx.x & 31) + _j; k < (N))
 
 __host__ __device__ inline int pk_canon_groups(int N) { return (N + PK_CANON_GROUP - 1) / PK_CANON_GROUP; }
 
 template <typename T>
 __device__ __forceinline__ T* pk_canon_buf(int ng, T* red, int& flip)
 {
-    T* buf = red + (flip ? 64 * ng : 0);
+    T* buf = red + (flip ? 64 * ng + 64 : 0);
     flip ^= 1;
     return buf;
+}
+
+// The maxima's part of the buffer that pk_canon_buf handed out last.
+template <typename T>
+__device__ __forceinline__ T* pk_canon_max_buf(int ng, T* red, int flip)
+{
+    return red + (flip ? 0 : 64 * ng + 64) + 64 * ng;
+}
+
+// Warp maximum, NaN ignored (redux.sync takes floats on sm_100a).
+__device__ __forceinline__ float pk_warp_max(float v)
+{
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ double pk_warp_max(double v)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(PK_FULL_MASK, v, o));
+    return v;
+}
+
+// The per-lane partials of ng groups added in group order.  The first eight are
+// read together (a group beyond ng adds +0, which changes no sum that started
+// from +0); one after the other each waited for its own load.
+template <typename T>
+__device__ __forceinline__ T pk_canon_groups_sum(const T* buf, int ng)
+{
+    const int lane = threadIdx.x & 31;
+    T v[8], r = T(0);
+#pragma unroll
+    for (int grp = 0; grp < 8; ++grp) v[grp] = grp < ng ? buf[grp * 32 + lane] : T(0);
+#pragma unroll
+    for (int grp = 0; grp < 8; ++grp) r = pk_radd(r, v[grp]);
+    for (int grp = 8; grp < ng; ++grp) r = pk_radd(r, buf[grp * 32 + lane]);
+    return r;
 }
 
 // Second half of a canonical sum: barrier, the groups' per-lane partials in
@@ -218,11 +255,19 @@ __device__ __forceinline__ T* pk_canon_buf(int ng, T* red, int& flip)
 template <typename T>
 __device__ __forceinline__ T pk_canon_finish(const T* buf, int ng)
 {
-    const int lane = threadIdx.x & 31;
     __syncthreads();
-    T r = T(0);
-    for (int grp = 0; grp < ng; ++grp) r = pk_radd(r, buf[grp * 32 + lane]);
-    return pk_warp_sum(r);
+    return pk_warp_sum(pk_canon_groups_sum(buf, ng));
+}
+
+// This lane's partial of one group: its (at most four) elements in k order.
+template <typename T, typename Get>
+__device__ __forceinline__ T pk_canon_partial(int grp, int N, Get get)
+{
+    T s = T(0);
+#pragma unroll
+    for (int j = 0; j < PK_CANON_GROUP; j += 32)
+        if (const int k = grp * PK_CANON_GROUP + (int)(threadIdx.x & 31) + j; k < N) s = pk_radd(s, get(k));
+    return s;
 }
 
 template <typename T, typename Get>
@@ -232,55 +277,63 @@ __device__ __forceinline__ T pk_canon_sum(int N, Get get, T* red, int& flip)
     const int nw = blockDim.x >> 5;
     const int ng = pk_canon_groups(N);
     T* buf = pk_canon_buf(ng, red, flip);
-    for (int grp = warp; grp < ng; grp += nw) {
-        T s = T(0);
-        const int end = min(N, (grp + 1) * PK_CANON_GROUP);
-        for (int k = grp * PK_CANON_GROUP + lane; k < end; k += 32) s = pk_radd(s, get(k));
-        buf[grp * 32 + lane] = s;
-    }
+    for (int grp = warp; grp < ng; grp += nw) buf[grp * 32 + lane] = pk_canon_partial<T>(grp, N, get);
     return pk_canon_finish(buf, ng);
 }
 
-// Two canonical sums with one barrier; each is bit-identical to its own
-// pk_canon_sum.
-template <typename T, typename Get>
-__device__ __forceinline__ void pk_canon_sum2(int N, Get get, T* red, int& flip, T& r0, T& r1)
+// NS canonical sums (each bit-identical to its own pk_canon_sum) and NM maxima
+// of absolute values (a maximum does not depend on the order; it starts from 0)
+// with one barrier.  get(k, s, m) gives the NS addends and NM values of element
+// k.  NS * ng * 32 + NM * warps entries of one buffer (64 ng of them).
+template <int NS, int NM, typename T, typename Get>
+__device__ __forceinline__ void pk_canon_reduce(int N, Get get, T* red, int& flip, T (&rs)[NS], T (&rm)[NM])
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nw = blockDim.x >> 5;
     const int ng = pk_canon_groups(N);
     T* buf = pk_canon_buf(ng, red, flip);
+    T* mbuf = pk_canon_max_buf(ng, red, flip);
+    T m[NM];
+#pragma unroll
+    for (int i = 0; i < NM; ++i) m[i] = T(0);
     for (int grp = warp; grp < ng; grp += nw) {
-        T s0 = T(0), s1 = T(0);
-        const int end = min(N, (grp + 1) * PK_CANON_GROUP);
-        for (int k = grp * PK_CANON_GROUP + lane; k < end; k += 32) {
-            T a, b;
-            get(k, a, b);
-            s0 = pk_radd(s0, a);
-            s1 = pk_radd(s1, b);
-        }
-        buf[grp * 32 + lane] = s0;
-        buf[(ng + grp) * 32 + lane] = s1;
+        T s[NS];
+#pragma unroll
+        for (int i = 0; i < NS; ++i) s[i] = T(0);
+#pragma unroll
+        for (int j = 0; j < PK_CANON_GROUP; j += 32)
+            if (const int k = grp * PK_CANON_GROUP + lane + j; k < N) {
+                T es[NS], em[NM];
+                get(k, es, em);
+#pragma unroll
+                for (int i = 0; i < NS; ++i) s[i] = pk_radd(s[i], es[i]);
+#pragma unroll
+                for (int i = 0; i < NM; ++i) m[i] = fmax(m[i], em[i]);
+            }
+#pragma unroll
+        for (int i = 0; i < NS; ++i) buf[(i * ng + grp) * 32 + lane] = s[i];
+    }
+#pragma unroll
+    for (int i = 0; i < NM; ++i) {
+        m[i] = pk_warp_max(m[i]);
+        if (lane == 0) mbuf[32 * i + warp] = m[i];
     }
     __syncthreads();
-    T a = T(0), b = T(0);
-    for (int grp = 0; grp < ng; ++grp) {
-        a = pk_radd(a, buf[grp * 32 + lane]);
-        b = pk_radd(b, buf[(ng + grp) * 32 + lane]);
-    }
-    r0 = pk_warp_sum(a);
-    r1 = pk_warp_sum(b);
+#pragma unroll
+    for (int i = 0; i < NM; ++i) rm[i] = pk_warp_max(lane < nw ? mbuf[32 * i + lane] : T(0));
+#pragma unroll
+    for (int i = 0; i < NS; ++i) rs[i] = pk_warp_sum(pk_canon_groups_sum(buf + i * ng * 32, ng));
 }
 
-// Maxima of two element functions over the owned elements with one barrier
-// (a maximum does not depend on the order).  Starts from 0: the callers
-// reduce absolute values.
+// Maxima of two element functions over the owned elements with one barrier.
+// Starts from 0: the callers reduce absolute values.
 template <typename T, typename Get>
 __device__ __forceinline__ void pk_canon_max2(int N, Get get, T* red, int& flip, T& r0, T& r1)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nw = blockDim.x >> 5;
-    T* buf = pk_canon_buf(pk_canon_groups(N), red, flip);
+    pk_canon_buf(pk_canon_groups(N), red, flip);   // keeps the buffers alternating
+    T* buf = pk_canon_max_buf(pk_canon_groups(N), red, flip);
     T a = T(0), b = T(0);
     PK_OWN_LOOP(k, N) {
         T u, v;
@@ -288,27 +341,20 @@ __device__ __forceinline__ void pk_canon_max2(int N, Get get, T* red, int& flip,
         a = fmax(a, u);
         b = fmax(b, v);
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        a = fmax(a, __shfl_xor_sync(PK_FULL_MASK, a, o));
-        b = fmax(b, __shfl_xor_sync(PK_FULL_MASK, b, o));
-    }
+    a = pk_warp_max(a);
+    b = pk_warp_max(b);
     if (lane == 0) {
-        buf[2 * warp] = a;
-        buf[2 * warp + 1] = b;
+        buf[warp] = a;
+        buf[32 + warp] = b;
     }
     __syncthreads();
-    for (int w = 0; w < nw; ++w) {
-        a = fmax(a, buf[2 * w]);
-        b = fmax(b, buf[2 * w + 1]);
-    }
-    r0 = a;
-    r1 = b;
+    r0 = pk_warp_max(lane < nw ? buf[lane] : T(0));
+    r1 = pk_warp_max(lane < nw ? buf[32 + lane] : T(0));
 }
 
-// Both buffers of the canonical reductions (2 x 64 per group; a block of at
-// most 32 warps fits the per-warp maxima in one buffer).
-__host__ __device__ inline int pk_canon_red_len(int N) { return 2 * 64 * pk_canon_groups(N); }
+// Both buffers of the canonical reductions: 64 per group (two sums) and 64 for
+// two maxima of at most 32 warps.
+__host__ __device__ inline int pk_canon_red_len(int N) { return 2 * (64 * pk_canon_groups(N) + 64); }
 
 // Bounded wrap of an angle difference into [-pi, pi], following the
 // reference's subtract-2pi loop (pack_cuda_lut.py:289-293) in FP32.  Angles

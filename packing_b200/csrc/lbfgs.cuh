@@ -30,10 +30,13 @@
 // holds its <= 4 elements of q in registers and loads the next history entry
 // while the current dot product is being reduced, so the chain of 2 hlen
 // dependent reductions does not also wait for a memory round trip per step.
-// Both paths perform the same operations in the same order.
+// Both paths perform the same operations in the same order.  Every thread
+// writes the same al[i] and later reads what it wrote: no barrier for it.
+// pg (register path only): the newest entry was appended in this iteration, so
+// it is taken from d t and g - pg, as it was written, and not read back.
 template <typename F>
 __device__ void pk_two_loop(const F* g, F* d, int N, const F* S, const F* Y, const F* ro, int m, int hlen,
-                            int hstart, F Hdiag, F* al, F* red, int& flip)
+                            int hstart, F Hdiag, F* al, F* red, int& flip, const F* pg = nullptr, F t = F(0))
 {
     const int ng = pk_canon_groups(N);
     const int nw = blockDim.x >> 5;
@@ -44,11 +47,10 @@ __device__ void pk_two_loop(const F* g, F* d, int N, const F* S, const F* Y, con
             const F* s = S + (size_t)slot * N;
             const F* y = Y + (size_t)slot * N;
             const F a = pk_rmul(pk_canon_sum<F>(N, [&](int k) { return pk_rmul(s[k], d[k]); }, red, flip), ro[slot]);
-            if (threadIdx.x == 0) al[i] = a;
+            al[i] = a;
             PK_OWN_LOOP(k, N) d[k] = pk_rsub(d[k], pk_rmul(y[k], a));
         }
         PK_OWN_LOOP(k, N) d[k] = pk_rmul(d[k], Hdiag);
-        __syncthreads();   // al[] visible
         for (int i = 0; i < hlen; ++i) {
             const int slot = (hstart + i) % m;
             const F* s = S + (size_t)slot * N;
@@ -83,7 +85,16 @@ __device__ void pk_two_loop(const F* g, F* d, int N, const F* S, const F* Y, con
     int slot = hlen > 0 ? (hstart + hlen - 1) % m : 0;
     const F* pcur = S + (size_t)slot * N + k0;
     if (hlen > 0) {
-        PK_TL_FETCH(sc, yc, pcur)
+        if (pg) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (j < nv) {
+                    sc[j] = pk_rmul(d[k0 + 32 * j], t);
+                    yc[j] = pk_rsub(g[k0 + 32 * j], pg[k0 + 32 * j]);
+                }
+        } else {
+            PK_TL_FETCH(sc, yc, pcur)
+        }
         rc = ro[slot];
     }
     for (int i = hlen - 1; i >= 0; --i) {
@@ -102,7 +113,7 @@ __device__ void pk_two_loop(const F* g, F* d, int N, const F* S, const F* Y, con
             buf[warp * 32 + lane] = p;
         }
         const F a = pk_rmul(pk_canon_finish(buf, ng), rc);
-        if (threadIdx.x == 0) al[i] = a;
+        al[i] = a;
 #pragma unroll
         for (int j = 0; j < 4; ++j) q[j] = pk_rsub(q[j], pk_rmul(yc[j], a));
         if (i > 0) {   // entry 0 stays in hand: the second loop starts with it
@@ -115,7 +126,6 @@ __device__ void pk_two_loop(const F* g, F* d, int N, const F* S, const F* Y, con
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) q[j] = pk_rmul(q[j], Hdiag);
-    __syncthreads();   // al[] visible
     // second loop: oldest entry first; the slot steps up with wraparound
     for (int i = 0; i < hlen; ++i) {
         const int nslot = slot == m - 1 ? 0 : slot + 1;
@@ -159,6 +169,32 @@ __device__ __forceinline__ void pk_own_absmax2(int N, const F* v, F scale, const
         a = (F)fabs(pk_rmul(v[k], scale));
         b = (F)fabs(pk_rmul(w[k], wscale));
     }, red, flip, rv, rw);
+}
+
+// After a step t d from gradient pg to g, with one barrier: y.s and y.y with
+// y = g - pg, s = t d (the curvature), max|g| and max|t d| (the stop tests).
+template <typename F>
+__device__ __forceinline__ void pk_step_reduce(int N, const F* g, const F* pg, const F* d, F t, F* red, int& flip,
+                                               F (&sums)[2], F (&maxima)[2])
+{
+    pk_canon_reduce<2, 2, F>(N, [&](int k, F (&s)[2], F (&m)[2]) {
+        const F y = pk_rsub(g[k], pg[k]), st = pk_rmul(d[k], t);
+        s[0] = pk_rmul(y, st);
+        s[1] = pk_rmul(y, y);
+        m[0] = (F)fabs(g[k]);
+        m[1] = (F)fabs(st);
+    }, red, flip, sums, maxima);
+}
+
+// Of a direction, with one barrier: g.d and max|t d|.
+template <typename F>
+__device__ __forceinline__ void pk_direction_reduce(int N, const F* g, const F* d, F t, F* red, int& flip,
+                                                    F (&gtd)[1], F (&pc)[1])
+{
+    pk_canon_reduce<1, 1, F>(N, [&](int k, F (&s)[1], F (&m)[1]) {
+        s[0] = pk_rmul(g[k], d[k]);
+        m[0] = (F)fabs(pk_rmul(d[k], t));
+    }, red, flip, gtd, pc);
 }
 
 // ---------------------------------------------------------------------------
@@ -207,13 +243,10 @@ __global__ void pk_lbfgs_direction_kernel(PkLbfgsState<F> s, int n_iter, F lr, F
     } else {
         t = lr;
     }
-    if (has_max_step) {
-        F pc, unused;
-        pk_own_absmax2<F>(N, d, t, d, t, red, flip, pc, unused);
-        if (pc > max_step) t = t * (max_step / pc);
-    }
-    const F gtd = pk_canon_sum<F>(N, [&](int k) { return pk_rmul(g[k], d[k]); }, red, flip);
-    if (gtd > -tol_change) active = 0;
+    F gtd[1], pc[1];
+    pk_direction_reduce<F>(N, g, d, t, red, flip, gtd, pc);
+    if (has_max_step && pc[0] > max_step) t = t * (max_step / pc[0]);
+    if (gtd[0] > -tol_change) active = 0;
     if (threadIdx.x == 0) {
         s.t[b] = t;
         s.H[b] = Hd;
@@ -251,13 +284,10 @@ __global__ void pk_lbfgs_update_kernel(PkLbfgsState<F> s, int n_iter, F tol_grad
     const F t = s.t[b];
     int active = s.active[b];
     int evals = s.evals[b] + 1;
+    F sums[2], maxima[2];
+    pk_step_reduce<F>(N, g, pg, d, t, red, flip, sums, maxima);
+    const F ys = sums[0], yy = sums[1], gmax = maxima[0], pc = maxima[1];
     if (n_iter > 1) {
-        F ys, yy;
-        pk_canon_sum2<F>(N, [&](int k, F& a, F& c) {
-            const F y = pk_rsub(g[k], pg[k]);
-            a = pk_rmul(y, pk_rmul(d[k], t));
-            c = pk_rmul(y, y);
-        }, red, flip, ys, yy);
         if (active && ys > (F)1e-10) {
             int hl = s.hlen[b], hs = s.hstart[b], slot;
             if (hl < m) { slot = (hs + hl) % m; ++hl; }
@@ -276,8 +306,6 @@ __global__ void pk_lbfgs_update_kernel(PkLbfgsState<F> s, int n_iter, F tol_grad
             }
         }
     }
-    F gmax, pc;
-    pk_own_absmax2<F>(N, g, (F)1, d, t, red, flip, gmax, pc);
     if (threadIdx.x == 0) {
         if (gmax <= tol_grad) active = 0;
         if (evals >= max_eval) active = 0;
@@ -413,6 +441,7 @@ __device__ bool pk_relax_iterate(float* x, float* g, float* pg, float* d, float*
     const int N = 3 * n + 3;
     const int m = prm.history;
     bool need_eval = !resume, final_pending = false, want_grad = true, skip_update = resume;
+    bool fresh = false;   // the newest history entry is this iteration's
     // Kept near lists when the step bound lets a list serve at least four
     // evaluations (every coordinate moves at most max_step per step); the
     // first evaluation of this call builds one.
@@ -438,30 +467,24 @@ __device__ bool pk_relax_iterate(float* x, float* g, float* pg, float* d, float*
             } else {
                 // after a step (:632-724)
                 ++v.evals;
-                if (v.it > 1) {
+                float sums[2], maxima[2];
+                pk_step_reduce<float>(N, g, pg, d, v.t, red, flip, sums, maxima);
+                const float ys = sums[0], yy = sums[1], gmax = maxima[0], pc = maxima[1];
+                if (v.it > 1 && ys > 1e-10f) {
+                    int slot;
+                    if (v.hlen < m) { slot = (v.hstart + v.hlen) % m; ++v.hlen; }
+                    else { slot = v.hstart; v.hstart = (v.hstart + 1) % m; }
+                    float* Sd = S + (size_t)slot * N;
+                    float* Yd = Y + (size_t)slot * N;
                     const float t = v.t;
-                    float ys, yy;
-                    pk_canon_sum2<float>(N, [&](int k, float& a, float& c) {
-                        const float y = pk_rsub(g[k], pg[k]);
-                        a = pk_rmul(y, pk_rmul(d[k], t));
-                        c = pk_rmul(y, y);
-                    }, red, flip, ys, yy);
-                    if (ys > 1e-10f) {
-                        int slot;
-                        if (v.hlen < m) { slot = (v.hstart + v.hlen) % m; ++v.hlen; }
-                        else { slot = v.hstart; v.hstart = (v.hstart + 1) % m; }
-                        float* Sd = S + (size_t)slot * N;
-                        float* Yd = Y + (size_t)slot * N;
-                        PK_OWN_LOOP(k, N) {
-                            Yd[k] = pk_rsub(g[k], pg[k]);
-                            Sd[k] = pk_rmul(d[k], t);
-                        }
-                        v.H = ys / yy;
-                        if (threadIdx.x == 0) ro[slot] = 1.f / ys;
+                    PK_OWN_LOOP(k, N) {
+                        Yd[k] = pk_rsub(g[k], pg[k]);
+                        Sd[k] = pk_rmul(d[k], t);
                     }
+                    v.H = ys / yy;
+                    ro[slot] = 1.f / ys;   // every thread writes it, and reads what it wrote
+                    fresh = true;
                 }
-                float gmax, pc;
-                pk_own_absmax2<float>(N, g, 1.f, d, v.t, red, flip, gmax, pc);
                 if (gmax <= prm.tol_grad) v.active = 0;
                 if (v.evals >= prm.max_eval) v.active = 0;
                 if (pc <= prm.tol_change) v.active = 0;
@@ -481,7 +504,8 @@ __device__ bool pk_relax_iterate(float* x, float* g, float* pg, float* d, float*
             PK_OWN_LOOP(k, N) d[k] = -g[k];
             v.H = 1.f;
         } else {
-            pk_two_loop<float>(g, d, N, S, Y, ro, m, v.hlen, v.hstart, v.H, al, red, flip);
+            pk_two_loop<float>(g, d, N, S, Y, ro, m, v.hlen, v.hstart, v.H, al, red, flip, fresh ? pg : nullptr, v.t);
+            fresh = false;
             hist_streamed += (unsigned long long)v.hlen;
         }
         PK_OWN_LOOP(k, N) pg[k] = g[k];
@@ -494,14 +518,11 @@ __device__ bool pk_relax_iterate(float* x, float* g, float* pg, float* d, float*
         } else {
             t = prm.lr;
         }
-        if (prm.has_max_step) {
-            float pc, unused;
-            pk_own_absmax2<float>(N, d, t, d, t, red, flip, pc, unused);
-            if (pc > prm.max_step) t = t * (prm.max_step / pc);
-        }
+        float gtd[1], pc[1];
+        pk_direction_reduce<float>(N, g, d, t, red, flip, gtd, pc);
+        if (prm.has_max_step && pc[0] > prm.max_step) t = t * (prm.max_step / pc[0]);
         v.t = t;
-        const float gtd = pk_canon_sum<float>(N, [&](int k) { return pk_rmul(g[k], d[k]); }, red, flip);
-        if (gtd > -prm.tol_change) { v.active = 0; --v.it; return true; }
+        if (gtd[0] > -prm.tol_change) { v.active = 0; --v.it; return true; }
         PK_OWN_LOOP(k, N) x[k] = pk_radd(x[k], pk_rmul(t, d[k]));
         need_eval = v.it != prm.max_iter;
         if (!need_eval && prm.final_eval) {
