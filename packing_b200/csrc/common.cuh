@@ -250,6 +250,14 @@ __device__ __forceinline__ T pk_canon_groups_sum(const T* buf, int ng)
     return r;
 }
 
+// Barrier of the first nw warps of the block (named barrier 1; all of those
+// warps, and only those, call it).
+__device__ __forceinline__ void pk_warps_barrier(int nw)
+{
+    if (nw == 1) __syncwarp();
+    else asm volatile("bar.sync 1, %0;" ::"r"(32 * nw) : "memory");
+}
+
 // Second half of a canonical sum: barrier, the groups' per-lane partials in
 // group order, then the shuffle tree.  buf holds ng * 32 partials.
 template <typename T>

@@ -30,13 +30,16 @@
 // holds its <= 4 elements of q in registers and loads the next history entry
 // while the current dot product is being reduced, so the chain of 2 hlen
 // dependent reductions does not also wait for a memory round trip per step.
+// Warps without a group leave at once; the rest meet at a barrier of their own.
+// The number of reductions is even, so the caller's flip is unchanged (its next
+// reduction writes the buffer that the last one here did not).
 // Both paths perform the same operations in the same order.  Every thread
 // writes the same al[i] and later reads what it wrote: no barrier for it.
 // pg (register path only): the newest entry was appended in this iteration, so
 // it is taken from d t and g - pg, as it was written, and not read back.
 template <typename F>
 __device__ void pk_two_loop(const F* g, F* d, int N, const F* S, const F* Y, const F* ro, int m, int hlen,
-                            int hstart, F Hdiag, F* al, F* red, int& flip, const F* pg = nullptr, F t = F(0))
+                            int hstart, F Hdiag, F* al, F* red, int flip, const F* pg = nullptr, F t = F(0))
 {
     const int ng = pk_canon_groups(N);
     const int nw = blockDim.x >> 5;
@@ -62,7 +65,8 @@ __device__ void pk_two_loop(const F* g, F* d, int N, const F* S, const F* Y, con
         return;
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int k0 = warp * PK_CANON_GROUP + lane;   // >= N for a warp that owns no group
+    if (warp >= ng) return;   // owns no element; the others' barrier counts ng warps
+    const int k0 = warp * PK_CANON_GROUP + lane;
     // this lane's elements are k0 + 32 j for j < nv
     const int nv = k0 < N ? min(4, (N - k0 + 31) >> 5) : 0;
     const ptrdiff_t yoff = Y - S;                  // Y entry = S entry + yoff
@@ -105,14 +109,13 @@ __device__ void pk_two_loop(const F* g, F* d, int N, const F* S, const F* Y, con
             rn = ro[nslot];
         }
         F* buf = pk_canon_buf(ng, red, flip);
-        if (warp < ng) {
-            F p = F(0);
+        F p = F(0);
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (j < nv) p = pk_radd(p, pk_rmul(sc[j], q[j]));
-            buf[warp * 32 + lane] = p;
-        }
-        const F a = pk_rmul(pk_canon_finish(buf, ng), rc);
+        for (int j = 0; j < 4; ++j)
+            if (j < nv) p = pk_radd(p, pk_rmul(sc[j], q[j]));
+        buf[warp * 32 + lane] = p;
+        pk_warps_barrier(ng);
+        const F a = pk_rmul(pk_warp_sum(pk_canon_groups_sum(buf, ng)), rc);
         al[i] = a;
 #pragma unroll
         for (int j = 0; j < 4; ++j) q[j] = pk_rsub(q[j], pk_rmul(yc[j], a));
@@ -135,14 +138,13 @@ __device__ void pk_two_loop(const F* g, F* d, int N, const F* S, const F* Y, con
             rn = ro[nslot];
         }
         F* buf = pk_canon_buf(ng, red, flip);
-        if (warp < ng) {
-            F p = F(0);
+        F p = F(0);
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (j < nv) p = pk_radd(p, pk_rmul(yc[j], q[j]));
-            buf[warp * 32 + lane] = p;
-        }
-        const F be = pk_rmul(pk_canon_finish(buf, ng), rc);
+        for (int j = 0; j < 4; ++j)
+            if (j < nv) p = pk_radd(p, pk_rmul(yc[j], q[j]));
+        buf[warp * 32 + lane] = p;
+        pk_warps_barrier(ng);
+        const F be = pk_rmul(pk_warp_sum(pk_canon_groups_sum(buf, ng)), rc);
         const F c = pk_rsub(al[i], be);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
