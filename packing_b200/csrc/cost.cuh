@@ -18,6 +18,8 @@
 #pragma once
 #include "common.cuh"
 
+#include <atomic>
+
 struct PkCostSmem {
     float4* pose;       // [n_max] x, y, cos, sin
     float* theta;       // [n_max]
@@ -1310,15 +1312,37 @@ __global__ void __launch_bounds__(256, MODE == PK_PAIR_LUT ? 4 : 3) pk_cost_kern
     if (threadIdx.x == 0) cost[e] = (float)tot;
 }
 
-// Threads per CTA as a function of the instance size only (so a packing's
-// result never depends on what else is in the batch).
-static inline int pk_cost_threads(int n_max)
+// Multiprocessors of the current device (0 on error), asked once per device.
+static int pk_sm_count()
 {
-    if (n_max <= 48) return 64;
-    if (n_max <= 128) return 128;
-    return 256;
+    static std::atomic<int> cache[64];
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    sms = cache[dev].load(std::memory_order_relaxed);
+    if (sms == 0 && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
+        cache[dev].store(sms, std::memory_order_relaxed);
+    return sms;
 }
 
+// Threads per CTA.  The results do not depend on them (fixed-point sums,
+// reductions whose order the packing alone fixes).  A batch that fills the GPU
+// gets about one thread per tree.  One that does not is as slow as its slowest
+// CTA, so its CTAs grow, up to 3 x 256 threads per SM over the whole batch and
+// to where more threads stop helping (n <= 24: 128, n <= 64: 192).  20
+// iterations of 8 packings, us with 64 / 128 / 192 / 256 threads: n = 20 299 /
+// 245 / 246 / 249, n = 50 486 / 358 / 320 / 310, n = 100 964 / 538 / 452 / 397;
+// 256 packings: n = 20 358 / 309 / 281 / 286, n = 50 566 / 410 / 364 / 388,
+// n = 100 1109 / 654 / 550 / 512.
+static inline int pk_cost_threads(int n_max, int count)
+{
+    const int full = n_max <= 48 ? 64 : (n_max <= 128 ? 128 : 256);
+    const int most = n_max <= 24 ? 128 : (n_max <= 64 ? 192 : 256);
+    const int sms = pk_sm_count() > 0 ? pk_sm_count() : 1;
+    const int per_sm = count > 0 ? (count + sms - 1) / sms : 1;   // CTAs an SM has to hold
+    const int room = (768 / per_sm) & ~31;
+    const int wide = room < most ? room : most;
+    return wide > full ? wide : full;
+}
 
 // count entries of the launch order (all E instances when order is NULL);
 // threads 0 = pk_cost_threads of the size bound.
@@ -1345,7 +1369,7 @@ static int pk_launch_cost(const float* xyt, const int* offsets, const int* order
         if (!L.vals || L.nx < 2 || L.ny < 2 || L.nt < 2)
             return pk_fail(PK_EINVAL, "pk_cost: LUT needs vals and at least 2 points per axis%s");
     }
-    int T = pk_cost_threads(n_max * pk_symmetry(*spec));
+    int T = pk_cost_threads(n_max * pk_symmetry(*spec), count);
     if (threads != 0) {
         if (threads < 32 || threads > 256 || (threads & 31) || 8 * threads < n_max * pk_symmetry(*spec) - 1)
             return pk_fail(PK_EINVAL, "pk_cost: threads must be 0 or a multiple of 32 in [32, 256] with "

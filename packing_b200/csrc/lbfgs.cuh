@@ -614,8 +614,12 @@ __device__ void pk_relax_instance(int e, const float* __restrict__ xyt_in, const
 // relaxes order[b], order[b + G], ...; largest-first orders keep the CTAs'
 // loads even.  Instances are indexed 0 .. E-1 whatever part of the order a
 // launch covers.
-template <int MODE, bool PERSISTENT, bool SYM>
-__global__ void __launch_bounds__(256, 3) pk_relax_kernel(const float* __restrict__ xyt_in, const float* __restrict__ h_in,
+// WIDE: for a batch of at most 512 threads per SM, whose time is that of its
+// slowest CTA: 128 registers instead of 80, so nothing spills (48 x 200 legalisation
+// iterations 25 -> 21 us each, 8 x 50 trees 10 % less; 4096 x 200, where the
+// third CTA per SM is worth as much, 1 % more).
+template <int MODE, bool PERSISTENT, bool SYM, bool WIDE = false>
+__global__ void __launch_bounds__(256, WIDE ? 2 : 3) pk_relax_kernel(const float* __restrict__ xyt_in, const float* __restrict__ h_in,
                                 const int* __restrict__ offsets, const int* __restrict__ order, int count, int E,
                                 int n_max, PkCostSpec spec, PkRelaxParams prm, float* __restrict__ xyt_out,
                                 float* __restrict__ h_out, float* __restrict__ loss_out, int* __restrict__ iters_out,
@@ -717,10 +721,10 @@ static size_t pk_relax_smem_bytes(int n_max, int sym, int cap_near, int cap_item
 // autotuned value) or the default for the instance size.  Any multiple of 32
 // up to 256 gives the same results (every reduction has an order fixed by
 // the instance alone); the near list (8 T pairs) must hold one tree's n_max - 1.
-static int pk_relax_threads(int n_max, int want, int* T, const char* who)
+static int pk_relax_threads(int n_max, int count, int want, int* T, const char* who)
 {
     if (want == 0) {
-        *T = pk_cost_threads(n_max);
+        *T = pk_cost_threads(n_max, count);
         return PK_OK;
     }
     if (want < 32 || want > 256 || (want & 31)) {
@@ -742,12 +746,12 @@ static int pk_relax_threads(int n_max, int want, int* T, const char* who)
 // attribute call (they can then be captured into a CUDA graph).
 static cudaError_t pk_set_smem(const void* fn, int slot, size_t smem)
 {
-    static size_t done[64][32];
+    static size_t done[64][48];
     static std::mutex mu;
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
     if (err != cudaSuccess) return err;
-    if (dev < 0 || dev >= 64 || slot < 0 || slot >= 32) return cudaErrorInvalidValue;
+    if (dev < 0 || dev >= 64 || slot < 0 || slot >= 48) return cudaErrorInvalidValue;
     std::lock_guard<std::mutex> lock(mu);
     if (smem <= done[dev][slot]) return cudaSuccess;
     err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -824,7 +828,7 @@ static int pk_relax_launch(const float* xyt_in, const float* h_in, const int* of
         return pk_fail(PK_EINVAL, "pk_relax: symmetry must be 0, 1, 2 or 4%s");
     const int sym = pk_symmetry(*spec);
     if ((long long)n_max * sym > PK_MAX_TREES) return pk_fail(PK_ERANGE, "pk_relax: more than 1024 phenotype trees%s");
-    rc = pk_relax_threads(n_max * sym, prm->threads, &T, "pk_relax");
+    rc = pk_relax_threads(n_max * sym, E, prm->threads, &T, "pk_relax");
     if (rc) return rc;
     int cap_near, cap_items;
     pk_caps(T, spec->pair_mode, &cap_near, &cap_items);
@@ -832,25 +836,28 @@ static int pk_relax_launch(const float* xyt_in, const float* h_in, const int* of
     cudaStream_t st = (cudaStream_t)stream;
     cudaError_t err = cudaSuccess;
     int grid = count;
+    // every packing of the batch resident at 128 registers (a class of a larger batch shares the SMs)
+    const bool wide = !prm->persistent && E <= pk_sm_count() * (512 / T);
     switch (spec->pair_mode) {
-#define PK_R3(M, P, S)                                                                                   \
+#define PK_R4(M, P, S, W, SLOT)                                                                          \
     {                                                                                                    \
-        err = pk_set_smem((const void*)pk_relax_kernel<M, P, S>, 4 + M + 4 * (P) + 8 * (S), smem);      \
+        err = pk_set_smem((const void*)pk_relax_kernel<M, P, S, W>, SLOT, smem);                         \
         if (err == cudaSuccess && (P))                                                                   \
-            err = pk_resident_grid((const void*)pk_relax_kernel<M, P, S>, T, smem, count, &grid);        \
+            err = pk_resident_grid((const void*)pk_relax_kernel<M, P, S, W>, T, smem, count, &grid);     \
         if (err == cudaSuccess)                                                                          \
-            pk_relax_kernel<M, P, S><<<grid, T, smem, st>>>(xyt_in, h_in, offsets, order, count, E, n_max, *spec, \
-                                                            *prm,                                        \
-                                                            xyt_out, h_out, loss_out, iters_out, work, cap_near, \
-                                                            cap_items);                                  \
+            pk_relax_kernel<M, P, S, W><<<grid, T, smem, st>>>(xyt_in, h_in, offsets, order, count, E, n_max, *spec, \
+                                                               *prm, xyt_out, h_out, loss_out, iters_out, work, \
+                                                               cap_near, cap_items);                     \
+    }
+#define PK_R3(M, S)                                                                                      \
+    {                                                                                                    \
+        if (prm->persistent) PK_R4(M, true, S, false, 8 + M + 8 * (S))                                   \
+        else if (wide) PK_R4(M, false, S, true, 32 + M + 4 * (S))                                        \
+        else PK_R4(M, false, S, false, 4 + M + 8 * (S))                                                  \
     }
 #define PK_R(M)                                                                                          \
     case M:                                                                                              \
-        if (prm->persistent) {                                                                           \
-            if (sym > 1) PK_R3(M, true, true) else PK_R3(M, true, false)                                 \
-        } else {                                                                                         \
-            if (sym > 1) PK_R3(M, false, true) else PK_R3(M, false, false)                               \
-        }                                                                                                \
+        if (sym > 1) PK_R3(M, true) else PK_R3(M, false)                                                 \
         break;
         PK_R(PK_PAIR_NONE)
         PK_R(PK_PAIR_AREA)
@@ -858,6 +865,7 @@ static int pk_relax_launch(const float* xyt_in, const float* h_in, const int* of
         PK_R(PK_PAIR_LUT)
 #undef PK_R
 #undef PK_R3
+#undef PK_R4
         default: return pk_fail(PK_EINVAL, "pk_relax: unknown pair_mode%s");
     }
     if (err != cudaSuccess) return pk_cuda_check(err, "pk_relax attribute");
@@ -899,7 +907,7 @@ extern "C" int pk_relax_jobs(PkJob* jobs, const int* list, int njobs, float* poo
         return pk_fail(PK_EINVAL, "pk_relax_jobs: symmetry must be 0, 1, 2 or 4%s");
     const int sym = pk_symmetry(*spec);
     if ((long long)n_max * sym > PK_MAX_TREES) return pk_fail(PK_ERANGE, "pk_relax_jobs: more than 1024 phenotype trees%s");
-    rc = pk_relax_threads(n_max * sym, prm->threads, &T, "pk_relax_jobs");
+    rc = pk_relax_threads(n_max * sym, njobs, prm->threads, &T, "pk_relax_jobs");
     if (rc) return rc;
     int cap_near, cap_items;
     pk_caps(T, spec->pair_mode, &cap_near, &cap_items);

@@ -220,3 +220,24 @@ def test_relax_into_refuses_short_or_wrong_buffers(cuda):
     with pytest.raises(ValueError):
         relax_into(xyt, h, ok["xyt_out"], ok["h_out"], ok["loss_out"], ok["work"], _spec(), prm,
                    iters_out=torch.empty(E, dtype=torch.int64, device=cuda))
+
+
+@pytest.mark.parametrize("pair,symmetry", [("area", 1), ("sep", 1), ("area", 4)])
+@pytest.mark.parametrize("n", [1, 24, 65, 129])
+def test_small_batches_equal_large_ones(cuda, n, pair, symmetry):
+    """A batch that leaves the GPU idle gets larger CTAs and the 128-register
+    build; a packing's result is the same as in a batch that fills it."""
+    from packing_b200.cost import CostSpec, compound_cost
+    from packing_b200.relax import RelaxParams, relax
+    if n * symmetry > 260:
+        n = 260 // symmetry
+    x = torch.from_numpy(poses(4, n, seed=n)).to(cuda)
+    h = torch.from_numpy(square_h(4, n * symmetry)).to(cuda)
+    spec = CostSpec(pair=pair, symmetry=symmetry, fixed_h=False)
+    prm = RelaxParams(n_iterations=12, history_size=4, max_step=0.01)
+    many = 1600 // 4
+    small = relax(x, h, spec, prm) + compound_cost(x, h, spec)
+    large = relax(x.repeat(many, 1, 1), h.repeat(many, 1), spec, prm)
+    large += compound_cost(x.repeat(many, 1, 1), h.repeat(many, 1), spec)
+    for a, b in zip(small, large):
+        assert torch.equal(a, b[:4]) and torch.equal(a, b[-4:])
