@@ -215,6 +215,8 @@ def _dev_index(device) -> int:
 
 def ensure_init(device: torch.device | int | None = None, geometry: PkGeometry | None = None):
     """pk_init on the given (or current) CUDA device, once per device."""
+    if geometry is None and isinstance(device, torch.device) and device.index in _inited_devices:
+        return   # the usual call, with a tensor's device
     if not torch.cuda.is_available():
         raise PackError("packing_b200 needs a CUDA device; no CPU fallback exists")
     dev = _dev_index(device)
@@ -249,10 +251,29 @@ def check_f32(t: torch.Tensor, name: str, shape: tuple | None = None):
         raise ValueError(f"{name} must have shape {tuple(shape)}, got {tuple(t.shape)}")
 
 
+class _Stay:
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_STAY = _Stay()
+
+
+def on_device(device: torch.device):
+    """Context that makes a CUDA device (with an index, as a tensor's has)
+    current; when it already is, one without the cost of switching."""
+    return _STAY if torch.cuda.current_device() == device.index else torch.cuda.device(device)
+
+
 def stream_handle(stream=None, device=None) -> int:
     """cudaStream_t as int for a torch stream, a cupy-style stream (.ptr),
     an int, or None (torch's current stream)."""
     if stream is None:
+        if isinstance(device, torch.device) and device.index is not None:
+            return torch._C._cuda_getCurrentRawStream(device.index)
         return torch.cuda.current_stream(device).cuda_stream
     if isinstance(stream, int):
         return stream
@@ -264,4 +285,5 @@ def stream_handle(stream=None, device=None) -> int:
 
 
 def ptr(t: torch.Tensor | None):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    """Device address for a void* argument (None: NULL)."""
+    return None if t is None else t.data_ptr()

@@ -12,6 +12,7 @@ from __future__ import annotations
 
 from dataclasses import dataclass
 
+import numpy as np
 import torch
 
 from . import _lib
@@ -44,30 +45,43 @@ def size_classes(sizes_in_order) -> list[SizeClass]:
     order (largest first).  A packing of n trees goes to the class of the
     smallest edge >= n in ``CLASS_TABLE``, whose CTAs have that entry's
     threads."""
-    sz = [int(v) for v in sizes_in_order]
-    if any(sz[k] < sz[k + 1] for k in range(len(sz) - 1)):
+    sz = np.array([int(v) for v in sizes_in_order]) if not isinstance(sizes_in_order, np.ndarray) else sizes_in_order
+    if len(sz) == 0:
+        return []
+    if (sz[:-1] < sz[1:]).any():
         raise ValueError("sizes must be in a largest-first order")
-    out, k = [], 0
-    while k < len(sz):
-        edge = next((e for e in CLASS_EDGES if sz[k] <= e), None)
-        if edge is None:
-            raise ValueError(f"{sz[k]} trees exceeds {CLASS_EDGES[-1]}")
-        lo = max([e for e in CLASS_EDGES if e < edge], default=0)
-        j = k
-        while j < len(sz) and sz[j] > lo:
-            j += 1
-        out.append(SizeClass(start=k, count=j - k, n_max=sz[k], threads=dict(CLASS_TABLE)[edge]))
-        k = j
-    return out
+    if sz[0] > CLASS_EDGES[-1]:
+        raise ValueError(f"{int(sz[0])} trees exceeds {CLASS_EDGES[-1]}")
+    cls = np.searchsorted(np.array(CLASS_EDGES), sz, side="left")   # class of each packing
+    starts = np.concatenate([[0], np.flatnonzero(np.diff(cls)) + 1])
+    ends = np.concatenate([starts[1:], [len(sz)]])
+    return [SizeClass(start=int(a), count=int(b - a), n_max=int(sz[a]), threads=CLASS_TABLE[cls[a]][1])
+            for a, b in zip(starts, ends)]
+
+
+def largest_first(sizes: np.ndarray) -> np.ndarray:
+    """Launch order of these tree counts: largest first, equal ones in order."""
+    return np.argsort(-sizes, kind="stable").astype(np.int32)
 
 
 def ragged_plan(sizes, device=None):
     """(order, classes) for a ragged batch with these tree counts: the
     largest-first launch order as a device int32 tensor and its size
-    classes."""
-    order_h = sorted(range(len(sizes)), key=lambda e: -int(sizes[e]))
-    order = torch.tensor(order_h, dtype=torch.int32, device=device or "cuda")
-    return order, size_classes([int(sizes[e]) for e in order_h])
+    classes (one class of all, with the library's choice of threads, for a
+    batch that leaves the GPU idle)."""
+    sz = np.array([int(s) for s in sizes], dtype=np.int64)
+    order = torch.tensor(largest_first(sz), dtype=torch.int32, device=device or "cuda")
+    classes = size_classes(-np.sort(-sz))   # refuses a tree count beyond the table
+    if len(sz) and not fills_gpu(len(sz), order.device):
+        classes = [SizeClass(0, len(sz), int(sz.max()), 0)]
+    return order, classes
+
+
+def fills_gpu(count: int, device) -> bool:
+    """Whether a batch of this many packings gives every SM of the device more
+    than two.  A smaller one is as slow as its slowest packing: one launch with
+    the library's choice of threads then beats classes sized for throughput."""
+    return count > 2 * torch.cuda.get_device_properties(device).multi_processor_count
 
 
 _side_streams: dict[int, list] = {}

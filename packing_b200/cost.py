@@ -30,24 +30,23 @@ class CostSpec:
     symmetry: int = 1   # 1: every tree given; 2 / 4: genotype of a 180 / 90 degree symmetric packing
 
     def to_c(self) -> _lib.PkCostSpec:
-        s = _lib.PkCostSpec()
-        modes = {"none": _lib.PK_PAIR_NONE, "area": _lib.PK_PAIR_AREA, "sep": _lib.PK_PAIR_SEP,
-                 "lut": _lib.PK_PAIR_LUT}
-        if self.pair not in modes:
-            raise ValueError(f"pair must be one of {sorted(modes)}")
-        s.pair_mode = modes[self.pair]
-        s.w_pair = float(self.w_pair)
-        s.w_boundary = float(self.w_boundary)
-        s.w_area = float(self.w_area)
-        s.fixed_h = int(bool(self.fixed_h))
+        mode = _PAIR_MODES.get(self.pair)
+        if mode is None:
+            raise ValueError(f"pair must be one of {sorted(_PAIR_MODES)}")
         if self.symmetry not in (1, 2, 4):
             raise ValueError("symmetry must be 1, 2 or 4")
-        s.symmetry = int(self.symmetry)
-        if self.pair == "lut":
+        if mode == _lib.PK_PAIR_LUT:
             if self.lut is None:
                 raise ValueError("pair='lut' needs a LookupTable")
-            s.lut = self.lut.c_struct()
-        return s
+            lut = self.lut.c_struct()
+        else:
+            lut = _NO_LUT
+        return _lib.PkCostSpec(mode, float(self.w_pair), float(self.w_boundary), float(self.w_area),
+                               int(bool(self.fixed_h)), lut, int(self.symmetry))
+
+
+_PAIR_MODES = {"none": _lib.PK_PAIR_NONE, "area": _lib.PK_PAIR_AREA, "sep": _lib.PK_PAIR_SEP, "lut": _lib.PK_PAIR_LUT}
+_NO_LUT = _lib.PkLut()   # copied into each spec
 
 
 def compound_cost(xyt, h, spec: CostSpec = CostSpec(), offsets=None, n_max=None, out_cost=None,
@@ -93,10 +92,10 @@ def compound_cost(xyt, h, spec: CostSpec = CostSpec(), offsets=None, n_max=None,
     if classes is not None:
         launch_cost_classes(x, off, order, E, nm, hh, cs, cost, grad, grad_h, classes, stream, "compound_cost")
         return cost, grad, grad_h
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         rc = _lib.load().pk_cost(_lib.ptr(x), _lib.ptr(off), E, nm, _lib.ptr(hh), ctypes.byref(cs),
                                  _lib.ptr(cost), _lib.ptr(grad), _lib.ptr(grad_h),
-                                 ctypes.c_void_p(_lib.stream_handle(stream, dev)))
+                                 _lib.stream_handle(stream, dev))
     _lib.check(rc, "compound_cost")
     return cost, grad, grad_h
 
@@ -116,5 +115,5 @@ def launch_cost_classes(x, off, order, E, n_max, h, cs, cost, grad, grad_h, clas
                                _lib.ptr(grad), _lib.ptr(grad_h), ctypes.c_void_p(st))
         _lib.check(rc, what)
 
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         launch_classes(x.device, stream, classes, launch)

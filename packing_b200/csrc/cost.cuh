@@ -17,8 +17,10 @@
 // O(1) numbers whatever the packing's extent.
 #pragma once
 #include "common.cuh"
+#include "geometry.cuh"
 
 #include <atomic>
+#include <mutex>
 
 struct PkCostSmem {
     float4* pose;       // [n_max] x, y, cos, sin
@@ -1344,6 +1346,30 @@ static inline int pk_cost_threads(int n_max, int count)
     return wide > full ? wide : full;
 }
 
+// Raises a kernel's dynamic shared memory limit only when a launch needs more
+// than any earlier one on this device, so warmed-up launches make no
+// attribute call (they can then be captured into a CUDA graph).  Slots: 0-3 and
+// 28-31 the cost kernels, 4-19, 32-39 the relaxation's, 20-27 the jobs'.
+static cudaError_t pk_set_smem(const void* fn, int slot, size_t smem)
+{
+    static size_t done[64][48];
+    static unsigned gen[64];
+    static std::mutex mu;
+    int dev = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err != cudaSuccess) return err;
+    if (dev < 0 || dev >= 64 || slot < 0 || slot >= 48) return cudaErrorInvalidValue;
+    std::lock_guard<std::mutex> lock(mu);
+    if (gen[dev] != g_pk_init_gen[dev]) {   // pk_init again, perhaps on a new context: nothing is raised there
+        memset(done[dev], 0, sizeof(done[dev]));
+        gen[dev] = g_pk_init_gen[dev];
+    }
+    if (smem <= done[dev][slot]) return cudaSuccess;
+    err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err == cudaSuccess) done[dev][slot] = smem;
+    return err;
+}
+
 // count entries of the launch order (all E instances when order is NULL);
 // threads 0 = pk_cost_threads of the size bound.
 static int pk_launch_cost(const float* xyt, const int* offsets, const int* order, int count, int E, int n_max,
@@ -1384,14 +1410,12 @@ static int pk_launch_cost(const float* xyt, const int* offsets, const int* order
 #define PK_CASE(M)                                                                                  \
     case M:                                                                                         \
         if (spec->symmetry > 1) {                                                                   \
-            err = cudaFuncSetAttribute(pk_cost_kernel<M, true>,                                     \
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
+            err = pk_set_smem((const void*)pk_cost_kernel<M, true>, 28 + M, smem);                  \
             if (err == cudaSuccess)                                                                 \
                 pk_cost_kernel<M, true><<<count, T, smem, st>>>(xyt, offsets, order, E, n_max, h, *spec, \
                                                                 cost, grad, grad_h, cap_near, cap_items); \
         } else {                                                                                    \
-            err = cudaFuncSetAttribute(pk_cost_kernel<M, false>,                                    \
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
+            err = pk_set_smem((const void*)pk_cost_kernel<M, false>, M, smem);                      \
             if (err == cudaSuccess)                                                                 \
                 pk_cost_kernel<M, false><<<count, T, smem, st>>>(xyt, offsets, order, E, n_max, h,    \
                                                                  *spec, cost, grad, grad_h, cap_near, \

@@ -17,8 +17,6 @@
 #include "common.cuh"
 #include "cost.cuh"
 
-#include <mutex>
-
 // Two-loop recursion (:533-572) for one system: d = -H g with the valid
 // history entries in logical order; al is shared scratch of m entries.
 // Every elementwise operation rounds as the reference's tensor operations do
@@ -741,24 +739,6 @@ static int pk_relax_threads(int n_max, int count, int want, int* T, const char* 
     return PK_OK;
 }
 
-// Raises a kernel's dynamic shared memory limit only when a launch needs more
-// than any earlier one on this device, so warmed-up launches make no
-// attribute call (they can then be captured into a CUDA graph).
-static cudaError_t pk_set_smem(const void* fn, int slot, size_t smem)
-{
-    static size_t done[64][48];
-    static std::mutex mu;
-    int dev = 0;
-    cudaError_t err = cudaGetDevice(&dev);
-    if (err != cudaSuccess) return err;
-    if (dev < 0 || dev >= 64 || slot < 0 || slot >= 48) return cudaErrorInvalidValue;
-    std::lock_guard<std::mutex> lock(mu);
-    if (smem <= done[dev][slot]) return cudaSuccess;
-    err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err == cudaSuccess) done[dev][slot] = smem;
-    return err;
-}
-
 // Grid of a persistent launch: every CTA the GPU can keep resident, at most
 // E.  The occupancy of a (kernel, threads, shared memory) shape is queried
 // once per device and remembered, so warmed-up launches make no query.
@@ -947,8 +927,6 @@ extern "C" int pk_relax_jobs(PkJob* jobs, const int* list, int njobs, float* poo
 // as a pointer, so the device address is fetched once per device with
 // cudaGetSymbolAddress (on the first call made with that device current).
 // ---------------------------------------------------------------------------
-#include <mutex>
-
 #define PK_NOALLOC_HISTORY_FLOATS (4u * 1024u * 1024u)   // 16 MiB per device
 
 static __device__ __align__(256) float pk_noalloc_history[PK_NOALLOC_HISTORY_FLOATS];

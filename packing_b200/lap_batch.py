@@ -50,9 +50,9 @@ def solve_lap_batch(cost_matrices_gpu, config: LAPConfig | None = None, return_s
     status = torch.zeros(B, dtype=torch.int32, device=dev)
     if config.algorithm == "hungarian":
         if B > 0:
-            with torch.cuda.device(dev):
+            with _lib.on_device(dev):
                 rc = _lib.load().pk_lap_solve(_lib.ptr(C), B, N, _lib.ptr(row_match), _lib.ptr(total),
-                                              _lib.ptr(status), ctypes.c_void_p(_lib.stream_handle(None, dev)))
+                                              _lib.ptr(status), _lib.stream_handle(None, dev))
             _lib.check(rc, "solve_lap_batch")
     elif config.algorithm == "min_cost_row":
         total = C.amin(dim=2).sum(dim=1).to(torch.float32)
@@ -78,10 +78,10 @@ def compute_diversity_shortcut_kernel(pop_xyt, ref_xyt, cos_a: float, sin_a: flo
     Nr = int(R32.shape[0])
     out = torch.empty(Np * Nr, dtype=torch.float32, device=P32.device)
     if Np * Nr > 0:
-        with torch.cuda.device(P32.device):
+        with _lib.on_device(P32.device):
             rc = _lib.load().pk_diversity_shortcut(_lib.ptr(P32), _lib.ptr(R32), Np, Nr, n, ctypes.c_float(cos_a),
                                                    ctypes.c_float(sin_a), int(bool(do_mirror)), _lib.ptr(out),
-                                                   ctypes.c_void_p(_lib.stream_handle(None, P32.device)))
+                                                   _lib.stream_handle(None, P32.device))
         _lib.check(rc, "compute_diversity_shortcut_kernel")
     res = out.reshape(Np, Nr)
     return res.to(orig) if orig != torch.float32 else res
@@ -99,8 +99,8 @@ def genetic_diversity_matrix(population_xyt, reference_xyt, transform: bool = Tr
     out = torch.empty((Np, Nr), dtype=torch.float32, device=P.device)
     if Np * Nr > 0:
         L, tf = _lib.load(), int(bool(transform))
-        with torch.cuda.device(P.device):
-            stream = ctypes.c_void_p(_lib.stream_handle(None, P.device))
+        with _lib.on_device(P.device):
+            stream = _lib.stream_handle(None, P.device)
             floats = L.pk_diversity_work_floats(Np, Nr, n, tf)
             try:
                 work = torch.empty(floats, dtype=torch.float32, device=P.device) if floats else None
@@ -125,8 +125,8 @@ def genetic_diversity_cost_matrices(population_xyt, reference_xyt, transform: bo
     ntf = 8 if transform else 1
     out = torch.empty((ntf * Np * Nr, n, n), dtype=torch.float32, device=P.device)
     if out.numel() > 0:
-        with torch.cuda.device(P.device):
+        with _lib.on_device(P.device):
             rc = _lib.load().pk_diversity_costs(_lib.ptr(P), _lib.ptr(R), Np, Nr, n, int(bool(transform)),
-                                                _lib.ptr(out), ctypes.c_void_p(_lib.stream_handle(None, P.device)))
+                                                _lib.ptr(out), _lib.stream_handle(None, P.device))
         _lib.check(rc, "genetic_diversity_cost_matrices")
     return out

@@ -53,9 +53,9 @@ def snap(xyt, h=None, stream=None):
     if E == 0:
         return xo, ho
     _lib.ensure_init(x.device)
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         rc = _lib.load().pk_snap(_lib.ptr(x), _lib.ptr(hh), E, n, _lib.ptr(xo), _lib.ptr(ho),
-                                 ctypes.c_void_p(_lib.stream_handle(stream, x.device)))
+                                 _lib.stream_handle(stream, x.device))
     _lib.check(rc, "snap")
     return xo, ho
 

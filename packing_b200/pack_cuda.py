@@ -73,8 +73,8 @@ def overlap_multi_ensemble(xyt1, xyt2, use_separation, out_cost=None, out_grads=
             g.zero_()
         return
     _lib.ensure_init(x1.device)
-    with torch.cuda.device(x1.device):
-        sh = ctypes.c_void_p(_lib.stream_handle(stream, x1.device))
+    with _lib.on_device(x1.device):
+        sh = _lib.stream_handle(stream, x1.device)
         if ax is None:
             rc = _lib.load().pk_overlap(_lib.ptr(x1), E, n, int(bool(use_separation)), _lib.ptr(c), _lib.ptr(g), sh)
         else:
@@ -111,7 +111,7 @@ def boundary_distance_multi_ensemble(xyt, h, out_cost=None, out_grads=None, out_
     if E == 0:
         return
     _lib.ensure_init(x.device)
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         rc = _lib.load().pk_boundary(_lib.ptr(x), _lib.ptr(hh), E, n, _lib.ptr(c), _lib.ptr(g), _lib.ptr(gh),
-                                     ctypes.c_void_p(_lib.stream_handle(stream, x.device)))
+                                     _lib.stream_handle(stream, x.device))
     _lib.check(rc, "boundary_distance_multi_ensemble")

@@ -127,9 +127,9 @@ class LookupTable:
         Td = torch.from_numpy(theta).to(dev)
         vals = torch.empty((len(X), len(Y), len(theta)), device=dev, dtype=torch.float32)
         mode = {"area": _lib.PK_PAIR_AREA, "sep": _lib.PK_PAIR_SEP}[pair]
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             rc = _lib.load().pk_lut_build(_lib.ptr(Xd), len(X), _lib.ptr(Yd), len(Y), _lib.ptr(Td), len(theta), mode,
-                                          _lib.ptr(vals), ctypes.c_void_p(_lib.stream_handle(None, dev)))
+                                          _lib.ptr(vals), _lib.stream_handle(None, dev))
         _lib.check(rc, "pk_lut_build")
         if trim_zeros:
             X, Y, theta, v = cls._trim_zero_edges(X, Y, theta, vals.cpu().numpy(), verbose=False)
@@ -154,10 +154,10 @@ class LookupTable:
         Yd = torch.from_numpy(np.ascontiguousarray(Y)).to(dev)
         Td = torch.from_numpy(np.ascontiguousarray(theta)).to(dev)
         vals = torch.empty((len(X), len(Y), len(theta)), device=dev, dtype=torch.float32)
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             rc = _lib.load().pk_lut_build_exact_sep(_lib.ptr(Xd), len(X), _lib.ptr(Yd), len(Y), _lib.ptr(Td),
                                                     len(theta), _lib.ptr(vals),
-                                                    ctypes.c_void_p(_lib.stream_handle(None, dev)))
+                                                    _lib.stream_handle(None, dev))
         _lib.check(rc, "pk_lut_build_exact_sep")
         if trim_zeros:
             X, Y, theta, vals = cls._trim_zero_edges_device(X, Y, theta, vals)
@@ -218,9 +218,9 @@ def overlap_multi_ensemble(xyt, out_cost, lut: LookupTable, out_grads=None, stre
         return
     _lib.ensure_init(x.device)
     L = lut.c_struct()
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         rc = _lib.load().pk_overlap_lut(_lib.ptr(x), None, E, n, ctypes.byref(L), _lib.ptr(c), _lib.ptr(g),
-                                        ctypes.c_void_p(_lib.stream_handle(stream, x.device)))
+                                        _lib.stream_handle(stream, x.device))
     _lib.check(rc, "pack_cuda_lut.overlap_multi_ensemble")
 
 
@@ -258,7 +258,7 @@ def overlap_multi_ensemble_ragged(xyt_packed, offsets, out_cost, lut: LookupTabl
         launch_cost_classes(x, off, order, E, int(n_max), None, cs, c, g, None, classes, stream,
                             "pack_cuda_lut.overlap_multi_ensemble_ragged")
         return
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         rc = _lib.load().pk_overlap_lut(_lib.ptr(x), _lib.ptr(off), E, int(n_max), ctypes.byref(L), _lib.ptr(c),
-                                        _lib.ptr(g), ctypes.c_void_p(_lib.stream_handle(stream, x.device)))
+                                        _lib.ptr(g), _lib.stream_handle(stream, x.device))
     _lib.check(rc, "pack_cuda_lut.overlap_multi_ensemble_ragged")

@@ -15,10 +15,12 @@ from __future__ import annotations
 import ctypes
 from dataclasses import dataclass
 
+import numpy as np
 import torch
 
 from . import _lib
-from .classes import CLASS_EDGES, CLASS_TABLE, SizeClass, launch_classes, size_classes  # noqa: F401
+from .classes import (CLASS_EDGES, CLASS_TABLE, SizeClass, fills_gpu, largest_first, launch_classes,  # noqa: F401
+                      size_classes)
 from .cost import CostSpec
 
 
@@ -129,11 +131,11 @@ def relax_into(xyt, h, xyt_out, h_out, loss_out, work, spec: CostSpec, params: R
     L = _lib.load()
     if classes is None:
         ps = params.to_c()
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             rc = L.pk_relax(_lib.ptr(x), _lib.ptr(h), _lib.ptr(offsets), _lib.ptr(order), E, nm,
                             ctypes.byref(cs), ctypes.byref(ps), _lib.ptr(xyt_out), _lib.ptr(h_out),
                             _lib.ptr(loss_out), _lib.ptr(iters_out), _lib.ptr(work),
-                            ctypes.c_void_p(_lib.stream_handle(stream, dev)))
+                            _lib.stream_handle(stream, dev))
         _lib.check(rc, "pk_relax")
         return
     if order is None or offsets is None:
@@ -150,7 +152,7 @@ def relax_into(xyt, h, xyt_out, h_out, loss_out, work, spec: CostSpec, params: R
                                 _lib.ptr(loss_out), _lib.ptr(iters_out), _lib.ptr(work), ctypes.c_void_p(st))
         _lib.check(rc, "pk_relax_ordered")
 
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         launch_classes(dev, stream, classes, launch)
 
 
@@ -180,30 +182,33 @@ def relax(xyt, h, spec: CostSpec = CostSpec(), params: RelaxParams = RelaxParams
 def relax_ragged(xyt_list, h, spec: CostSpec = CostSpec(), params: RelaxParams = RelaxParams(), stream=None):
     """Relax packings of different tree counts together, largest first:
     one launch per size class (``size_classes``), side by side on forked
-    streams; with ``params.threads`` set, one launch for all.  xyt_list: list
+    streams; one launch for all of a batch that leaves the GPU idle, or with
+    ``params.threads`` set.  xyt_list: list
     of (n_e, 3) CUDA tensors; h (E, 3).  Returns (list of relaxed (n_e, 3),
     h_out, loss (E,), iterations (E,))."""
-    sizes = [int(a.shape[0]) for a in xyt_list]
-    E = len(sizes)
+    E = len(xyt_list)
     if E == 0:
         return [], None, None, None
+    sizes = [a.shape[0] for a in xyt_list]
     dev = xyt_list[0].device
     _lib.ensure_init(dev)
-    flat = torch.cat([a.reshape(-1, 3).to(torch.float32) for a in xyt_list]).contiguous()
-    off_h = [0]
-    for s in sizes:
-        off_h.append(off_h[-1] + s)
-    offsets = torch.tensor(off_h, dtype=torch.int32, device=dev)
-    order_h = sorted(range(E), key=lambda e: -sizes[e])
-    order = torch.tensor(order_h, dtype=torch.int32, device=dev)
+    if all(a.dim() == 2 for a in xyt_list):
+        flat = torch.cat(xyt_list).to(torch.float32)
+    else:
+        flat = torch.cat([a.reshape(-1, 3).to(torch.float32) for a in xyt_list]).contiguous()
+    sz = np.array(sizes, dtype=np.int64)
+    order_h = largest_first(sz)
+    # one copy to the device: the offsets, then the launch order
+    plan = torch.from_numpy(np.concatenate([[0], np.cumsum(sz), order_h]).astype(np.int32)).to(dev)
+    offsets, order = plan[:E + 1], plan[E + 1:]
     hh = _lib.as_tensor(h, "h").contiguous() if h is not None else None
     xo = torch.empty_like(flat)
     ho = torch.empty_like(hh) if hh is not None else None
     loss = torch.empty(E, dtype=torch.float32, device=dev)
     iters = torch.empty(E, dtype=torch.int32, device=dev)
-    work = torch.empty(max(1, workspace_floats(sizes, params.history_size)), dtype=torch.float32, device=dev)
-    classes = size_classes([sizes[e] for e in order_h]) if params.threads == 0 else None
-    relax_into(flat, hh, xo, ho, loss, work, spec, params, offsets=offsets, order=order, n_max=max(sizes),
+    work = torch.empty(max(1, 2 * int(params.history_size) * int(3 * sz.sum() + 3 * E)), dtype=torch.float32,
+                       device=dev)
+    classes = size_classes(sz[order_h]) if params.threads == 0 and fills_gpu(E, dev) else None
+    relax_into(flat, hh, xo, ho, loss, work, spec, params, offsets=offsets, order=order, n_max=int(sz.max()),
                iters_out=iters, stream=stream, classes=classes)
-    outs = [xo[off_h[e]:off_h[e + 1]] for e in range(E)]
-    return outs, ho, loss, iters
+    return list(torch.split(xo, sizes)), ho, loss, iters

@@ -30,9 +30,9 @@ def validate(xyt, stream=None):
     if E == 0:
         return ov, side
     _lib.ensure_init(x.device)
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         rc = _lib.load().pk_validate_fp64(_lib.ptr(x), x.element_size(), E, n, _lib.ptr(ov), _lib.ptr(side),
-                                          ctypes.c_void_p(_lib.stream_handle(stream, x.device)))
+                                          _lib.stream_handle(stream, x.device))
     _lib.check(rc, "validate")
     return ov, side
 

@@ -241,3 +241,23 @@ def test_small_batches_equal_large_ones(cuda, n, pair, symmetry):
     large += compound_cost(x.repeat(many, 1, 1), h.repeat(many, 1), spec)
     for a, b in zip(small, large):
         assert torch.equal(a, b[:4]) and torch.equal(a, b[-4:])
+
+
+@pytest.mark.parametrize("E", [3, 400])
+def test_ragged_list_forms(cuda, E):
+    """relax_ragged takes (n, 3) tensors of mixed floating types and strides,
+    below and above the batch that is split into size classes; each packing's
+    result is its own relaxation's."""
+    from packing_b200.relax import RelaxParams, relax, relax_ragged
+    sizes = [1 + (7 * k) % 45 for k in range(E)]
+    xs = [torch.from_numpy(poses(1, n, seed=n)[0]).to(cuda) for n in sizes]
+    h = torch.from_numpy(np.concatenate([square_h(1, n) for n in sizes])).to(cuda)
+    prm = RelaxParams(n_iterations=6, history_size=3)
+    out, ho, loss, it = relax_ragged(xs, h, params=prm)
+    odd = [x.double() if k % 3 == 0 else x.t().contiguous().t() if k % 3 == 1 else x for k, x in enumerate(xs)]
+    out2, ho2, loss2, it2 = relax_ragged(odd, h, params=prm)
+    assert torch.equal(loss, loss2) and torch.equal(it, it2) and torch.equal(ho, ho2)
+    assert all(torch.equal(a, b) and a.shape == x.shape for a, b, x in zip(out, out2, xs))
+    for k in (0, 1, E - 1):
+        xo, _, l1, i1 = relax(xs[k][None], h[k:k + 1], params=prm)
+        assert torch.equal(xo[0], out[k]) and torch.equal(l1[0], loss[k]) and torch.equal(i1[0], it[k])
