@@ -899,11 +899,109 @@ struct PkEvalOut {
 
 __device__ __forceinline__ float pk_near_skin() { return PK_NEAR_SKIN * sqrtf(c_geom.cutoff_sq); }
 
+// Broad phase by testing every pair, for packings of at most 256 trees: thread
+// per tree a, offsets 1 .. n/2 read from a position array that runs on past n
+// (kept in the near list's space until that is written), one mask bit per test.
+// Masks stay in the grid's cell arrays for pass 2, which expands them and tests
+// nothing again.  Three barriers and about six instructions a test, against the
+// grid's sorting by cell, two scans and two walks of the neighbourhoods behind a
+// dozen barriers: n (n - 1) / 2 tests are the cheaper ones up to the 256 trees
+// that the masks allow (one-shot area cost, grid -> this: 8192 x 40 201 -> 153 us,
+// 4096 x 200 380 -> 344, 2048 x 250 231 -> 216; LUT, 8192 of 5 to 200 125 -> 102).
+// Counts go to near_cnt, list offsets to near_start (in list order only if the
+// list overflows), flags as in pk_broad_phase.  All threads call it, behind a
+// barrier; pass 2 needs none in between.
+__device__ __forceinline__ bool pk_all_pairs_fit(const PkCostSmem& sm, int n)
+{
+    return n <= 256 && (n + (n >> 1) + 32) * 8 <= sm.cap_near * 4;
+}
+
+template <bool KEEP>
+__device__ __forceinline__ void pk_all_pairs(const PkCostSmem& sm, int n, bool build)
+{
+    const int T = blockDim.x, lane = threadIdx.x & 31, half = n >> 1;
+    float2* pos = (float2*)sm.near;
+    uint32_t* masks = (uint32_t*)sm.cell_start;   // [(half + 31) / 32][n]
+    for (int t = threadIdx.x; t < n + half; t += T) {
+        const float4 A = sm.pose[t < n ? t : t - n];
+        pos[t] = make_float2(A.x, A.y);
+    }
+    if (threadIdx.x == 0) sm.near_start[n] = 0;
+    float cut_list = c_geom.cutoff_sq;
+    if (build) {
+        const float r = sqrtf(cut_list) + pk_near_skin();
+        cut_list = r * r;
+    }
+    for (;;) {
+        __syncthreads();
+        for (int a0 = 0; a0 < n; a0 += T) {
+            const int a = a0 + threadIdx.x;
+            int k = 0;
+            if (a < n) {
+                const float2 A = pos[a], nA = make_float2(-A.x, -A.y);
+                for (int w = 0; 32 * w < half; ++w) {
+                    const float2* o = pos + a + 1 + 32 * w;
+                    const int nb = min(32, half - 32 * w);
+                    uint32_t m = 0;
+                    // rounded as pk_is_near rounds
+#define PK_NEAR_BIT(B)                                                                       \
+    {                                                                                        \
+        const float2 d = __fadd2_rn(o[B], nA), q = __fmul2_rn(d, d);                         \
+        if (__fadd_rn(q.x, q.y) <= cut_list) m |= 1u << (B);                                 \
+    }
+                    if (nb == 32) {
+#pragma unroll
+                        for (int b = 0; b < 32; ++b) PK_NEAR_BIT(b)
+                    } else {
+                        for (int b = 0; b < nb; b += 4)   // up to 3 past half: masked below
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) PK_NEAR_BIT(b + u)
+                        m &= (1u << nb) - 1u;
+                    }
+#undef PK_NEAR_BIT
+                    if (32 * w + nb == half && 2 * half == n && a >= half) m &= ~(1u << (nb - 1));   // met twice
+                    masks[w * n + a] = m;
+                    k += __popc(m);
+                }
+                sm.near_cnt[a] = k;
+            }
+            int incl = k;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(PK_FULL_MASK, incl, o);
+                if (lane >= o) incl += v;
+            }
+            int base = 0;
+            if (lane == 31 && incl) base = atomicAdd(&sm.near_start[n], incl);
+            base = __shfl_sync(PK_FULL_MASK, base, 31);
+            if (a < n) sm.near_start[a] = base + incl - k;
+        }
+        if (KEEP && threadIdx.x == 0) {
+            pk_nlist(sm)[2] = build;
+            ((float*)pk_nlist(sm))[3] = cut_list;
+        }
+        __syncthreads();
+        if (sm.near_start[n] <= sm.cap_near) break;
+        if (!KEEP || !build) {   // several chunks: offsets in list order
+            __syncthreads();
+            pk_block_exclusive_scan(sm.near_cnt, sm.near_start, n, (int*)sm.redl);
+            break;
+        }
+        // a kept list must fit in one piece: again at the cutoff, and no kept lists from now on
+        build = false;
+        cut_list = c_geom.cutoff_sq;
+        __syncthreads();
+        if (threadIdx.x == 0) { pk_nlist(sm)[0] = -1; sm.near_start[n] = 0; }
+    }
+    if (threadIdx.x == 0) sm.cnt[0] += (unsigned)(n * (n - 1) / 2);
+}
+
 // Broad phase on a uniform grid of cells at least the interaction distance
 // wide: tree i only meets trees of the 3 x 3 cells around its own, and each
 // pair is found once, from its lower index.  Builds the grid (sm.cell_start,
 // sm.sorted, sm.tcell), counts each sorted position's near pairs (pass 1)
-// and scans the counts into sm.near_start; returns the grid's (gx, gy).
+// and scans the counts into sm.near_start; returns the grid's (gx, gy), or (0, 0)
+// when pk_all_pairs did it without a grid.
 // build: take pairs within cutoff + skin for a kept list, falling back to the
 // cutoff (and to no kept lists from then on) when they do not fit the near
 // list in one piece.  Leaves pk_nlist(sm)[2] (list kept) and [3] (the
@@ -913,6 +1011,10 @@ __device__ __forceinline__ float pk_near_skin() { return PK_NEAR_SKIN * sqrtf(c_
 template <bool KEEP>
 __device__ __forceinline__ int2 pk_broad_phase(const PkCostSmem& sm, int n, bool build)
 {
+    if (pk_all_pairs_fit(sm, n)) {
+        pk_all_pairs<KEEP>(sm, n, build);
+        return make_int2(0, 0);
+    }
     const int T = blockDim.x;
     const float cutoff = c_geom.cutoff_sq;
     float cut_list = cutoff;
@@ -1018,30 +1120,47 @@ template <bool KEEP>
 __device__ __forceinline__ int2 pk_write_near(const PkCostSmem& sm, int n, int a0, int gx, int gy)
 {
     const int T = blockDim.x;
-    // the longest run of positions from a0 whose pairs fit the list
-    // (a single position's pairs always do: cap_near >= n_max)
-    int lo = a0 + 1, hi = n;
-    const int lim = sm.near_start[a0] + sm.cap_near;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (sm.near_start[mid] <= lim) lo = mid; else hi = mid - 1;
+    int a1 = n, base = 0;
+    if (gx > 0 || sm.near_start[n] > sm.cap_near) {
+        // the longest run of positions from a0 whose pairs fit the list
+        // (a single position's pairs always do: cap_near >= n_max)
+        int lo = a0 + 1, hi = n;
+        const int lim = sm.near_start[a0] + sm.cap_near;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (sm.near_start[mid] <= lim) lo = mid; else hi = mid - 1;
+        }
+        a1 = lo;
+        base = sm.near_start[a0];
     }
-    const int a1 = lo, base = sm.near_start[a0];
     const int cn = sm.near_start[a1] - base;
-    const float cut2 = KEEP ? ((const float*)pk_nlist(sm))[3] : c_geom.cutoff_sq;   // pass 1's distance
-    for (int a = a0 + threadIdx.x; a < a1; a += T) {
-        int b0, b1, b2, b3;
-        pk_half_neighbourhood(sm, a, gx, gy, b0, b1, b2, b3);
-        const int ia = sm.sorted[a];
-        const float4 A = sm.pose[ia];
-        uint32_t* out = sm.near + (sm.near_start[a] - base);
-        const int kmax = sm.near_cnt[a];
-        int k = 0;
-        for (int b = b0; b < b3 && k < kmax; ++b) {
-            if (b == b1) { b = b2; if (b >= b3) break; }
-            const int ib = sm.sorted[b];
-            if (pk_is_near(A, sm.pose[ib], cut2))
-                out[k++] = (uint32_t)min(ia, ib) | ((uint32_t)max(ia, ib) << 11);
+    if (gx == 0) {
+        const uint32_t* masks = (const uint32_t*)sm.cell_start;
+        for (int a = a0 + threadIdx.x; a < a1; a += T) {
+            uint32_t* out = sm.near + (sm.near_start[a] - base);
+            for (int w = 0; 64 * w < n - 1; ++w)   // the words pass 1 wrote: 32 w < n / 2
+                for (uint32_t m = masks[w * n + a]; m; m &= m - 1) {
+                    int j = a + 32 * w + __ffs(m);
+                    if (j >= n) j -= n;
+                    *out++ = (uint32_t)min(a, j) | ((uint32_t)max(a, j) << 11);
+                }
+        }
+    } else {
+        const float cut2 = KEEP ? ((const float*)pk_nlist(sm))[3] : c_geom.cutoff_sq;   // pass 1's distance
+        for (int a = a0 + threadIdx.x; a < a1; a += T) {
+            int b0, b1, b2, b3;
+            pk_half_neighbourhood(sm, a, gx, gy, b0, b1, b2, b3);
+            const int ia = sm.sorted[a];
+            const float4 A = sm.pose[ia];
+            uint32_t* out = sm.near + (sm.near_start[a] - base);
+            const int kmax = sm.near_cnt[a];
+            int k = 0;
+            for (int b = b0; b < b3 && k < kmax; ++b) {
+                if (b == b1) { b = b2; if (b >= b3) break; }
+                const int ib = sm.sorted[b];
+                if (pk_is_near(A, sm.pose[ib], cut2))
+                    out[k++] = (uint32_t)min(ia, ib) | ((uint32_t)max(ia, ib) << 11);
+            }
         }
     }
     __syncthreads();

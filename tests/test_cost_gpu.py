@@ -250,3 +250,21 @@ def test_piled_trees_overflow_the_lists(cuda, n, pair):
     np.testing.assert_allclose(got[0][0].cpu().numpy(), oc, rtol=RTOL_COST)
     if pair == "area":   # the separation's smallest axis can differ between FP32 and FP64 where two tie
         np.testing.assert_allclose(got[0][1].cpu().numpy().reshape(E, n, 3), og, rtol=TOL_GRAD, atol=TOL_GRAD)
+
+
+@pytest.mark.parametrize("n", [2, 3, 63, 64, 65, 66, 127, 128, 129, 255, 256])
+def test_broad_phase_sizes(cuda, n):
+    """Packings of at most 256 trees test every pair, larger ones go through the
+    cell grid: with trees added far away, so that the grid serves it, a packing has
+    the same cost and gradient bit for bit.  Sizes around the mask words' edges (32
+    offsets each), odd and even, spread and piled (the near list overflows)."""
+    far = np.zeros((2, 300 - n, 3), np.float32)
+    far[:, :, 0] = 50.0 + 5.0 * np.arange(300 - n)
+    for seed, side in ((n, 1.3), (n + 1, 0.35)):
+        x = poses(2, n, seed=seed, side_factor=side)
+        for sep in (False, True):
+            c, g = _overlap(x, sep, cuda)
+            cf, gf = _overlap(np.concatenate([x, far], 1), sep, cuda)
+            assert np.array_equal(c, cf) and np.array_equal(g, gf[:, :n]) and not gf[:, n:].any()
+            oc, _ = O.pair_cost(x.astype(np.float64), sep)
+            np.testing.assert_allclose(c, oc, rtol=RTOL_COST)
