@@ -407,60 +407,61 @@ __device__ __forceinline__ void pk_piece_sat_grad(const float2 (&P)[4], bool p_t
     sep = 0.f;
     gP = make_float3(0.f, 0.f, 0.f);
     gQ = make_float3(0.f, 0.f, 0.f);
+    // The smallest overlap over the axes, by selects: a warp's lanes separate or
+    // improve at different axes.  The extreme vertices are found once, for the axis
+    // that won, from its projections computed again (the same operations).
     float best = 1.0e30f;
-    bool found = false, from1 = false;
-    float sigma = 1.f;
-    float2 bn = make_float2(0.f, 0.f), bv = bn, bw = bn;
+    bool apart = false, found = false, from1 = false, c1 = true;
+    float2 bn = make_float2(0.f, 0.f);
 #pragma unroll
     for (int pass = 0; pass < 2; ++pass) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const bool tri = pass == 0 ? p_tri : q_tri;
-            if (k == 3 && tri) continue;
             const float2 a = pass == 0 ? P[k] : Q[k];
             const float2 b = pass == 0 ? P[(k + 1) & 3] : Q[(k + 1) & 3];
             float2 nr = make_float2(-(b.y - a.y), b.x - a.x);
             const float len = sqrtf(nr.x * nr.x + nr.y * nr.y);
-            if (len < 1.0e-12f) continue;
+            const bool real = !(k == 3 && tri) && !(len < 1.0e-12f);
             nr.x /= len;
             nr.y /= len;
-            float p1[4], p2[4];
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                p1[v] = P[v].x * nr.x + P[v].y * nr.y;
-                p2[v] = Q[v].x * nr.x + Q[v].y * nr.y;
-            }
-            float mn1 = p1[0], mx1 = p1[0], mn2 = p2[0], mx2 = p2[0];
+            float mn1 = P[0].x * nr.x + P[0].y * nr.y, mx1 = mn1, mn2 = Q[0].x * nr.x + Q[0].y * nr.y, mx2 = mn2;
 #pragma unroll
             for (int v = 1; v < 4; ++v) {
-                mn1 = fminf(mn1, p1[v]); mx1 = fmaxf(mx1, p1[v]);
-                mn2 = fminf(mn2, p2[v]); mx2 = fmaxf(mx2, p2[v]);
+                const float p1 = P[v].x * nr.x + P[v].y * nr.y, p2 = Q[v].x * nr.x + Q[v].y * nr.y;
+                mn1 = fminf(mn1, p1); mx1 = fmaxf(mx1, p1);
+                mn2 = fminf(mn2, p2); mx2 = fmaxf(mx2, p2);
             }
-            if (mx1 < mn2 || mx2 < mn1) return;   // separating axis: no overlap
-            found = true;
+            apart |= real & ((mx1 < mn2) | (mx2 < mn1));   // separating axis: no overlap
+            found |= real;
             const float pen1 = mx1 - mn2, pen2 = mx2 - mn1;
             const float pen = pen1 < pen2 ? pen1 : pen2;
-            if (pen < best) {
-                best = pen;
-                bn = nr;
-                from1 = pass == 0;
-                const bool c1 = pen1 <= pen2;
-                sigma = c1 ? 1.f : -1.f;
-                // first vertex attaining the extreme, like the reference scans
-                float2 v = P[0], w = Q[0];
-                float pv = p1[0], pw = p2[0];
-#pragma unroll
-                for (int q = 1; q < 4; ++q) {
-                    if (c1 ? (p1[q] > pv) : (p1[q] < pv)) { pv = p1[q]; v = P[q]; }
-                    if (c1 ? (p2[q] < pw) : (p2[q] > pw)) { pw = p2[q]; w = Q[q]; }
-                }
-                bv = v;
-                bw = w;
-            }
+            const bool less = real & (pen < best);
+            best = less ? pen : best;
+            bn.x = less ? nr.x : bn.x;
+            bn.y = less ? nr.y : bn.y;
+            from1 = less ? pass == 0 : from1;
+            c1 = less ? pen1 <= pen2 : c1;
         }
     }
-    if (!found || best <= 1.0e-12f) return;
+    if (apart || !found || best <= 1.0e-12f) return;
     sep = best;
+    if (!(best < 1.0e30f)) return;   // a NaN angle: no axis says anything
+    const float sigma = c1 ? 1.f : -1.f;
+    // first vertex attaining the extreme, like the reference scans
+    float2 bv = P[0], bw = Q[0];
+    float pv = P[0].x * bn.x + P[0].y * bn.y, pw = Q[0].x * bn.x + Q[0].y * bn.y;
+#pragma unroll
+    for (int q = 1; q < 4; ++q) {
+        const float p1 = P[q].x * bn.x + P[q].y * bn.y, p2 = Q[q].x * bn.x + Q[q].y * bn.y;
+        const bool v1 = c1 ? p1 > pv : p1 < pv, v2 = c1 ? p2 < pw : p2 > pw;
+        pv = v1 ? p1 : pv;
+        bv.x = v1 ? P[q].x : bv.x;
+        bv.y = v1 ? P[q].y : bv.y;
+        pw = v2 ? p2 : pw;
+        bw.x = v2 ? Q[q].x : bw.x;
+        bw.y = v2 ? Q[q].y : bw.y;
+    }
     const float2 gv = make_float2(sigma * bn.x, sigma * bn.y);
     const float2 rn = make_float2(-bn.y, bn.x);                     // d n / d theta
     const float2 vw = make_float2(bv.x - bw.x, bv.y - bw.y);
