@@ -122,6 +122,16 @@ int pk_cost_ordered(const float* xyt, const int* offsets, const int* order, int 
                     const float* h, const PkCostSpec* spec, int threads, float* cost, float* grad, float* grad_h,
                     void* stream);
 
+/* pk_cost_ordered for every size class of a largest-first order: class k is
+ * order[start .. start + count - 1] (the classes cover it once), none with more
+ * than n_max trees, on CTAs of `threads` (0: the library's choice), on
+ * stream side[k], forked from and joined to `stream` (a single class runs on
+ * `stream` itself).  The same results as one launch. */
+typedef struct PkSizeClass { int start, count, n_max, threads; } PkSizeClass;
+int pk_cost_classes(const float* xyt, const int* offsets, const int* order, const PkSizeClass* classes, int n_classes,
+                    int E, int n_max, const float* h, const PkCostSpec* spec, float* cost, float* grad, float* grad_h,
+                    void* stream, void* const* side);
+
 /* pack_cuda.overlap_multi_ensemble(xyt, xyt, use_separation, out_cost,
  * out_grads) (pack_cuda.py:1040-1183), non-periodic form. */
 int pk_overlap(const float* xyt, int E, int n, int use_separation, float* cost, float* grad,

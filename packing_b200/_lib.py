@@ -60,6 +60,10 @@ class PkCostSpec(ctypes.Structure):
     ]
 
 
+class PkSizeClass(ctypes.Structure):
+    _fields_ = [("start", ctypes.c_int), ("count", ctypes.c_int), ("n_max", ctypes.c_int), ("threads", ctypes.c_int)]
+
+
 class PkRelaxParams(ctypes.Structure):
     _fields_ = [
         ("max_iter", ctypes.c_int), ("history", ctypes.c_int), ("lr", ctypes.c_float),
@@ -125,6 +129,8 @@ SIGNATURES = {
     "pk_last_error": [],
     "pk_cost": [_P, _P, _I, _I, _P, ctypes.POINTER(PkCostSpec), _P, _P, _P, _P],
     "pk_cost_ordered": [_P, _P, _P, _I, _I, _I, _P, ctypes.POINTER(PkCostSpec), _I, _P, _P, _P, _P],
+    "pk_cost_classes": [_P, _P, _P, ctypes.POINTER(PkSizeClass), _I, _I, _I, _P, ctypes.POINTER(PkCostSpec), _P, _P, _P,
+                        _P, ctypes.POINTER(ctypes.c_void_p)],
     "pk_overlap": [_P, _I, _I, _I, _P, _P, _P],
     "pk_overlap_crystal": [_P, _I, _I, _I, _P, _I, _I, _P, _P, _P],
     "pk_boundary": [_P, _P, _I, _I, _P, _P, _P, _P],

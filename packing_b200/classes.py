@@ -108,8 +108,11 @@ def base_stream(stream, dev):
 def launch_classes(dev, stream, classes, launch):
     """Call launch(cls, stream_handle) for every class, each on its own side
     stream forked from ``stream`` (None: the current stream) and joined back
-    to it."""
+    to it; a single class on ``stream`` itself."""
     base = base_stream(stream, dev)
+    if len(classes) == 1:
+        launch(classes[0], base.cuda_stream)
+        return
     side = side_streams(dev, len(classes))
     fork = torch.cuda.Event()
     fork.record(base)

@@ -102,18 +102,16 @@ def compound_cost(xyt, h, spec: CostSpec = CostSpec(), offsets=None, n_max=None,
 
 def launch_cost_classes(x, off, order, E, n_max, h, cs, cost, grad, grad_h, classes, stream, what):
     """One pk_cost_ordered launch per size class, side by side on forked streams."""
-    from .classes import launch_classes
+    from .classes import side_streams
     if off is None or order is None:
         raise ValueError(f"{what}: classes need a ragged batch with a largest-first order")
     if sum(c.count for c in classes) != E or any(c.n_max > n_max for c in classes):
         raise ValueError(f"{what}: classes must cover the order once, each within n_max")
-    L = _lib.load()
-
-    def launch(c, st):
-        rc = L.pk_cost_ordered(_lib.ptr(x), _lib.ptr(off), ctypes.c_void_p(order.data_ptr() + 4 * c.start), c.count,
-                               E, c.n_max, _lib.ptr(h), ctypes.byref(cs), int(c.threads), _lib.ptr(cost),
-                               _lib.ptr(grad), _lib.ptr(grad_h), ctypes.c_void_p(st))
-        _lib.check(rc, what)
-
+    k = len(classes)
+    table = (_lib.PkSizeClass * k)(*[(c.start, c.count, c.n_max, c.threads) for c in classes])
+    side = (ctypes.c_void_p * k)(*[s.cuda_stream for s in side_streams(x.device, k)])
     with _lib.on_device(x.device):
-        launch_classes(x.device, stream, classes, launch)
+        rc = _lib.load().pk_cost_classes(_lib.ptr(x), _lib.ptr(off), _lib.ptr(order), table, k, E, int(n_max),
+                                         _lib.ptr(h), ctypes.byref(cs), _lib.ptr(cost), _lib.ptr(grad),
+                                         _lib.ptr(grad_h), _lib.stream_handle(stream, x.device), side)
+    _lib.check(rc, what)

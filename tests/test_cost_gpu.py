@@ -268,3 +268,24 @@ def test_broad_phase_sizes(cuda, n):
             assert np.array_equal(c, cf) and np.array_equal(g, gf[:, :n]) and not gf[:, n:].any()
             oc, _ = O.pair_cost(x.astype(np.float64), sep)
             np.testing.assert_allclose(c, oc, rtol=RTOL_COST)
+
+
+@pytest.mark.parametrize("E", [7, 2400])
+def test_size_classes_of_a_cost_call(cuda, E):
+    """Classes below and above the batch that is worth forking streams for, in any
+    order and with any threads, equal one launch; a class table that does not cover
+    the batch is refused."""
+    from packing_b200.classes import SizeClass, ragged_plan, size_classes
+    from packing_b200.cost import CostSpec, compound_cost
+    sizes = np.array([2 + (11 * k) % 90 for k in range(E)])
+    flat = _t(np.concatenate([poses(1, int(n), seed=int(n))[0] for n in sizes]), cuda)
+    h = _t(np.concatenate([square_h(1, int(n)) for n in sizes]), cuda)
+    off = torch.tensor(np.concatenate([[0], np.cumsum(sizes)]), dtype=torch.int32, device=cuda)
+    order, plan = ragged_plan(sizes.tolist(), cuda)
+    table = size_classes(-np.sort(-sizes))
+    one = compound_cost(flat, h, CostSpec(), offsets=off, n_max=91)
+    for cls in (plan, table, list(reversed(table)), [SizeClass(c.start, c.count, 91, 0) for c in table]):
+        got = compound_cost(flat, h, CostSpec(), offsets=off, n_max=91, order=order, classes=cls)
+        assert all(torch.equal(a, b) for a, b in zip(one, got))
+    with pytest.raises(ValueError):
+        compound_cost(flat, h, CostSpec(), offsets=off, n_max=91, order=order, classes=table[1:])
