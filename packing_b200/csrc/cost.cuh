@@ -31,7 +31,7 @@ struct PkCostSmem {
     float4* bnd;        // [n_max] boundary: cost, dh0, dh1, dh2 (unweighted)
     uint16_t* items;    // [cap_items] piece pairs: near list index | pi << 11 | pj << 13
     uint32_t* near;     // [cap_near] centre-culled pairs: i | j << 11
-    int* count;         // items in the list
+    int* count;         // [2] items reserved in the list; first reservation that did not fit (its base)
     double* red;        // [32]
     long long* redl;    // [32]
     float2* piece;      // [16]
@@ -819,11 +819,12 @@ __device__ __forceinline__ long long pk_flush_near(const PkCostSmem& sm, int cn,
                 const int wtot = __shfl_sync(PK_FULL_MASK, incl, 31);
                 int wbase = 0;
                 if (lane == 31 && wtot) {
-                    // once a reservation fails every later one does (the count
-                    // is above the capacity until it is taken back), so the
-                    // list has no gaps
-                    wbase = atomicAdd(sm.count, wtot);
-                    if (wbase + wtot > sm.cap_items) { atomicSub(sm.count, wtot); wbase = -1; }
+                    // A reservation that does not fit stays counted, so every
+                    // later one fails too and the list has no gaps: it ends where
+                    // the first one failed.  (Taken back, a failed reservation
+                    // could let another in behind one not yet taken back.)
+                    wbase = atomicAdd(&sm.count[0], wtot);
+                    if (wbase + wtot > sm.cap_items) { atomicMin(&sm.count[1], wbase); wbase = -1; }
                 }
                 wbase = __shfl_sync(PK_FULL_MASK, wbase, 31);
                 if (wbase < 0) break;
@@ -836,19 +837,22 @@ __device__ __forceinline__ long long pk_flush_near(const PkCostSmem& sm, int cn,
                 }
             }
             const int more = __syncthreads_or(ch < chunks);
-            const int ci = *sm.count;
+            const int ci = min(sm.count[0], sm.count[1]);
             if (threadIdx.x == 0) sm.cnt[2] += (unsigned)ci;
             tot += KEEP ? pk_process_items_outlined<MODE>(sm.n_cap, sm.cap_near, sm.cap_items, ci, spec.w_pair)
                         : pk_process_items<MODE>(sm, ci, spec.w_pair);
             if (!more) break;
             __syncthreads();
-            if (threadIdx.x == 0) *sm.count = 0;
+            if (threadIdx.x == 0) { sm.count[0] = 0; sm.count[1] = 0x7fffffff; }
             __syncthreads();
         }
         if (near && lane == 0) atomicAdd(&sm.cnt[1], near);
     }
     __syncthreads();
-    if (MODE != PK_PAIR_LUT && threadIdx.x == 0) *sm.count = 0;   // the next flush appends after another barrier
+    if (MODE != PK_PAIR_LUT && threadIdx.x == 0) {   // the next flush appends after another barrier
+        sm.count[0] = 0;
+        sm.count[1] = 0x7fffffff;
+    }
     return tot;
 }
 
@@ -1303,7 +1307,8 @@ __device__ double pk_eval_instance(const float* X, int ng, const float* H, const
         sm.bnd[t] = bnd;
     }
     if (threadIdx.x == 0) {
-        *sm.count = 0;
+        sm.count[0] = 0;
+        sm.count[1] = 0x7fffffff;
         sm.cnt[3] += 1;
     }
     if (nstate == 1) {

@@ -246,6 +246,12 @@ def test_piled_trees_overflow_the_lists(cuda, n, pair):
            for t in (32, 64, 96, 256)]
     for c, g in got[1:]:
         assert torch.equal(c, got[0][0]) and torch.equal(g, got[0][1])
+    # many copies at once: however the warps' reservations in a full list interleave
+    many = 300
+    xm = _t(np.tile(x, (many, 1, 1)), cuda)
+    cm, gm, _ = compound_cost(xm, None, spec)
+    assert torch.equal(cm, got[0][0].repeat(many))
+    assert torch.equal(gm, got[0][1].reshape(E, n, 3).repeat(many, 1, 1))
     oc, og = O.pair_cost(x.astype(np.float64), pair == "sep")
     np.testing.assert_allclose(got[0][0].cpu().numpy(), oc, rtol=RTOL_COST)
     if pair == "area":   # the separation's smallest axis can differ between FP32 and FP64 where two tie
