@@ -241,6 +241,20 @@ int pk_validate_fp64(const void* xyt, int dtype_bytes, int E, int n, int* overla
 int pk_lbfgs_phase(int phase, int dtype_bytes, void* const* arrays, int M, int N, int m, int n_iter, double p0,
                    double p1, double p2, double p3, int i1, int i2, void* stream);
 
+/* Iteration n_iter (1, 2, ...) of the same loop without a line search, up to and
+ * including its step, in two launches: phase 3 of the iteration before (phase 0
+ * for n_iter = 1) with loss and gradient at the current x, phase 1, and x += t d
+ * if any system is active.  The arrays of pk_lbfgs_phase, with any_active int32
+ * (2,), zero before the first call; arrays[1] and arrays[2] (gradient, loss) may
+ * be the objective's own output.  host_flag: pinned host memory that holds, once
+ * the stream has been waited for, whether any system is active. */
+typedef struct PkLbfgsParams {
+    double lr, max_step, tol_grad, tol_change, tol_rel_change;
+    int has_max_step, stop_on_cost_increase, max_eval;
+} PkLbfgsParams;
+int pk_lbfgs_iterate(int dtype_bytes, void* const* arrays, int M, int N, int m, int n_iter, const PkLbfgsParams* params,
+                     int* host_flag, void* stream);
+
 /* Batched strong-Wolfe line search of the drop-in lbfgs
  * (_strong_wolfe_batched, lbfgs_torch_parallel.py:70-407, with its defaults
  * c1 = 1e-4, c2 = 0.9, tolerance_change = 1e-9, max_ls = 25 as the main loop

@@ -75,6 +75,14 @@ class PkRelaxParams(ctypes.Structure):
     ]
 
 
+class PkLbfgsParams(ctypes.Structure):
+    _fields_ = [
+        ("lr", ctypes.c_double), ("max_step", ctypes.c_double), ("tol_grad", ctypes.c_double),
+        ("tol_change", ctypes.c_double), ("tol_rel_change", ctypes.c_double),
+        ("has_max_step", ctypes.c_int), ("stop_on_cost_increase", ctypes.c_int), ("max_eval", ctypes.c_int),
+    ]
+
+
 class PkJob(ctypes.Structure):
     _fields_ = [
         ("n", ctypes.c_int), ("max_iter", ctypes.c_int),
@@ -147,6 +155,7 @@ SIGNATURES = {
     "pk_diversity_costs": [_P, _P, _I, _I, _I, _I, _P, _P],
     "pk_diversity_shortcut": [_P, _P, _I, _I, _I, _F, _F, _I, _P, _P],
     "pk_lbfgs_phase": [_I, _I, _P, _I, _I, _I, _I, _D, _D, _D, _D, _I, _I, _P],
+    "pk_lbfgs_iterate": [_I, _P, _I, _I, _I, _I, ctypes.POINTER(PkLbfgsParams), _P, _P],
     "pk_wolfe_phase": [_I, _I, _P, _I, _I, _I, _D, _D, _D, _I, _P],
     "pk_wolfe_apply": [_I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _P],
     "pk_relax": [_P, _P, _P, _P, _I, _I, ctypes.POINTER(PkCostSpec), ctypes.POINTER(PkRelaxParams), _P, _P, _P,

@@ -345,6 +345,121 @@ __global__ void pk_lbfgs_init_kernel(PkLbfgsState<F> s, F tol_grad)
     }
 }
 
+// Iteration n_iter up to its step in one kernel: the update of the iteration
+// before with the objective's new loss and gradient (iteration 1: the initial
+// activity instead), then the direction, first step length, clamp and
+// directional-derivative stop.  The same operations as the kernels above, for
+// the loop without a line search.
+template <typename F>
+__global__ void pk_lbfgs_iterate_kernel(PkLbfgsState<F> s, int n_iter, PkLbfgsParams prm)
+{
+    extern __shared__ __align__(16) unsigned char pk_smem[];
+    const int N = s.N, m = s.m;
+    F* al = (F*)pk_smem;
+    F* red = al + m;
+    int flip = 0;
+    const int b = blockIdx.x;
+    const F* g = s.g + (size_t)b * N;
+    F* d = s.d + (size_t)b * N;
+    F* pg = s.pg + (size_t)b * N;
+    F* Sb = s.S + (size_t)b * m * N;
+    F* Yb = s.Y + (size_t)b * m * N;
+    F* ro = s.ro + (size_t)b * m;
+    const F loss = s.loss[b];
+    F t;
+    if (n_iter == 1) {
+        const F gs = pk_canon_sum<F>(N, [&](int k) { return (F)fabs(g[k]); }, red, flip);
+        F gm, unused;
+        pk_own_absmax2<F>(N, g, (F)1, g, (F)1, red, flip, gm, unused);
+        const int active = gm <= (F)prm.tol_grad ? 0 : 1;
+        PK_OWN_LOOP(k, N) {
+            d[k] = -g[k];
+            pg[k] = g[k];
+        }
+        t = (F)1 / gs;
+        t = (t < (F)1 ? t : (F)1) * (F)prm.lr;   // torch.minimum(1, 1/sum|g|) * lr
+        if (!active) t = 0;
+        if (threadIdx.x == 0) {
+            s.active[b] = active;   // read back below by this thread
+            s.hlen[b] = 0;
+            s.hstart[b] = 0;
+            s.evals[b] = 1;
+            s.H[b] = 1;
+            s.loss0[b] = loss;
+        }
+    } else {
+        const F told = s.t[b];
+        int active = s.active[b], hl = s.hlen[b], hs = s.hstart[b];
+        const int evals = s.evals[b] + 1;
+        F H = s.H[b];
+        F sums[2], maxima[2];
+        pk_step_reduce<F>(N, g, pg, d, told, red, flip, sums, maxima);   // its barrier: every thread has read the state
+        const F ys = sums[0], yy = sums[1], gmax = maxima[0], pc = maxima[1];
+        bool fresh = false;
+        if (n_iter > 2 && active && ys > (F)1e-10) {
+            int slot;
+            if (hl < m) { slot = (hs + hl) % m; ++hl; }
+            else { slot = hs; hs = (hs + 1) % m; }
+            F* S = Sb + (size_t)slot * N;
+            F* Y = Yb + (size_t)slot * N;
+            PK_OWN_LOOP(k, N) {
+                Y[k] = pk_rsub(g[k], pg[k]);
+                S[k] = pk_rmul(d[k], told);
+            }
+            H = ys / yy;
+            ro[slot] = (F)1 / ys;   // every thread writes it, and reads what it wrote
+            fresh = true;
+        }
+        if (threadIdx.x == 0) {
+            if (gmax <= (F)prm.tol_grad) active = 0;
+            if (evals >= prm.max_eval) active = 0;
+            if (pc <= (F)prm.tol_change && active) active = 0;
+            const F ploss = s.ploss[b];
+            const F lc = fabs(loss - ploss);
+            if (lc < (F)prm.tol_change && active) active = 0;
+            if (prm.tol_rel_change > 0 && n_iter - 1 > m) {
+                if (lc / (fabs(ploss) + (F)1e-12) < (F)prm.tol_rel_change && active) active = 0;
+            }
+            if (prm.stop_on_cost_increase && loss > s.loss0[b] && active) active = 0;
+            s.active[b] = active;
+            s.evals[b] = evals;
+            s.H[b] = H;
+            s.hlen[b] = hl;
+            s.hstart[b] = hs;
+        }
+        pk_two_loop<F>(g, d, N, Sb, Yb, ro, m, hl, hs, H, al, red, flip, fresh ? pg : nullptr, told);
+        PK_OWN_LOOP(k, N) pg[k] = g[k];
+        t = (F)prm.lr;
+    }
+    F gtd[1], pc[1];
+    pk_direction_reduce<F>(N, g, d, t, red, flip, gtd, pc);
+    if (prm.has_max_step && pc[0] > (F)prm.max_step) t = t * ((F)prm.max_step / pc[0]);
+    if (threadIdx.x == 0) {
+        int active = s.active[b];
+        if (gtd[0] > -(F)prm.tol_change) active = 0;
+        s.t[b] = t;
+        s.ploss[b] = loss;
+        s.active[b] = active;
+        if (active) atomicOr(s.any_active + (n_iter & 1), 1);
+    }
+}
+
+// x += t d for every system if iteration n_iter left any active; tells the host
+// and clears the flag of the next iteration.
+template <typename F>
+__global__ void pk_lbfgs_step_if_kernel(PkLbfgsState<F> s, int n_iter, int* host_flag)
+{
+    const int any = s.any_active[n_iter & 1];
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *host_flag = any;
+        s.any_active[(n_iter + 1) & 1] = 0;
+    }
+    if (!any) return;
+    const size_t total = (size_t)s.M * s.N;
+    for (size_t w = blockIdx.x * (size_t)blockDim.x + threadIdx.x; w < total; w += (size_t)gridDim.x * blockDim.x)
+        s.x[w] = pk_radd(s.x[w], pk_rmul(s.t[w / s.N], s.d[w]));
+}
+
 // One warp per canonical group (so the two-loop keeps its elements in
 // registers), between 2 and 8 warps.
 static inline int pk_lbfgs_threads(int N)
@@ -394,7 +509,7 @@ extern "C" int pk_lbfgs_phase(int phase, int dtype_bytes, void* const* arrays, i
     if (!arrays) return pk_fail(PK_EINVAL, "pk_lbfgs_phase: arrays is NULL%s");
     if (M < 0 || N < 1 || m < 1) return pk_fail(PK_EINVAL, "pk_lbfgs_phase: bad sizes%s");
     cudaStream_t st = (cudaStream_t)stream;
-#define PK_FILL(F)                                                                                     \
+#define PK_LBFGS_FILL(F)                                                                                     \
     PkLbfgsState<F> s;                                                                                 \
     s.x = (F*)arrays[0]; s.g = (F*)arrays[1]; s.loss = (F*)arrays[2]; s.d = (F*)arrays[3];             \
     s.pg = (F*)arrays[4]; s.ploss = (F*)arrays[5]; s.loss0 = (F*)arrays[6]; s.S = (F*)arrays[7];        \
@@ -403,15 +518,53 @@ extern "C" int pk_lbfgs_phase(int phase, int dtype_bytes, void* const* arrays, i
     s.active = (int*)arrays[15]; s.any_active = (int*)arrays[16];                                      \
     s.M = M; s.N = N; s.m = m;
     if (dtype_bytes == 4) {
-        PK_FILL(float)
+        PK_LBFGS_FILL(float)
         return pk_lbfgs_phase<float>(phase, s, n_iter, p0, p1, p2, p3, i1, i2, st);
     } else if (dtype_bytes == 8) {
-        PK_FILL(double)
+        PK_LBFGS_FILL(double)
         return pk_lbfgs_phase<double>(phase, s, n_iter, p0, p1, p2, p3, i1, i2, st);
     }
-#undef PK_FILL
     return pk_fail(PK_EINVAL, "pk_lbfgs_phase: dtype must be float32 or float64%s");
 }
+
+template <typename F>
+static int pk_lbfgs_iterate_launch(const PkLbfgsState<F>& s, int n_iter, const PkLbfgsParams& prm, int* host_flag,
+                                   cudaStream_t st)
+{
+    const size_t smem = ((size_t)s.m + pk_canon_red_len(s.N)) * sizeof(F);
+    cudaError_t err = cudaFuncSetAttribute(pk_lbfgs_iterate_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)smem);
+    if (err != cudaSuccess) return pk_cuda_check(err, "pk_lbfgs_iterate attribute");
+    pk_lbfgs_iterate_kernel<F><<<s.M, pk_lbfgs_threads(s.N), smem, st>>>(s, n_iter, prm);
+    const size_t total = (size_t)s.M * s.N, want = (total + 255) / 256;
+    pk_lbfgs_step_if_kernel<F><<<want < 148 * 8 ? (int)want : 148 * 8, 256, 0, st>>>(s, n_iter, host_flag);
+    return pk_cuda_check(cudaGetLastError(), "pk_lbfgs_iterate launch");
+}
+
+// One iteration of the loop without a line search in two launches instead of
+// four, a memset and a copy: update, direction and stop tests, then the step
+// with the activity flag written where the host reads it.
+extern "C" int pk_lbfgs_iterate(int dtype_bytes, void* const* arrays, int M, int N, int m, int n_iter,
+                                const PkLbfgsParams* prm, int* host_flag, void* stream)
+{
+    if (!arrays || !prm || !host_flag) return pk_fail(PK_EINVAL, "pk_lbfgs_iterate: NULL pointer%s");
+    if (M < 1 || N < 1 || m < 1 || n_iter < 1) return pk_fail(PK_EINVAL, "pk_lbfgs_iterate: bad sizes%s");
+    int* dev_flag = nullptr;
+    const int rc = pk_cuda_check(cudaHostGetDevicePointer((void**)&dev_flag, host_flag, 0),
+                                 "pk_lbfgs_iterate: host_flag must be pinned");
+    if (rc) return rc;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (dtype_bytes == 4) {
+        PK_LBFGS_FILL(float)
+        return pk_lbfgs_iterate_launch<float>(s, n_iter, *prm, dev_flag, st);
+    }
+    if (dtype_bytes == 8) {
+        PK_LBFGS_FILL(double)
+        return pk_lbfgs_iterate_launch<double>(s, n_iter, *prm, dev_flag, st);
+    }
+    return pk_fail(PK_EINVAL, "pk_lbfgs_iterate: dtype must be float32 or float64%s");
+}
+#undef PK_LBFGS_FILL
 
 // ---------------------------------------------------------------------------
 // Fused relaxation: one CTA per packing runs the L-BFGS loop with the

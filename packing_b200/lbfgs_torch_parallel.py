@@ -5,10 +5,10 @@ synchronisations per iteration.
 ``lbfgs(func, x0, ...)`` keeps the reference's signature, defaults and
 semantics (``lbfgs_torch_parallel.py:411-729``): ``func(x, is_main)`` returns
 ``(cost (M,), grad (M, N))``; ``x0`` (M, N) float32 or float64 on a CUDA
-device is updated in place and returned.  Per iteration: direction kernel
-(two-loop recursion, first-step scaling, ``max_step`` clamp, ``g.d`` stop) ->
-one host read of "any system active" -> the step -> history / convergence
-kernel.
+device is updated in place and returned.  Per iteration without a line
+search: one kernel (the last step's history update and convergence tests, the
+two-loop recursion, first-step scaling, ``max_step`` clamp, ``g.d`` stop), the
+step if any system is active, one host read of that.
 
 * ``line_search_fn=None`` (production, ``pack_dynamics.py:39``): every system
   steps by ``t d`` while any system of the batch is active, then ``func`` is
@@ -138,10 +138,13 @@ def lbfgs(func, x0: Tensor, lr: float = 1.0, max_iter: int = 20, max_eval: Optio
         return loss, g
 
     loss, g = call(x)
-    loss = loss.clone()
-    g = g.clone()
     if M == 0:
         return x0
+    if N < 1 or m < 1:
+        raise ValueError("lbfgs: x0 needs columns and history_size must be at least 1")
+    if line_search_fn:   # the search updates both in place
+        loss = loss.clone()
+        g = g.clone()
     z = lambda *s: torch.zeros(*s, dtype=dt, device=dev)   # noqa: E731
     zi = lambda *s: torch.zeros(*s, dtype=torch.int32, device=dev)   # noqa: E731
     d, pg = z(M, N), z(M, N)
@@ -149,7 +152,7 @@ def lbfgs(func, x0: Tensor, lr: float = 1.0, max_iter: int = 20, max_eval: Optio
     S, Y, ro = z(M, m, N), z(M, m, N), z(M, m)
     H, t = z(M), z(M)
     hlen, hstart, evals, active = zi(M), zi(M), zi(M), zi(M)
-    flag = zi(1)
+    flag = zi(2)
     host_flag = torch.zeros(1, dtype=torch.int32, pin_memory=True)
     L = _lib.load()
     nbytes = 4 if dt == torch.float32 else 8
@@ -159,6 +162,28 @@ def lbfgs(func, x0: Tensor, lr: float = 1.0, max_iter: int = 20, max_eval: Optio
         return (ctypes.c_void_p * 17)(*[a.data_ptr() for a in arrays_t])
 
     arr = ptrs()
+    has_ms = max_step is not None
+    n_iter = 0
+    if line_search_fn is None:
+        prm = _lib.PkLbfgsParams(float(lr), float(max_step) if has_ms else 0.0, float(tolerance_grad),
+                                 float(tolerance_change), float(tolerance_rel_change), int(has_ms),
+                                 int(bool(stop_on_cost_increase)), int(max_eval))
+        stream = torch.cuda.current_stream(dev)
+        while n_iter < max_iter:
+            n_iter += 1
+            with _lib.on_device(dev):
+                rc = L.pk_lbfgs_iterate(nbytes, arr, M, N, m, n_iter, ctypes.byref(prm), host_flag.data_ptr(),
+                                        stream.cuda_stream)
+            _lib.check(rc, "lbfgs")
+            stream.synchronize()
+            if not host_flag.item():
+                break
+            if n_iter != max_iter:
+                # the next iteration reads them before func is called again
+                loss, g = call(x)
+                arr[1], arr[2] = g.data_ptr(), loss.data_ptr()
+        x0.copy_(x)
+        return x0
 
     def phase(p, n_iter, p0=0.0, p1=0.0, p2=0.0, i1=0, i2=0):
         with torch.cuda.device(dev):
@@ -167,32 +192,22 @@ def lbfgs(func, x0: Tensor, lr: float = 1.0, max_iter: int = 20, max_eval: Optio
         _lib.check(rc, "lbfgs")
 
     def any_active() -> bool:
-        host_flag.copy_(flag, non_blocking=True)
+        host_flag.copy_(flag[:1], non_blocking=True)
         torch.cuda.current_stream(dev).synchronize()
         return bool(host_flag.item())
 
-    search = _WolfeSearch(L, M, N, dt, dev, x, d, g, loss, t, active, evals) if line_search_fn else None
-    flag.zero_()
+    search = _WolfeSearch(L, M, N, dt, dev, x, d, g, loss, t, active, evals)
     phase(0, 0, tolerance_grad)
     if not any_active():
         x0.copy_(x)
         return x0
-    has_ms = max_step is not None
-    n_iter = 0
     while n_iter < max_iter:
         n_iter += 1
         flag.zero_()
         phase(1, n_iter, lr, max_step if has_ms else 0.0, tolerance_change, i1=int(has_ms))
         if not any_active():
             break
-        if search is not None:
-            search.run(call)
-        else:
-            phase(2, n_iter)
-            if n_iter != max_iter:
-                nl, ng = call(x)
-                loss.copy_(nl)
-                g.copy_(ng)
+        search.run(call)
         phase(3, n_iter, tolerance_grad, tolerance_change, tolerance_rel_change, i1=int(stop_on_cost_increase),
               i2=max_eval)
     x0.copy_(x)

@@ -189,3 +189,50 @@ def test_headline_full_run_final_state_matches_fp64(cuda):
     # the relaxation lowered every packing's cost well below its start
     c0, _, _ = O.compound_cost(xyt.astype(np.float64), h.astype(np.float64), w_area=1e-2, fixed_h=True)
     assert np.all(oc < 0.5 * c0)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("M,N,hist", [(1, 1, 1), (5, 127, 3), (3, 128, 2), (4, 129, 5), (2, 1100, 4)])
+def test_one_kernel_iteration_matches_the_phases(cuda, M, N, hist, dtype):
+    """The loop's fused iteration equals the separate phases (which the line
+    search still uses) bit for bit: group edges of the reductions, more groups than
+    warps, systems that stop early, an objective that returns x itself as gradient."""
+    import ctypes
+
+    from packing_b200 import _lib
+    from packing_b200.lbfgs_torch_parallel import lbfgs
+    g = torch.Generator().manual_seed(N)
+    x0 = torch.randn(M, N, generator=g, dtype=dtype)
+    x0[0] = 0.0 if M > 1 else x0[0]           # zero gradient: inactive from the start
+    x0 = x0.to(cuda)
+    scale = torch.linspace(0.5, 3.0, N, dtype=dtype, device=cuda)
+
+    def func(x, is_main):
+        return 0.5 * (x * x).sum(1), (x if N == 127 else x * scale)
+
+    kw = dict(lr=0.7, max_iter=9, history_size=hist, max_step=0.3, tolerance_grad=0.0, tolerance_change=0.0)
+    got = lbfgs(func, x0.clone(), **kw)
+    # the same loop over the phases
+    L, nb = _lib.load(), 4 if dtype == torch.float32 else 8
+    x = x0.clone()
+    z = lambda *s: torch.zeros(*s, dtype=dtype, device=cuda)   # noqa: E731
+    zi = lambda *s: torch.zeros(*s, dtype=torch.int32, device=cuda)   # noqa: E731
+    loss, grad = (t.clone() for t in func(x, True))
+    arrs = [x, grad, loss, z(M, N), z(M, N), z(M), z(M), z(M, hist, N), z(M, hist, N), z(M, hist), z(M), z(M), zi(M),
+            zi(M), zi(M), zi(M), zi(1)]
+    arr = (ctypes.c_void_p * 17)(*[a.data_ptr() for a in arrs])
+    ph = lambda p, it, a=0., b=0., c=0., i1=0, i2=0: _lib.check(L.pk_lbfgs_phase(   # noqa: E731
+        p, nb, arr, M, N, hist, it, a, b, c, 0., i1, i2, _lib.stream_handle(None, x.device)), "phase")
+    ph(0, 0, 0.0)
+    for it in range(1, 10):
+        arrs[16].zero_()
+        ph(1, it, 0.7, 0.3, 0.0, 1)
+        if not arrs[16].item():
+            break
+        ph(2, it)
+        if it != 9:
+            nl, ng = func(x, True)
+            loss.copy_(nl)
+            grad.copy_(ng)
+        ph(3, it, 0.0, 0.0, 0.0, 0, 9 * 5 // 4)
+    assert torch.equal(got, x)
