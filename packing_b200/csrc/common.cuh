@@ -196,7 +196,9 @@ __device__ __forceinline__ double pk_rsqrt(double a) { return __dsqrt_rn(a); }
 // + 64 entries, alternated by `flip` (one barrier per reduction: a thread can only
 // write a buffer again after the next reduction's barrier, by which time every
 // thread has finished reading it).  All threads call these and all get the
-// result.
+// result.  (The two-loop recursion's own barrier counts only some of the warps:
+// between two reductions of the whole block it stays within the one buffer that
+// the first of them did not use.)
 #define PK_CANON_GROUP 128
 #define PK_OWN_LOOP(k, N)                                                                      \
     for (int _g = (int)(threadIdx.x >> 5); _g * PK_CANON_GROUP < (N); _g += (int)(blockDim.x >> 5)) \

@@ -29,8 +29,11 @@
 // while the current dot product is being reduced, so the chain of 2 hlen
 // dependent reductions does not also wait for a memory round trip per step.
 // Warps without a group leave at once; the rest meet at a barrier of their own.
-// The number of reductions is even, so the caller's flip is unchanged (its next
-// reduction writes the buffer that the last one here did not).
+// A warp that leaves may still be reading the buffer of the reduction before, so
+// the recursion keeps to the two halves (32 ng entries each) of the buffer that
+// flip names next.  The number of reductions is even: the caller's flip is
+// unchanged, and its next reduction may write the lower half, which the last one
+// here did not read, but not the upper one (one sum, like pk_direction_reduce).
 // Both paths perform the same operations in the same order.  Every thread
 // writes the same al[i] and later reads what it wrote: no barrier for it.
 // pg (register path only): the newest entry was appended in this iteration, so
@@ -64,6 +67,8 @@ __device__ void pk_two_loop(const F* g, F* d, int N, const F* S, const F* Y, con
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp >= ng) return;   // owns no element; the others' barrier counts ng warps
+    F* buf = pk_canon_buf(ng, red, flip);
+    int step = 32 * ng;
     const int k0 = warp * PK_CANON_GROUP + lane;
     // this lane's elements are k0 + 32 j for j < nv
     const int nv = k0 < N ? min(4, (N - k0 + 31) >> 5) : 0;
@@ -106,7 +111,6 @@ __device__ void pk_two_loop(const F* g, F* d, int N, const F* S, const F* Y, con
             PK_TL_FETCH(sn, yn, pnext)
             rn = ro[nslot];
         }
-        F* buf = pk_canon_buf(ng, red, flip);
         F p = F(0);
 #pragma unroll
         for (int j = 0; j < 4; ++j)
@@ -114,6 +118,8 @@ __device__ void pk_two_loop(const F* g, F* d, int N, const F* S, const F* Y, con
         buf[warp * 32 + lane] = p;
         pk_warps_barrier(ng);
         const F a = pk_rmul(pk_warp_sum(pk_canon_groups_sum(buf, ng)), rc);
+        buf += step;
+        step = -step;
         al[i] = a;
 #pragma unroll
         for (int j = 0; j < 4; ++j) q[j] = pk_rsub(q[j], pk_rmul(yc[j], a));
@@ -135,7 +141,6 @@ __device__ void pk_two_loop(const F* g, F* d, int N, const F* S, const F* Y, con
             PK_TL_FETCH(sn, yn, pnext)
             rn = ro[nslot];
         }
-        F* buf = pk_canon_buf(ng, red, flip);
         F p = F(0);
 #pragma unroll
         for (int j = 0; j < 4; ++j)
@@ -143,6 +148,8 @@ __device__ void pk_two_loop(const F* g, F* d, int N, const F* S, const F* Y, con
         buf[warp * 32 + lane] = p;
         pk_warps_barrier(ng);
         const F be = pk_rmul(pk_warp_sum(pk_canon_groups_sum(buf, ng)), rc);
+        buf += step;
+        step = -step;
         const F c = pk_rsub(al[i], be);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
