@@ -193,7 +193,7 @@ __device__ __forceinline__ double pk_rsqrt(double a) { return __dsqrt_rn(a); }
 // next reduction.  pk_canon_sum adds each group's per-lane partial in k
 // order, then the groups in order, then a fixed shuffle tree, so the sum
 // depends on N alone, not on blockDim.  red: two buffers of 64 * ngroups
-// + 64 entries, alternated by `flip` (one barrier per reduction: a thread can only
+// entries, alternated by `flip` (one barrier per reduction: a thread can only
 // write a buffer again after the next reduction's barrier, by which time every
 // thread has finished reading it).  All threads call these and all get the
 // result.  (The two-loop recursion's own barrier counts only some of the warps:
@@ -210,16 +210,23 @@ __host__ __device__ inline int pk_canon_groups(int N) { return (N + PK_CANON_GRO
 template <typename T>
 __device__ __forceinline__ T* pk_canon_buf(int ng, T* red, int& flip)
 {
-    T* buf = red + (flip ? 64 * ng + 64 : 0);
+    T* buf = red + (flip ? 64 * ng : 0);
     flip ^= 1;
     return buf;
 }
 
-// The maxima's part of the buffer that pk_canon_buf handed out last.
-template <typename T>
-__device__ __forceinline__ T* pk_canon_max_buf(int ng, T* red, int flip)
+// Whether two maxima get room of their own behind the buffers (8 warps' worth
+// of each), so that one barrier serves them and the sums.  Only where shared
+// memory is never short of it: beyond 1024 elements, or with a history whose
+// coefficients lie in shared memory beside them, the last bytes can decide
+// whether a launch is possible, and the maxima take a buffer in their turn.
+#define PK_CANON_MAX_WARPS 8
+__host__ __device__ inline bool pk_canon_joint(int N, int m) { return N <= 1024 && m <= 1024; }
+
+// Entries of red for N elements and a history of m.
+__host__ __device__ inline int pk_canon_red_len(int N, int m)
 {
-    return red + (flip ? 0 : 64 * ng + 64) + 64 * ng;
+    return 128 * pk_canon_groups(N) + (pk_canon_joint(N, m) ? 4 * PK_CANON_MAX_WARPS : 0);
 }
 
 // Warp maximum, NaN ignored (redux.sync takes floats on sm_100a).
@@ -292,17 +299,18 @@ __device__ __forceinline__ T pk_canon_sum(int N, Get get, T* red, int& flip)
 }
 
 // NS canonical sums (each bit-identical to its own pk_canon_sum) and NM maxima
-// of absolute values (a maximum does not depend on the order; it starts from 0)
-// with one barrier.  get(k, s, m) gives the NS addends and NM values of element
-// k.  NS * ng * 32 + NM * warps entries of one buffer (64 ng of them).
+// of absolute values (a maximum does not depend on the order; it starts from 0):
+// at most two of each, in blocks of at most 8 warps.  get(k, s, m) gives the NS
+// addends and NM values of element k.  joint: pk_canon_joint of the red at hand;
+// one barrier then, three otherwise.
 template <int NS, int NM, typename T, typename Get>
-__device__ __forceinline__ void pk_canon_reduce(int N, Get get, T* red, int& flip, T (&rs)[NS], T (&rm)[NM])
+__device__ __forceinline__ void pk_canon_reduce(int N, Get get, T* red, int& flip, bool joint, T (&rs)[NS], T (&rm)[NM])
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nw = blockDim.x >> 5;
     const int ng = pk_canon_groups(N);
+    T* mbuf = red + 128 * ng + (flip ? 2 * PK_CANON_MAX_WARPS : 0);
     T* buf = pk_canon_buf(ng, red, flip);
-    T* mbuf = pk_canon_max_buf(ng, red, flip);
     T m[NM];
 #pragma unroll
     for (int i = 0; i < NM; ++i) m[i] = T(0);
@@ -324,15 +332,20 @@ __device__ __forceinline__ void pk_canon_reduce(int N, Get get, T* red, int& fli
         for (int i = 0; i < NS; ++i) buf[(i * ng + grp) * 32 + lane] = s[i];
     }
 #pragma unroll
-    for (int i = 0; i < NM; ++i) {
-        m[i] = pk_warp_max(m[i]);
-        if (lane == 0) mbuf[32 * i + warp] = m[i];
+    for (int i = 0; i < NM; ++i) m[i] = pk_warp_max(m[i]);
+    if (!joint) {
+        __syncthreads();
+        mbuf = pk_canon_buf(ng, red, flip);
     }
+#pragma unroll
+    for (int i = 0; i < NM; ++i)
+        if (lane == 0) mbuf[PK_CANON_MAX_WARPS * i + warp] = m[i];
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < NM; ++i) rm[i] = pk_warp_max(lane < nw ? mbuf[32 * i + lane] : T(0));
+    for (int i = 0; i < NM; ++i) rm[i] = pk_warp_max(lane < nw ? mbuf[PK_CANON_MAX_WARPS * i + lane] : T(0));
 #pragma unroll
     for (int i = 0; i < NS; ++i) rs[i] = pk_warp_sum(pk_canon_groups_sum(buf + i * ng * 32, ng));
+    if (!joint) __syncthreads();   // both buffers have been read
 }
 
 // Maxima of two element functions over the owned elements with one barrier.
@@ -342,8 +355,7 @@ __device__ __forceinline__ void pk_canon_max2(int N, Get get, T* red, int& flip,
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nw = blockDim.x >> 5;
-    pk_canon_buf(pk_canon_groups(N), red, flip);   // keeps the buffers alternating
-    T* buf = pk_canon_max_buf(pk_canon_groups(N), red, flip);
+    T* buf = pk_canon_buf(pk_canon_groups(N), red, flip);
     T a = T(0), b = T(0);
     PK_OWN_LOOP(k, N) {
         T u, v;
@@ -361,10 +373,6 @@ __device__ __forceinline__ void pk_canon_max2(int N, Get get, T* red, int& flip,
     r0 = pk_warp_max(lane < nw ? buf[lane] : T(0));
     r1 = pk_warp_max(lane < nw ? buf[32 + lane] : T(0));
 }
-
-// Both buffers of the canonical reductions: 64 per group (two sums) and 64 for
-// two maxima of at most 32 warps.
-__host__ __device__ inline int pk_canon_red_len(int N) { return 2 * (64 * pk_canon_groups(N) + 64); }
 
 // Bounded wrap of an angle difference into [-pi, pi], following the
 // reference's subtract-2pi loop (pack_cuda_lut.py:289-293) in FP32.  Angles

@@ -182,7 +182,7 @@ __device__ __forceinline__ void pk_own_absmax2(int N, const F* v, F scale, const
 // y = g - pg, s = t d (the curvature), max|g| and max|t d| (the stop tests).
 template <typename F>
 __device__ __forceinline__ void pk_step_reduce(int N, const F* g, const F* pg, const F* d, F t, F* red, int& flip,
-                                               F (&sums)[2], F (&maxima)[2])
+                                               bool joint, F (&sums)[2], F (&maxima)[2])
 {
     pk_canon_reduce<2, 2, F>(N, [&](int k, F (&s)[2], F (&m)[2]) {
         const F y = pk_rsub(g[k], pg[k]), st = pk_rmul(d[k], t);
@@ -190,18 +190,18 @@ __device__ __forceinline__ void pk_step_reduce(int N, const F* g, const F* pg, c
         s[1] = pk_rmul(y, y);
         m[0] = (F)fabs(g[k]);
         m[1] = (F)fabs(st);
-    }, red, flip, sums, maxima);
+    }, red, flip, joint, sums, maxima);
 }
 
 // Of a direction, with one barrier: g.d and max|t d|.
 template <typename F>
 __device__ __forceinline__ void pk_direction_reduce(int N, const F* g, const F* d, F t, F* red, int& flip,
-                                                    F (&gtd)[1], F (&pc)[1])
+                                                    bool joint, F (&gtd)[1], F (&pc)[1])
 {
     pk_canon_reduce<1, 1, F>(N, [&](int k, F (&s)[1], F (&m)[1]) {
         s[0] = pk_rmul(g[k], d[k]);
         m[0] = (F)fabs(pk_rmul(d[k], t));
-    }, red, flip, gtd, pc);
+    }, red, flip, joint, gtd, pc);
 }
 
 // ---------------------------------------------------------------------------
@@ -251,7 +251,7 @@ __global__ void pk_lbfgs_direction_kernel(PkLbfgsState<F> s, int n_iter, F lr, F
         t = lr;
     }
     F gtd[1], pc[1];
-    pk_direction_reduce<F>(N, g, d, t, red, flip, gtd, pc);
+    pk_direction_reduce<F>(N, g, d, t, red, flip, pk_canon_joint(N, s.m), gtd, pc);
     if (has_max_step && pc[0] > max_step) t = t * (max_step / pc[0]);
     if (gtd[0] > -tol_change) active = 0;
     if (threadIdx.x == 0) {
@@ -292,7 +292,7 @@ __global__ void pk_lbfgs_update_kernel(PkLbfgsState<F> s, int n_iter, F tol_grad
     int active = s.active[b];
     int evals = s.evals[b] + 1;
     F sums[2], maxima[2];
-    pk_step_reduce<F>(N, g, pg, d, t, red, flip, sums, maxima);
+    pk_step_reduce<F>(N, g, pg, d, t, red, flip, pk_canon_joint(N, m), sums, maxima);
     const F ys = sums[0], yy = sums[1], gmax = maxima[0], pc = maxima[1];
     if (n_iter > 1) {
         if (active && ys > (F)1e-10) {
@@ -400,7 +400,8 @@ __global__ void pk_lbfgs_iterate_kernel(PkLbfgsState<F> s, int n_iter, PkLbfgsPa
         const int evals = s.evals[b] + 1;
         F H = s.H[b];
         F sums[2], maxima[2];
-        pk_step_reduce<F>(N, g, pg, d, told, red, flip, sums, maxima);   // its barrier: every thread has read the state
+        // its barrier: every thread has read the state
+        pk_step_reduce<F>(N, g, pg, d, told, red, flip, pk_canon_joint(N, m), sums, maxima);
         const F ys = sums[0], yy = sums[1], gmax = maxima[0], pc = maxima[1];
         bool fresh = false;
         if (n_iter > 2 && active && ys > (F)1e-10) {
@@ -439,7 +440,7 @@ __global__ void pk_lbfgs_iterate_kernel(PkLbfgsState<F> s, int n_iter, PkLbfgsPa
         t = (F)prm.lr;
     }
     F gtd[1], pc[1];
-    pk_direction_reduce<F>(N, g, d, t, red, flip, gtd, pc);
+    pk_direction_reduce<F>(N, g, d, t, red, flip, pk_canon_joint(N, m), gtd, pc);
     if (prm.has_max_step && pc[0] > (F)prm.max_step) t = t * ((F)prm.max_step / pc[0]);
     if (threadIdx.x == 0) {
         int active = s.active[b];
@@ -480,7 +481,7 @@ static int pk_lbfgs_phase(int phase, const PkLbfgsState<F>& s, int n_iter, doubl
                           int i1, int i2, cudaStream_t st)
 {
     const int T = pk_lbfgs_threads(s.N);
-    const size_t smem = ((size_t)s.m + pk_canon_red_len(s.N)) * sizeof(F);
+    const size_t smem = ((size_t)s.m + pk_canon_red_len(s.N, s.m)) * sizeof(F);
     if (s.M == 0) return PK_OK;
     cudaError_t err = cudaSuccess;
     switch (phase) {
@@ -538,7 +539,7 @@ template <typename F>
 static int pk_lbfgs_iterate_launch(const PkLbfgsState<F>& s, int n_iter, const PkLbfgsParams& prm, int* host_flag,
                                    cudaStream_t st)
 {
-    const size_t smem = ((size_t)s.m + pk_canon_red_len(s.N)) * sizeof(F);
+    const size_t smem = ((size_t)s.m + pk_canon_red_len(s.N, s.m)) * sizeof(F);
     cudaError_t err = cudaFuncSetAttribute(pk_lbfgs_iterate_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)smem);
     if (err != cudaSuccess) return pk_cuda_check(err, "pk_lbfgs_iterate attribute");
@@ -628,7 +629,7 @@ __device__ bool pk_relax_iterate(float* x, float* g, float* pg, float* d, float*
                 // after a step (:632-724)
                 ++v.evals;
                 float sums[2], maxima[2];
-                pk_step_reduce<float>(N, g, pg, d, v.t, red, flip, sums, maxima);
+                pk_step_reduce<float>(N, g, pg, d, v.t, red, flip, pk_canon_joint(N, m), sums, maxima);
                 const float ys = sums[0], yy = sums[1], gmax = maxima[0], pc = maxima[1];
                 if (v.it > 1 && ys > 1e-10f) {
                     int slot;
@@ -679,7 +680,7 @@ __device__ bool pk_relax_iterate(float* x, float* g, float* pg, float* d, float*
             t = prm.lr;
         }
         float gtd[1], pc[1];
-        pk_direction_reduce<float>(N, g, d, t, red, flip, gtd, pc);
+        pk_direction_reduce<float>(N, g, d, t, red, flip, pk_canon_joint(N, m), gtd, pc);
         if (prm.has_max_step && pc[0] > prm.max_step) t = t * (prm.max_step / pc[0]);
         v.t = t;
         if (gtd[0] > -prm.tol_change) { v.active = 0; --v.it; return true; }
@@ -872,7 +873,7 @@ static size_t pk_relax_smem_bytes(int n_max, int sym, int cap_near, int cap_item
 {
     const int NM = 3 * n_max + 3;
     return pk_cost_smem_bytes(n_max * sym, cap_near, cap_items, true) +
-           ((size_t)4 * NM + 2 * (size_t)m + pk_canon_red_len(NM)) * 4;
+           ((size_t)4 * NM + 2 * (size_t)m + pk_canon_red_len(NM, m)) * 4;
 }
 
 // Threads per CTA of the relaxation kernels: the caller's choice (an

@@ -325,7 +325,7 @@ static int pk_wolfe_phase_t(int phase, const PkWolfeState<F>& s, int ls_iter, do
 {
     if (s.M == 0) return PK_OK;
     const int T = pk_lbfgs_threads(s.N);
-    const size_t smem = (size_t)pk_canon_red_len(s.N) * sizeof(F);
+    const size_t smem = (size_t)pk_canon_red_len(s.N, 0) * sizeof(F);
     switch (phase) {
         case 0: pk_wolfe_init_kernel<F><<<s.M, T, smem, st>>>(s); break;
         case 1: pk_wolfe_after_eval_kernel<F><<<s.M, T, smem, st>>>(s, flag_arg); break;

@@ -52,6 +52,6 @@ def emulator(tmp_path_factory):
 # owning one group (8 of 8), and more groups than warps
 @pytest.mark.parametrize("N,threads", [(100, 64), (128, 64), (603, 256), (30, 256), (1024, 256), (300, 64), (1153, 256)])
 def test_results_do_not_depend_on_which_warp_runs_ahead(emulator, N, threads):
-    for m in (1, 3):
-        r = subprocess.run([emulator, str(N), str(m), str(threads)], capture_output=True, text=True, timeout=120)
+    for m in (1, 3) + ((1030,) if N in (100, 603) else ()):   # 1030: the maxima have no room beside the sums
+        r = subprocess.run([emulator, str(N), str(m), str(threads)], capture_output=True, text=True, timeout=300)
         assert r.returncode == 0, r.stdout + r.stderr
