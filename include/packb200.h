@@ -126,7 +126,11 @@ int pk_cost_ordered(const float* xyt, const int* offsets, const int* order, int 
  * order[start .. start + count - 1] (the classes cover it once), none with more
  * than n_max trees, on CTAs of `threads` (0: the library's choice), on
  * stream side[k], forked from and joined to `stream` (a single class runs on
- * `stream` itself).  The same results as one launch. */
+ * `stream` itself).  A batch that the GPU takes in a few waves of the largest
+ * class's CTAs goes in one launch on `stream` instead, with the library's choice
+ * of threads; the classes' bounds hold all the same (a packing beyond its
+ * class's n_max costs NaN), and a class with bad threads or n_max is refused.
+ * The same results either way. */
 typedef struct PkSizeClass { int start, count, n_max, threads; } PkSizeClass;
 int pk_cost_classes(const float* xyt, const int* offsets, const int* order, const PkSizeClass* classes, int n_classes,
                     int E, int n_max, const float* h, const PkCostSpec* spec, float* cost, float* grad, float* grad_h,

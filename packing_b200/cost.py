@@ -54,8 +54,9 @@ def compound_cost(xyt, h, spec: CostSpec = CostSpec(), offsets=None, n_max=None,
     """Fused compound cost and gradient.  Uniform batch: ``xyt`` (E, n, 3).
     Ragged batch: ``xyt`` (sum n, 3) with int32 ``offsets`` (E+1,) on the
     device and ``n_max`` >= every instance's tree count; with a largest-first
-    ``order`` and its ``classes`` (``classes.ragged_plan``), one launch per
-    size class side by side, bit-identical to one launch."""
+    ``order`` and its ``classes`` (``classes.ragged_plan``), the size classes
+    side by side or in one launch, whichever is faster, bit-identical to one
+    launch without classes."""
     x = _lib.as_tensor(xyt, "xyt")
     _lib.check_f32(x, "xyt")
     if offsets is None:
@@ -101,14 +102,15 @@ def compound_cost(xyt, h, spec: CostSpec = CostSpec(), offsets=None, n_max=None,
 
 
 def launch_cost_classes(x, off, order, E, n_max, h, cs, cost, grad, grad_h, classes, stream, what):
-    """One pk_cost_ordered launch per size class, side by side on forked streams."""
+    """The size classes of a largest-first order in one call: side by side on
+    forked streams, or in one launch where that is faster (pk_cost_classes)."""
     from .classes import side_streams
     if off is None or order is None:
         raise ValueError(f"{what}: classes need a ragged batch with a largest-first order")
     if sum(c.count for c in classes) != E or any(c.n_max > n_max for c in classes):
         raise ValueError(f"{what}: classes must cover the order once, each within n_max")
     k = len(classes)
-    table = (_lib.PkSizeClass * k)(*[(c.start, c.count, c.n_max, c.threads) for c in classes])
+    table = (_lib.PkSizeClass * k)(*[(c.start, c.count, c.n_max, int(c.threads)) for c in classes])
     side = (ctypes.c_void_p * k)(*[s.cuda_stream for s in side_streams(x.device, k)])
     with _lib.on_device(x.device):
         rc = _lib.load().pk_cost_classes(_lib.ptr(x), _lib.ptr(off), _lib.ptr(order), table, k, E, int(n_max),

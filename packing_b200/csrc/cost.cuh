@@ -1410,23 +1410,38 @@ __device__ double pk_eval_instance(const float* X, int ng, const float* H, const
     return total;
 }
 
+// The size classes of an order that one launch covers: position b of the order
+// belongs to the first class whose end lies beyond it (all ends 0: no classes).
+// A build of its own reads them (CLASSES; 2000 packings of 5 to 200 trees, LUT:
+// 39 -> 42 us): read by every launch they cost the six forked ones of a large
+// batch 18 of 111 us, whose parameters together then no longer fit the SM's
+// constant cache.
+#define PK_MAX_BOUNDS 8
+struct PkClassBounds { unsigned c[PK_MAX_BOUNDS]; };   // end << 11 | n_max
+
 // CTA b costs instance order[b] (instance b without an order).  The LUT
 // mode has no clipper: it fits 64 registers without spilling, so four CTAs of
 // 256 threads share an SM and one CTA's broad phase overlaps the others'
 // gathers (4096 x n = 200: 0.201 -> 0.183 ms, the same bits).
-template <int MODE, bool SYM>
+template <int MODE, bool SYM, bool CLASSES>
 __global__ void __launch_bounds__(256, MODE == PK_PAIR_LUT ? 4 : 3) pk_cost_kernel(const float* __restrict__ xyt, const int* __restrict__ offsets,
                                const int* __restrict__ order, int E,
                                int n_max, const float* __restrict__ h, PkCostSpec spec,
                                float* __restrict__ cost, float* __restrict__ grad,
-                               float* __restrict__ grad_h, int cap_near, int cap_items)
+                               float* __restrict__ grad_h, int cap_near, int cap_items, const PkClassBounds cls)
 {
     extern __shared__ __align__(16) unsigned char pk_smem[];
     const int e = order ? order[blockIdx.x] : blockIdx.x;
+    int most = n_max;
+    if (CLASSES)
+#pragma unroll
+        for (int c = PK_MAX_BOUNDS - 1; c >= 0; --c)
+            if (blockIdx.x < (cls.c[c] >> 11)) most = cls.c[c] & 2047;
+
     if (e < 0 || e >= E) return;
     const int base = offsets ? offsets[e] : e * n_max;
     const int n = offsets ? offsets[e + 1] - base : n_max;
-    if (n < 0 || n > n_max) {
+    if (n < 0 || n > most) {
         if (threadIdx.x == 0) cost[e] = __int_as_float(0x7fc00000);   // NaN marks a bad offset
         return;
     }
@@ -1474,7 +1489,7 @@ static inline int pk_cost_threads(int n_max, int count)
 // Raises a kernel's dynamic shared memory limit only when a launch needs more
 // than any earlier one on this device, so warmed-up launches make no
 // attribute call (they can then be captured into a CUDA graph).  Slots: 0-3 and
-// 28-31 the cost kernels, 4-19, 32-39 the relaxation's, 20-27 the jobs'.
+// 28-31, 40-47 the cost kernels, 4-19, 32-39 the relaxation's, 20-27 the jobs'.
 static cudaError_t pk_set_smem(const void* fn, int slot, size_t smem)
 {
     static size_t done[64][48];
@@ -1495,12 +1510,15 @@ static cudaError_t pk_set_smem(const void* fn, int slot, size_t smem)
     return err;
 }
 
-// count entries of the launch order (all E instances when order is NULL);
-// threads 0 = pk_cost_threads of the size bound.
-static int pk_launch_cost(const float* xyt, const int* offsets, const int* order, int count, int E, int n_max,
-                          const float* h, const PkCostSpec* spec, int threads, float* cost, float* grad,
-                          float* grad_h, cudaStream_t st)
+// Checks the arguments of a cost launch of count instances with at most n_max
+// trees, and gives its threads (threads 0: pk_cost_threads of the size bound) and
+// shared memory.  *T = 0: nothing to do.
+struct PkCostLaunch { int T, cap_near, cap_items; size_t smem; };
+
+static int pk_cost_args(const float* xyt, const int* order, int count, int E, int n_max, const float* h,
+                        const PkCostSpec* spec, int threads, const float* cost, PkCostLaunch* L)
 {
+    L->T = 0;
     int rc = pk_check_init();
     if (rc) return rc;
     if (!spec) return pk_fail(PK_EINVAL, "pk_cost: spec is NULL%s");
@@ -1508,44 +1526,54 @@ static int pk_launch_cost(const float* xyt, const int* offsets, const int* order
     if (count < 0 || count > E) return pk_fail(PK_EINVAL, "pk_cost: order count must be in [0, E]%s");
     if (count < E && !order) return pk_fail(PK_EINVAL, "pk_cost: a partial launch needs an order%s");
     if (E == 0 || count == 0) return PK_OK;
-    if (spec && spec->symmetry != 0 && spec->symmetry != 1 && spec->symmetry != 2 && spec->symmetry != 4)
+    if (spec->symmetry != 0 && spec->symmetry != 1 && spec->symmetry != 2 && spec->symmetry != 4)
         return pk_fail(PK_EINVAL, "pk_cost: symmetry must be 0, 1, 2 or 4%s");
-    if (n_max > PK_MAX_TREES || (spec && (long long)n_max * pk_symmetry(*spec) > PK_MAX_TREES))
+    if (n_max > PK_MAX_TREES || (long long)n_max * pk_symmetry(*spec) > PK_MAX_TREES)
         return pk_fail(PK_ERANGE, "pk_cost: more than 1024 (phenotype) trees per instance%s");
     if (!cost || (!xyt && n_max > 0)) return pk_fail(PK_EINVAL, "pk_cost: xyt and cost are required%s");
     if (spec->w_boundary != 0.f && !h) return pk_fail(PK_EINVAL, "pk_cost: boundary term needs h%s");
     if (spec->w_area != 0.f && !h) return pk_fail(PK_EINVAL, "pk_cost: area term needs h%s");
+    if (spec->pair_mode < PK_PAIR_NONE || spec->pair_mode > PK_PAIR_LUT)
+        return pk_fail(PK_EINVAL, "pk_cost: unknown pair_mode%s");
     if (spec->pair_mode == PK_PAIR_LUT) {
-        const PkLut& L = spec->lut;
-        if (!L.vals || L.nx < 2 || L.ny < 2 || L.nt < 2)
+        const PkLut& l = spec->lut;
+        if (!l.vals || l.nx < 2 || l.ny < 2 || l.nt < 2)
             return pk_fail(PK_EINVAL, "pk_cost: LUT needs vals and at least 2 points per axis%s");
     }
-    int T = pk_cost_threads(n_max * pk_symmetry(*spec), count);
-    if (threads != 0) {
-        if (threads < 32 || threads > 256 || (threads & 31) || 8 * threads < n_max * pk_symmetry(*spec) - 1)
-            return pk_fail(PK_EINVAL, "pk_cost: threads must be 0 or a multiple of 32 in [32, 256] with "
-                                      "8 * threads >= n - 1%s");
-        T = threads;
-    }
-    int cap_near, cap_items;
-    pk_caps(T, spec->pair_mode, &cap_near, &cap_items);
-    const size_t smem = pk_cost_smem_bytes(n_max * pk_symmetry(*spec), cap_near, cap_items);
+    const int n = n_max * pk_symmetry(*spec);
+    if (threads != 0 && (threads < 32 || threads > 256 || (threads & 31) || 8 * threads < n - 1))
+        return pk_fail(PK_EINVAL, "pk_cost: threads must be 0 or a multiple of 32 in [32, 256] with "
+                                  "8 * threads >= n - 1%s");
+    L->T = threads != 0 ? threads : pk_cost_threads(n, count);
+    pk_caps(L->T, spec->pair_mode, &L->cap_near, &L->cap_items);
+    L->smem = pk_cost_smem_bytes(n, L->cap_near, L->cap_items);
+    return PK_OK;
+}
+
+// count entries of the launch order (all E instances when order is NULL).
+static int pk_launch_cost(const float* xyt, const int* offsets, const int* order, int count, int E, int n_max,
+                          const float* h, const PkCostSpec* spec, int threads, float* cost, float* grad,
+                          float* grad_h, cudaStream_t st, const PkClassBounds* classes = nullptr)
+{
+    PkCostLaunch L;
+    const int rc = pk_cost_args(xyt, order, count, E, n_max, h, spec, threads, cost, &L);
+    if (rc || L.T == 0) return rc;
+    const PkClassBounds cls = classes ? *classes : PkClassBounds{};
     cudaError_t err = cudaSuccess;
     switch (spec->pair_mode) {
+#define PK_CASE2(M, S, C, SLOT)                                                                     \
+    {                                                                                               \
+        err = pk_set_smem((const void*)pk_cost_kernel<M, S, C>, SLOT, L.smem);                      \
+        if (err == cudaSuccess)                                                                     \
+            pk_cost_kernel<M, S, C><<<count, L.T, L.smem, st>>>(xyt, offsets, order, E, n_max, h, *spec, cost, grad, \
+                                                                grad_h, L.cap_near, L.cap_items, cls); \
+    }
 #define PK_CASE(M)                                                                                  \
     case M:                                                                                         \
-        if (spec->symmetry > 1) {                                                                   \
-            err = pk_set_smem((const void*)pk_cost_kernel<M, true>, 28 + M, smem);                  \
-            if (err == cudaSuccess)                                                                 \
-                pk_cost_kernel<M, true><<<count, T, smem, st>>>(xyt, offsets, order, E, n_max, h, *spec, \
-                                                                cost, grad, grad_h, cap_near, cap_items); \
-        } else {                                                                                    \
-            err = pk_set_smem((const void*)pk_cost_kernel<M, false>, M, smem);                      \
-            if (err == cudaSuccess)                                                                 \
-                pk_cost_kernel<M, false><<<count, T, smem, st>>>(xyt, offsets, order, E, n_max, h,    \
-                                                                 *spec, cost, grad, grad_h, cap_near, \
-                                                                 cap_items);                          \
-        }                                                                                           \
+        if (classes && spec->symmetry > 1) PK_CASE2(M, true, true, 44 + M)                          \
+        else if (classes) PK_CASE2(M, false, true, 40 + M)                                          \
+        else if (spec->symmetry > 1) PK_CASE2(M, true, false, 28 + M)                               \
+        else PK_CASE2(M, false, false, M)                                                           \
         if (err == cudaSuccess) err = cudaGetLastError();                                           \
         break;
         PK_CASE(PK_PAIR_NONE)
@@ -1553,8 +1581,7 @@ static int pk_launch_cost(const float* xyt, const int* offsets, const int* order
         PK_CASE(PK_PAIR_SEP)
         PK_CASE(PK_PAIR_LUT)
 #undef PK_CASE
-        default:
-            return pk_fail(PK_EINVAL, "pk_cost: unknown pair_mode%s");
+#undef PK_CASE2
     }
     return pk_cuda_check(err, "pk_cost launch");
 }
@@ -1576,8 +1603,9 @@ extern "C" int pk_cost_ordered(const float* xyt, const int* offsets, const int* 
 }
 
 // The size classes of a largest-first order, class k on side[k], forked from and
-// joined to stream: one call instead of a launch and five event calls per class
-// from Python (16 us each, 100 for a ragged batch whose kernels take 100).
+// joined to stream, or in one launch on stream: one call instead of a launch and
+// five event calls per class from Python (16 us each, 100 for a ragged batch
+// whose kernels take 100).
 extern "C" int pk_cost_classes(const float* xyt, const int* offsets, const int* order, const PkSizeClass* cls,
                                int ncls, int E, int n_max, const float* h, const PkCostSpec* spec, float* cost,
                                float* grad, float* grad_h, void* stream, void* const* side)
@@ -1597,11 +1625,33 @@ extern "C" int pk_cost_classes(const float* xyt, const int* offsets, const int* 
     cudaStream_t base = (cudaStream_t)stream;
     if (ncls == 1)
         return pk_launch_cost(xyt, offsets, order, E, E, cls[0].n_max, h, spec, cls[0].threads, cost, grad, grad_h, base);
-    // Forking and joining takes about 20 us: one launch is faster up to 16
-    // packings per SM (LUT cost, 5 to 200 trees: 1000 packings 26 us against 46,
-    // 3000 58 against 55, 8192 133 against 105).
-    if (E <= 16 * pk_sm_count())
-        return pk_launch_cost(xyt, offsets, order, E, E, most, h, spec, 0, cost, grad, grad_h, base);
+    // One launch does without forking and joining (about 20 us), but gives every
+    // packing the CTA of the largest one.  It is faster while the GPU takes the
+    // batch in a few waves of such CTAs; by (E / resident CTAs), one launch
+    // against forked, in us:
+    //   LUT, 5 to 200 trees:  3.4  38 / 52,  5.1  58 / 55;  5 to 900:  3.4  54 / 62,  6.8  95 / 75,  14  184 / 128
+    //   area, 5 to 200: 1.1  30 / 43,  4.5  75 / 72;  5 to 900: 3.4  95 / 114,  6.8  155 / 138,  14  305 / 230
+    //   separation, 5 to 200:  4.5  85 / 88;  2000 of 10 trees and one of 900, LUT:  14  80 / 58
+    PkClassBounds bounds = {};
+    bool one = E <= 16 * pk_sm_count() && ncls <= PK_MAX_BOUNDS;
+    for (int k = 0, at = 0; k < ncls && one; ++k) {
+        one = cls[k].start == at;   // positions left out or named twice: class by class
+        at += cls[k].count;
+        bounds.c[k] = ((unsigned)at << 11) | (unsigned)(cls[k].n_max & 2047);   // n_max <= 1024 is checked below
+    }
+    if (one) {
+        PkCostLaunch L;
+        for (int k = 0; k < ncls; ++k) {   // what a class of its own refuses stays refused
+            const int rc = pk_cost_args(xyt, order, cls[k].count, E, cls[k].n_max, h, spec, cls[k].threads, cost, &L);
+            if (rc) return rc;
+        }
+        const int rc = pk_cost_args(xyt, order, E, E, most, h, spec, 0, cost, &L);
+        if (rc || L.T == 0) return rc;
+        const int by_regs = (spec->pair_mode == PK_PAIR_LUT ? 1024 : 768) / L.T;   // the kernel's launch bounds
+        const int by_smem = (int)((size_t)228 * 1024 / (L.smem + 1024));
+        if (E <= 5LL * pk_sm_count() * (by_smem < by_regs ? by_smem : by_regs))
+            return pk_launch_cost(xyt, offsets, order, E, E, most, h, spec, 0, cost, grad, grad_h, base, &bounds);
+    }
     cudaEvent_t fork = nullptr, join = nullptr;
     cudaError_t err = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
     if (err == cudaSuccess) err = cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
