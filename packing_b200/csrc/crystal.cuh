@@ -162,11 +162,11 @@ extern "C" int pk_overlap_crystal(const float* xyt, int E, int n, int use_separa
     cudaStream_t st = (cudaStream_t)stream;
     cudaError_t err;
     if (use_separation) {
-        err = cudaFuncSetAttribute(pk_crystal_kernel<PK_PAIR_SEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        err = pk_raise_smem((const void*)pk_crystal_kernel<PK_PAIR_SEP>, smem);
         if (err == cudaSuccess)
             pk_crystal_kernel<PK_PAIR_SEP><<<E, T, smem, st>>>(xyt, crystal_axes, E, n, only_self, n_periodic, cost, grad);
     } else {
-        err = cudaFuncSetAttribute(pk_crystal_kernel<PK_PAIR_AREA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        err = pk_raise_smem((const void*)pk_crystal_kernel<PK_PAIR_AREA>, smem);
         if (err == cudaSuccess)
             pk_crystal_kernel<PK_PAIR_AREA><<<E, T, smem, st>>>(xyt, crystal_axes, E, n, only_self, n_periodic, cost, grad);
     }

@@ -4,6 +4,8 @@
 
 #include <string.h>
 
+#include <mutex>
+
 static thread_local char g_pk_err[512] = "";
 static bool g_pk_inited[64];
 // pk_init calls per device: a cached device address (pk_relax_noalloc's
@@ -23,6 +25,21 @@ static int pk_cuda_check(cudaError_t e, const char* where)
     if (e == cudaSuccess) return PK_OK;
     snprintf(g_pk_err, sizeof(g_pk_err), "%s: %s", where, cudaGetErrorString(e));
     return PK_ECUDA;
+}
+
+// Raises a kernel's dynamic shared memory limit to what a launch needs.  Never
+// lowers it: the limit belongs to the process, and another thread may be between
+// this call and a larger launch.  The limit is asked for and not remembered, so
+// it holds in a context made anew, too (kernels that are launched many times per
+// call keep it by slot: pk_set_smem).
+static cudaError_t pk_raise_smem(const void* fn, size_t smem)
+{
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    cudaFuncAttributes a;
+    const cudaError_t err = cudaFuncGetAttributes(&a, fn);
+    if (err != cudaSuccess || (size_t)a.maxDynamicSharedSizeBytes >= smem) return err;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
 static int pk_check_init()

@@ -284,8 +284,7 @@ static cudaError_t pk_lap_staged_slots(int N, long long* slots)
     const size_t ssm = pk_lap_smem_bytes(N);
     if (ssm > PK_LAP_SMEM_MAX) return cudaSuccess;
     int dev = 0, sms = 0, per_sm = 0;
-    cudaError_t err = cudaFuncSetAttribute(pk_hungarian_smem_kernel<CPL, VEC>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm);
+    cudaError_t err = pk_raise_smem((const void*)pk_hungarian_smem_kernel<CPL, VEC>, ssm);
     if (err == cudaSuccess) err = cudaGetDevice(&dev);
     if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (err == cudaSuccess)
@@ -604,8 +603,7 @@ extern "C" int pk_diversity_matrix(const float* pop, const float* ref, int Np, i
     switch (cpl) {
 #define PK_D(K)                                                                                        \
     case K:                                                                                            \
-        err = cudaFuncSetAttribute(pk_diversity_lap_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                   (int)smem);                                                         \
+        err = pk_raise_smem((const void*)pk_diversity_lap_kernel<K>, smem);                            \
         if (err == cudaSuccess) pk_diversity_lap_kernel<K><<<Np * Nr, 256, smem, st>>>(pop, ref, Np, Nr, n, ntf, out); \
         break;
         PK_D(1) PK_D(2) PK_D(3) PK_D(4) PK_D(5) PK_D(6) PK_D(7) PK_D(8)
@@ -660,8 +658,7 @@ static int pk_diversity_launch(const float* pop, const float* ref, int Np, int N
     const size_t ssm = pk_lap_smem_bytes(n);
     if (n > 128 && ssm <= PK_LAP_SMEM_MAX) {
         int dev = 0, sms = 0, per_sm = 0;
-        err = cudaFuncSetAttribute(pk_diversity_staged_kernel<CPL, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)ssm);
+        err = pk_raise_smem((const void*)pk_diversity_staged_kernel<CPL, VEC>, ssm);
         if (err == cudaSuccess) err = cudaGetDevice(&dev);
         if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (err == cudaSuccess)

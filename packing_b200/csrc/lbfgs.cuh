@@ -491,7 +491,7 @@ static int pk_lbfgs_phase(int phase, const PkLbfgsState<F>& s, int n_iter, doubl
             const void* fn = phase == 0 ? (const void*)pk_lbfgs_init_kernel<F>
                            : phase == 1 ? (const void*)pk_lbfgs_direction_kernel<F>
                                         : (const void*)pk_lbfgs_update_kernel<F>;
-            err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            err = pk_raise_smem(fn, smem);
             if (err != cudaSuccess) return pk_cuda_check(err, "pk_lbfgs attribute");
             if (phase == 0) pk_lbfgs_init_kernel<F><<<s.M, T, smem, st>>>(s, (F)a);
             else if (phase == 1) pk_lbfgs_direction_kernel<F><<<s.M, T, smem, st>>>(s, n_iter, (F)a, (F)b_, i1, (F)c);
@@ -540,8 +540,7 @@ static int pk_lbfgs_iterate_launch(const PkLbfgsState<F>& s, int n_iter, const P
                                    cudaStream_t st)
 {
     const size_t smem = ((size_t)s.m + pk_canon_red_len(s.N, s.m)) * sizeof(F);
-    cudaError_t err = cudaFuncSetAttribute(pk_lbfgs_iterate_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem);
+    cudaError_t err = pk_raise_smem((const void*)pk_lbfgs_iterate_kernel<F>, smem);
     if (err != cudaSuccess) return pk_cuda_check(err, "pk_lbfgs_iterate attribute");
     pk_lbfgs_iterate_kernel<F><<<s.M, pk_lbfgs_threads(s.N), smem, st>>>(s, n_iter, prm);
     const size_t total = (size_t)s.M * s.N, want = (total + 255) / 256;

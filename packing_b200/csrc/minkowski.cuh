@@ -328,7 +328,7 @@ extern "C" int pk_lut_build_exact_sep(const float* X, int nx, const float* Y, in
     err = cudaMemsetAsync(overflow, 0, sizeof(int), st);
     const size_t smem = pk_mk_grid_smem();
     if (err == cudaSuccess)
-        err = cudaFuncSetAttribute(pk_mk_grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        err = pk_raise_smem((const void*)pk_mk_grid_kernel, smem);
     const long long tiles = (long long)((nx + PK_MK_TILE - 1) / PK_MK_TILE) * ((ny + PK_MK_TILE - 1) / PK_MK_TILE);
     const int per_slice = (int)(tiles < 64 ? tiles : 64);   // 256 slices x 64 CTAs fill the GPU many times over
     for (int t0 = 0; t0 < nt && err == cudaSuccess; t0 += batch) {

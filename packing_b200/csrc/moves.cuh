@@ -764,7 +764,7 @@ extern "C" int pk_moves(float* xyt, const float* h, int E, int n, const int* ind
         return pk_fail(PK_EINVAL, "pk_moves: NULL pointer%s");
     cudaStream_t st = (cudaStream_t)stream;
     const size_t smem = pk_moves_smem(n);
-    cudaError_t err = cudaFuncSetAttribute(pk_moves_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t err = pk_raise_smem((const void*)pk_moves_kernel, smem);
     if (err != cudaSuccess) return pk_cuda_check(err, "pk_moves attribute");
     pk_moves_kernel<<<C, PK_MV_THREADS, smem, st>>>(xyt, h, E, n, inds_to_do, C, mate_xyt, mate_h, M, inds_mate, *set,
                                                     (uint32_t)seed, (uint32_t)(seed >> 32), (uint32_t)call,

@@ -319,10 +319,10 @@ extern "C" int pk_validate_fp64(const void* xyt, int dtype_bytes, int E, int n, 
     cudaStream_t st = (cudaStream_t)stream;
     cudaError_t err;
     if (dtype_bytes == 4) {
-        err = cudaFuncSetAttribute(pk_validate_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        err = pk_raise_smem((const void*)pk_validate_kernel<float>, smem);
         if (err == cudaSuccess) pk_validate_kernel<float><<<E, T, smem, st>>>((const float*)xyt, E, n, overlaps, side);
     } else if (dtype_bytes == 8) {
-        err = cudaFuncSetAttribute(pk_validate_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        err = pk_raise_smem((const void*)pk_validate_kernel<double>, smem);
         if (err == cudaSuccess)
             pk_validate_kernel<double><<<E, T, smem, st>>>((const double*)xyt, E, n, overlaps, side);
     } else {
