@@ -93,7 +93,7 @@ __device__ __forceinline__ bool pk_hungarian_warp(int N, RowFn rowfn, int (&cm)[
     }
     if (PREFETCH) rowfn(0, c);
     for (int i = 0; i < N; ++i) {
-        unsigned used = invalid;
+        unsigned used = invalid, closed = invalid;   // in the tree; not to be chosen
         float ui = 0.f, urow = 0.f;
         int cur_row = i, cur_col = -1;
 #pragma unroll
@@ -106,7 +106,7 @@ __device__ __forceinline__ bool pk_hungarian_warp(int N, RowFn rowfn, int (&cm)[
             unsigned ss[CPL];   // column << 16 | row matched to it (0xffff: none)
 #pragma unroll
             for (int k = 0; k < CPL; ++k) {
-                const bool open = !((used >> k) & 1u);
+                const bool open = !((closed >> k) & 1u);
                 const float red = (c[k] - urow) - v[k];
                 const bool better = open && red < minv[k];
                 minv[k] = better ? red : minv[k];
@@ -124,7 +124,8 @@ __device__ __forceinline__ bool pk_hungarian_warp(int N, RowFn rowfn, int (&cm)[
                     su[k] = right ? su[k + o] : su[k];
                     ss[k] = right ? ss[k + o] : ss[k];
                 }
-            // slacks are never NaN: a NaN cost fails the '<' above and leaves minv untouched
+            // open slacks are never NaN: a NaN cost fails the '<' above and leaves minv
+            // untouched, and what becomes NaN below is closed
             const float delta = pk_redux_min(sl[0]);
             if (!(delta < 1e30f)) return false;   // no finite slack: infeasible input
             const unsigned sel = __reduce_min_sync(PK_FULL_MASK, sl[0] == delta ? ss[0] : 0xffffffffu);
@@ -146,7 +147,13 @@ __device__ __forceinline__ bool pk_hungarian_warp(int N, RowFn rowfn, int (&cm)[
             }
             ui += delta;
             if (free_col) break;
-            used |= lane == owner ? 1u << pk_lap_slot<VEC>(cur_col) : 0u;
+            const unsigned taken = lane == owner ? 1u << pk_lap_slot<VEC>(cur_col) : 0u;
+            used |= taken;
+            closed |= taken;
+            if (delta == -INFINITY) {   // of several -inf slacks the others are NaN now: no '<' finds them
+#pragma unroll
+                for (int k = 0; k < CPL; ++k) closed |= minv[k] != minv[k] ? 1u << k : 0u;
+            }
         }
         // flip the alternating path (lap_batch.py:157-163): every column on it
         // takes the row (and that row's dual) of its parent column, the first

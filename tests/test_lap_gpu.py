@@ -274,3 +274,24 @@ def test_diversity_forms_agree(cuda, Np, Nr, n, transform):
         assert torch.equal(torch.isnan(got), torch.isnan(want))
         assert torch.equal(got.nan_to_num(-1.0), want.nan_to_num(-1.0))
     assert bool(torch.isnan(D[1]).all()) == (Np > 2) if Np > 1 else True
+
+
+@pytest.mark.parametrize("N,second,best", [(33, 1, 32), (64, 1, 33), (97, 1, 33), (100, 2, 3), (128, 2, 3), (160, 2, 3),
+                                           (256, 2, 128)])
+@pytest.mark.parametrize("B", [2, 1200])
+def test_several_infinite_slacks_bitexact(cuda, B, N, second, best):
+    """Two costs of -inf in one row: when the first is taken the other's slack is
+    NaN, which hides no other column of its lane (best shares one with it, or with
+    column 0).  Staged (2 problems) and from L2 (1200)."""
+    rng = np.random.default_rng(N)
+    C = rng.uniform(1.0, 2.0, (B, N, N)).astype(np.float32)
+    C[:, 0, 0] = 0.0
+    C[:, 0, best] = 0.5
+    C[:, 1, [0, second]] = -np.inf
+    rm, tot = _solve(C, cuda)
+    orm, otot = O.hungarian(C[:2])
+    assert (orm[:, 0] == best).all() and (orm[:, 1] == 0).all()
+    assert np.array_equal(rm[:2], orm) and np.array_equal(tot[:2], otot)
+    if B > 2:
+        orm, otot = O.hungarian(C)
+        assert np.array_equal(rm, orm) and np.array_equal(tot, otot)
