@@ -57,8 +57,8 @@ __device__ __forceinline__ void pk_block_max4d(double (&v)[4], double* red)
 // The same test in FP32 on coordinates about one tree's centre, decided only
 // where rounding cannot matter: -1 if some edge normal separates the pieces by
 // more than margin, 1 if every normal has them overlap by more than margin, 0
-// if FP64 has to say.  (The normals are not unit vectors but shorter than 1, so
-// the margin in distance is larger still.)
+// if FP64 has to say.  (The margin is in the units of the projections: the normals
+// are as long as their edges.)
 __device__ __forceinline__ int pk_pieces_overlap32(const float2 (&P)[4], bool pt, const float2 (&Q)[4], bool qt,
                                                    float margin)
 {
@@ -162,10 +162,16 @@ pk_validate_kernel(const T* __restrict__ xyt, int E, int n, int* __restrict__ ov
         }
     }
     pk_block_max4d(bb, red);
-    // FP32 rounding of centres and boxes is below 1e-6 of the extent
+    // FP32 rounding of centres and boxes is below 1e-6 of the extent and of the
+    // tree's radius R.  Along an edge normal (not a unit vector: as long as the
+    // edge) it is below 1.3e-5 R^2: vertices of at most 3 R with 11 roundings,
+    // normals of at most 2 R with 24, the products' own, and both pieces' sum.
+    // Trees so large that FP32 products leave its range: FP64 decides everything.
     const double ext = fmax(fmax(fabs(bb[0]), fabs(bb[1])), fmax(fabs(bb[2]), fabs(bb[3])));
-    const float margin = (float)(1e-5 + 1e-6 * ext);
-    const float reach = 2.0f * (float)c_geom64.legal_radius + 2.0f * margin;
+    const double R = c_geom64.legal_radius;
+    const float margin = R <= 1e12 ? (float)(1e-5 * fmax(1.0, R) + 1e-6 * ext) : __int_as_float(0x7f800000);
+    const float margin_side = fmaxf(margin, (float)(2e-5 * R * R));
+    const float reach = 2.0f * (float)R + 2.0f * margin;
     const float reach2 = reach * reach;
     const int half = n >> 1;
     for (int t = threadIdx.x; t < n + half; t += blockDim.x) {
@@ -268,7 +274,7 @@ pk_validate_kernel(const T* __restrict__ xyt, int E, int n, int* __restrict__ ov
                     P[k2] = make_float2(ac * l.x - as * l.y, as * l.x + ac * l.y);
                     Q[k2] = make_float2(bc * m.x - bs * m.y + fx, bs * m.x + bc * m.y + fy);
                 }
-                const int r = pk_pieces_overlap32(P, c_geom64.piece_nv[p] == 3, Q, c_geom64.piece_nv[q] == 3, margin);
+                const int r = pk_pieces_overlap32(P, c_geom64.piece_nv[p] == 3, Q, c_geom64.piece_nv[q] == 3, margin_side);
                 if (r > 0) {
                     if (!(atomicOr(&near[wn], 0x80000000u) >> 31)) atomicAdd(&cnt[2], 1);
                 } else if (r == 0) {

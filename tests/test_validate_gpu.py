@@ -99,3 +99,71 @@ def test_list_edges_match_oracle(cuda, n, kind):
                                                 2))[0] for k in range(n // 3))
         assert np.array_equal(ov, oov)
         np.testing.assert_allclose(side, oside, rtol=1e-12)
+
+
+def _scaled_geometry(S):
+    from packing_b200 import _lib
+    g = _lib.default_geometry()
+    for name in ("piece_xy", "legal_piece_xy"):
+        for p in getattr(g, name):
+            for v in p:
+                v[0], v[1] = v[0] * S, v[1] * S
+    for name in ("tree_xy", "legal_tree_xy"):
+        for v in getattr(g, name):
+            v[0], v[1] = v[0] * S, v[1] * S
+    g.max_radius *= S
+    g.area *= S * S
+    return g
+
+
+def _interiors_meet(x):
+    """Separating-axis test in float64 on the legality pieces, of pairs x (E, 2, 3)."""
+    from packing_b200 import _lib
+    g = _lib.default_geometry()
+    c, s = np.cos(x[:, :, 2])[..., None], np.sin(x[:, :, 2])[..., None]
+    pieces = [np.array([[v[0], v[1]] for v in g.legal_piece_xy[p]][:g.piece_nv[p]]) for p in range(4)]
+    V = [np.stack([c * l[:, 0] - s * l[:, 1] + x[:, :, :1], s * l[:, 0] + c * l[:, 1] + x[:, :, 1:2]], -1) for l in pieces]
+    meet = np.zeros(len(x), bool)
+    for p in range(4):
+        for q in range(4):
+            P, Q = V[p][:, 0], V[q][:, 1]   # (E, vertices, 2)
+            apart = np.zeros(len(x), bool)
+            for W in (P, Q):
+                e = np.roll(W, -1, 1) - W
+                n = np.stack([-e[..., 1], e[..., 0]], -1)
+                a, b = P @ n.transpose(0, 2, 1), Q @ n.transpose(0, 2, 1)
+                apart |= ((a.max(1) <= b.min(1)) | (b.max(1) <= a.min(1))).any(1)
+            meet |= ~apart
+    return meet
+
+
+@pytest.mark.parametrize("S", [1.0, 2.0 ** 10, 2.0 ** 45, 2.0 ** -10])
+def test_decisions_scale_with_the_tree(cuda, S):
+    """Pairs 1e-8 to 1e-6 from contact, with a geometry of any size: powers of two
+    scale the FP64 test exactly, so the answers are those at scale 1."""
+    from packing_b200 import _lib
+    rng = np.random.default_rng(21)
+    E = 600
+    x = np.zeros((E, 2, 3))
+    x[:, :, 2] = rng.uniform(0, 2 * np.pi, (E, 2))
+    phi = rng.uniform(0, 2 * np.pi, E)
+    d = np.stack([np.cos(phi), np.sin(phi)], 1)
+    lo, hi = np.zeros(E), np.full(E, 1.3)
+    for _ in range(60):
+        mid = 0.5 * (lo + hi)
+        x[:, 1, :2] = mid[:, None] * d
+        hit = _interiors_meet(x)
+        lo, hi = np.where(hit, mid, lo), np.where(hit, hi, mid)
+    try:
+        _lib.ensure_init(cuda, _scaled_geometry(S))
+        for delta in (1e-8, -1e-8, 1e-7, -1e-7, 1e-6, -1e-6):
+            x[:, 1, :2] = (hi + delta)[:, None] * d
+            want = _interiors_meet(x)
+            assert want.mean() < 0.1 if delta > 0 else want.mean() > 0.9
+            y = x.copy()
+            y[:, :, :2] *= S
+            ov, side = _val(y, cuda)
+            assert np.array_equal(ov, want), (delta, int((ov != want).sum()))
+            np.testing.assert_allclose(side, O.validate(x)[1] * S, rtol=1e-14)
+    finally:
+        _lib.ensure_init(cuda, _lib.default_geometry())
