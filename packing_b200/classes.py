@@ -68,11 +68,11 @@ def ragged_plan(sizes, device=None):
     """(order, classes) for a ragged batch with these tree counts: the
     largest-first launch order as a device int32 tensor and its size
     classes (one class of all, with the library's choice of threads, for a
-    batch that leaves the GPU idle)."""
+    batch that leaves the GPU of that device idle)."""
     sz = np.array([int(s) for s in sizes], dtype=np.int64)
     order = torch.tensor(largest_first(sz), dtype=torch.int32, device=device or "cuda")
     classes = size_classes(-np.sort(-sz))   # refuses a tree count beyond the table
-    if len(sz) and not fills_gpu(len(sz), order.device):
+    if len(sz) and order.is_cuda and not fills_gpu(len(sz), order.device):
         classes = [SizeClass(0, len(sz), int(sz.max()), 0)]
     return order, classes
 

@@ -31,3 +31,14 @@ def test_class_edge_cases():
         size_classes([5, 200])
     with pytest.raises(ValueError):
         size_classes([2000])
+
+
+def test_ragged_plan_without_a_gpu():
+    """A plan made for the CPU has its order there and the table's classes."""
+    import torch
+    from packing_b200.classes import ragged_plan
+    order, classes = ragged_plan([5, 200, 7, 200, 5], device="cpu")
+    assert order.dtype == torch.int32 and order.tolist() == [1, 3, 2, 0, 4]
+    assert classes == size_classes([200, 200, 7, 5, 5])
+    order, classes = ragged_plan([], device="cpu")
+    assert order.numel() == 0 and classes == []
