@@ -179,6 +179,19 @@ def relax(xyt, h, spec: CostSpec = CostSpec(), params: RelaxParams = RelaxParams
     return xo, ho, loss, iters
 
 
+def _flat_poses(xyt_list):
+    """The packings' poses (sum n, 3) in float32 and the tree counts: each
+    element converted from its own type."""
+    shapes = [a.shape for a in xyt_list]
+    sizes = [s[0] for s in shapes]
+    if all(len(s) == 2 and s[1] == 3 for s in shapes):
+        flat = torch.cat(xyt_list)
+        # what the list's types are promoted to holds them exactly, or is float32 itself
+        if flat.dtype == torch.float32 or all(a.dtype == flat.dtype for a in xyt_list):
+            return flat.to(torch.float32), sizes
+    return torch.cat([a.reshape(-1, 3).to(torch.float32) for a in xyt_list]).contiguous(), sizes
+
+
 def relax_ragged(xyt_list, h, spec: CostSpec = CostSpec(), params: RelaxParams = RelaxParams(), stream=None):
     """Relax packings of different tree counts together, largest first:
     one launch per size class (``size_classes``), side by side on forked
@@ -189,13 +202,9 @@ def relax_ragged(xyt_list, h, spec: CostSpec = CostSpec(), params: RelaxParams =
     E = len(xyt_list)
     if E == 0:
         return [], None, None, None
-    sizes = [a.shape[0] for a in xyt_list]
     dev = xyt_list[0].device
     _lib.ensure_init(dev)
-    if all(a.dim() == 2 for a in xyt_list):
-        flat = torch.cat(xyt_list).to(torch.float32)
-    else:
-        flat = torch.cat([a.reshape(-1, 3).to(torch.float32) for a in xyt_list]).contiguous()
+    flat, sizes = _flat_poses(xyt_list)
     sz = np.array(sizes, dtype=np.int64)
     order_h = largest_first(sz)
     # one copy to the device: the offsets, then the launch order

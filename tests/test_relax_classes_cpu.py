@@ -42,3 +42,26 @@ def test_ragged_plan_without_a_gpu():
     assert classes == size_classes([200, 200, 7, 5, 5])
     order, classes = ragged_plan([], device="cpu")
     assert order.numel() == 0 and classes == []
+
+
+@pytest.mark.parametrize("types", [("float32",), ("float64",), ("float16",), ("int64",), ("float64", "float32"),
+                                   ("int64", "float16"), ("float16", "bfloat16"), ("int64", "float32"),
+                                   ("int64", "float64")])
+def test_poses_are_converted_one_by_one(types):
+    """A list of several types is not promoted to a common one on the way to
+    float32 (int64 beside float16 would pass through float16); shapes other than
+    (n, 3) are read as rows of three, as ever."""
+    import torch
+    from packing_b200.relax import _flat_poses
+    rng = np.random.default_rng(2)
+    xs = [torch.from_numpy(rng.uniform(-3000, 3000, (n, 3))).to(getattr(torch, types[k % len(types)]))
+          for k, n in enumerate([4, 1, 7, 0, 2])]
+    xs[0][0, 0] = 2049     # not a float16
+    if types[0] == "int64":
+        xs[0][1, 1] = 2 ** 61 + 2 ** 37 + 1   # halfway between two float32 but for its last bit, which float64 drops
+    want = torch.cat([a.reshape(-1, 3).to(torch.float32) for a in xs])
+    flat, sizes = _flat_poses(xs)
+    assert flat.dtype == torch.float32 and flat.is_contiguous() and torch.equal(flat, want)
+    assert sizes == [4, 1, 7, 0, 2]
+    flat, sizes = _flat_poses(xs + [xs[0][:1].reshape(3)])   # one tree as a vector: rows of three
+    assert torch.equal(flat, torch.cat([want, want[:1]]))
