@@ -192,6 +192,13 @@ def _flat_poses(xyt_list):
     return torch.cat([a.reshape(-1, 3).to(torch.float32) for a in xyt_list]).contiguous(), sizes
 
 
+def _split_poses(flat, sizes):
+    """The packings' rows of flat, each a tensor of its own that may be changed in
+    place (the views of torch.split refuse that under autograd; half the time of
+    slicing)."""
+    return list(torch.unsafe_split_with_sizes(flat, sizes))
+
+
 def relax_ragged(xyt_list, h, spec: CostSpec = CostSpec(), params: RelaxParams = RelaxParams(), stream=None):
     """Relax packings of different tree counts together, largest first:
     one launch per size class (``size_classes``), side by side on forked
@@ -220,4 +227,4 @@ def relax_ragged(xyt_list, h, spec: CostSpec = CostSpec(), params: RelaxParams =
     classes = size_classes(sz[order_h]) if params.threads == 0 and fills_gpu(E, dev) else None
     relax_into(flat, hh, xo, ho, loss, work, spec, params, offsets=offsets, order=order, n_max=int(sz.max()),
                iters_out=iters, stream=stream, classes=classes)
-    return list(torch.split(xo, sizes)), ho, loss, iters
+    return _split_poses(xo, sizes), ho, loss, iters

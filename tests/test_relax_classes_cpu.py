@@ -65,3 +65,21 @@ def test_poses_are_converted_one_by_one(types):
     assert sizes == [4, 1, 7, 0, 2]
     flat, sizes = _flat_poses(xs + [xs[0][:1].reshape(3)])   # one tree as a vector: rows of three
     assert torch.equal(flat, torch.cat([want, want[:1]]))
+
+
+def test_relaxed_poses_may_be_changed_in_place():
+    """The results of a ragged relaxation are written over by callers, also with
+    tensors that need gradients, and share one buffer."""
+    import torch
+    from packing_b200.relax import _split_poses
+    flat = torch.arange(18, dtype=torch.float32).reshape(6, 3)
+    outs = _split_poses(flat, [2, 0, 4])
+    assert [tuple(o.shape) for o in outs] == [(2, 3), (0, 3), (4, 3)]
+    assert all(torch.equal(o, f) for o, f in zip(outs, (flat[:2], flat[2:2], flat[2:])))
+    w = torch.full((2, 3), 2.0, requires_grad=True)
+    outs[0].mul_(w)
+    outs[0].sum().backward()
+    assert torch.equal(w.grad, torch.arange(6, dtype=torch.float32).reshape(2, 3))
+    outs[2].zero_()
+    assert float(flat[2:].abs().sum()) == 0.0 and float(flat[1, 2]) == 10.0
+    outs[2].requires_grad_()
