@@ -189,7 +189,10 @@ def _flat_poses(xyt_list):
         # what the list's types are promoted to holds them exactly, or is float32 itself
         if flat.dtype == torch.float32 or all(a.dtype == flat.dtype for a in xyt_list):
             return flat.to(torch.float32), sizes
-    return torch.cat([a.reshape(-1, 3).to(torch.float32) for a in xyt_list]).contiguous(), sizes
+    flat = torch.cat([a.reshape(-1, 3).to(torch.float32) for a in xyt_list]).contiguous()
+    if flat.shape[0] < sum(sizes):   # the launch would read beyond them
+        raise ValueError(f"packings must be (n, 3), got {[tuple(s) for s in shapes if len(s) != 2 or s[1] != 3][0]}")
+    return flat, sizes
 
 
 def _split_poses(flat, sizes):

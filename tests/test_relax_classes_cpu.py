@@ -49,8 +49,8 @@ def test_ragged_plan_without_a_gpu():
                                    ("int64", "float64")])
 def test_poses_are_converted_one_by_one(types):
     """A list of several types is not promoted to a common one on the way to
-    float32 (int64 beside float16 would pass through float16); shapes other than
-    (n, 3) are read as rows of three, as ever."""
+    float32 (int64 beside float16 would pass through float16); a shape other than
+    (n, 3) is read as rows of three, as ever."""
     import torch
     from packing_b200.relax import _flat_poses
     rng = np.random.default_rng(2)
@@ -63,8 +63,8 @@ def test_poses_are_converted_one_by_one(types):
     flat, sizes = _flat_poses(xs)
     assert flat.dtype == torch.float32 and flat.is_contiguous() and torch.equal(flat, want)
     assert sizes == [4, 1, 7, 0, 2]
-    flat, sizes = _flat_poses(xs + [xs[0][:1].reshape(3)])   # one tree as a vector: rows of three
-    assert torch.equal(flat, torch.cat([want, want[:1]]))
+    flat, sizes = _flat_poses(xs + [xs[0][:1].reshape(1, 1, 3)])
+    assert torch.equal(flat, torch.cat([want, want[:1]])) and sizes == [4, 1, 7, 0, 2, 1]
 
 
 def test_relaxed_poses_may_be_changed_in_place():
@@ -83,3 +83,13 @@ def test_relaxed_poses_may_be_changed_in_place():
     outs[2].zero_()
     assert float(flat[2:].abs().sum()) == 0.0 and float(flat[1, 2]) == 10.0
     outs[2].requires_grad_()
+
+
+@pytest.mark.parametrize("shape", [(3, 2), (3,), (4, 1), (6, 1, 1)])
+def test_poses_with_fewer_rows_than_trees_are_refused(shape):
+    """What has fewer rows of three than its first dimension says would be read
+    out of range on the device."""
+    import torch
+    from packing_b200.relax import _flat_poses
+    with pytest.raises((ValueError, RuntimeError)):
+        _flat_poses([torch.zeros(5, 3), torch.zeros(shape)])
