@@ -20,9 +20,12 @@ static int pk_fail(int code, const char* fmt, const char* detail = "")
     return code;
 }
 
+// The error reported here is taken off the host thread's record: the next call's
+// launch check would report it again as its own.
 static int pk_cuda_check(cudaError_t e, const char* where)
 {
     if (e == cudaSuccess) return PK_OK;
+    (void)cudaGetLastError();
     snprintf(g_pk_err, sizeof(g_pk_err), "%s: %s", where, cudaGetErrorString(e));
     return PK_ECUDA;
 }

@@ -32,3 +32,14 @@ def test_lbfgs_at_227_kb(cuda, dt, N, m):
     x = torch.ones(1, N, device=cuda, dtype=dt)
     lbfgs(_quadratic(cuda, dt, N), x, max_iter=12, history_size=m, max_step=None)
     assert float(x.abs().max()) < 0.1
+
+
+def test_a_refused_size_does_not_fail_the_next_call(cuda):
+    from packing_b200 import _lib
+    from packing_b200.cost import compound_cost
+    from packing_b200.lbfgs_torch_parallel import lbfgs
+    x = torch.ones(1, 70000, device=cuda)
+    with pytest.raises(_lib.PackError):   # more shared memory than a CTA can have
+        lbfgs(_quadratic(cuda, torch.float32, 70000), x, max_iter=2, history_size=3)
+    cost, _, _ = compound_cost(torch.zeros(1, 1, 3, device=cuda), torch.ones(1, 3, device=cuda) * 4)
+    assert torch.isfinite(cost).all()
