@@ -69,51 +69,6 @@ __device__ __forceinline__ T pk_warp_sum(T v)
     return v;
 }
 
-// Deterministic block-wide sum: fixed warp-shuffle tree, then warp 0 sums the
-// per-warp partials in warp order.  scratch needs blockDim.x/32 entries.
-// Every thread gets the result.
-template <typename T>
-__device__ __forceinline__ T pk_block_sum(T v, T* scratch)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nw = (blockDim.x + 31) >> 5;
-    v = pk_warp_sum(v);
-    __syncthreads();
-    if (lane == 0) scratch[warp] = v;
-    __syncthreads();
-    T r = (lane < nw) ? scratch[lane] : T(0);
-    if (warp == 0) {
-        r = pk_warp_sum(r);
-        if (lane == 0) scratch[0] = r;
-    }
-    __syncthreads();
-    r = scratch[0];
-    __syncthreads();
-    return r;
-}
-
-template <typename T>
-__device__ __forceinline__ T pk_block_max(T v, T* scratch)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(PK_FULL_MASK, v, o));
-    __syncthreads();
-    if (lane == 0) scratch[warp] = v;
-    __syncthreads();
-    T r = (lane < nw) ? scratch[lane] : scratch[0];
-    if (warp == 0) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) r = max(r, __shfl_xor_sync(PK_FULL_MASK, r, o));
-        if (lane == 0) scratch[0] = r;
-    }
-    __syncthreads();
-    r = scratch[0];
-    __syncthreads();
-    return r;
-}
-
 // Block-wide maximum of four floats at once (one round trip through
 // shared memory); scratch needs 4 * warps floats.  All threads get the result.
 __device__ __forceinline__ float4 pk_block_max4(float4 v, float* scratch)

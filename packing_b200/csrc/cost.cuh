@@ -55,11 +55,11 @@ __host__ __device__ inline int pk_grid_cap(int n_max) { return n_max < 32 ? 64 :
 
 // List capacities.  The near list takes 8 T pairs (2048 at most: an item names
 // its pair by an 11-bit index), at least the n_max - 1 pairs of one tree for
-// every n_max that pk_cost_threads gives T for; an expansion chunk appends at
-// most 16 T piece pairs to the item list, which is flushed before the next
-// chunk could overflow it: above 20 T items, so that the about 7 T of a packing
-// of n = T trees are evaluated in one go (the LUT's items are the near pairs
-// themselves).
+// every n_max that pk_cost_threads gives T for.  Each warp reserves room in the
+// item list for the piece pairs of 32 near pairs at a time, at most 512, and the
+// list is evaluated when a warp finds none: 36 T items hold the about 7 T of a
+// packing of n = T trees several times over, so they are evaluated in one go
+// (the LUT's items are the near pairs themselves).
 __host__ __device__ inline void pk_caps(int T, int mode, int* cap_near, int* cap_items)
 {
     *cap_near = 8 * T;
@@ -793,10 +793,6 @@ __device__ __forceinline__ long long pk_flush_near(const PkCostSmem& sm, int cn,
                     keep = !filter || pk_is_near(A, B, c_geom.cutoff_sq);
                     if (keep) {
                         const float dx = B.x - A.x, dy = B.y - A.y;
-                        float4 bq[4];
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                        }
 #pragma unroll
                         for (int p = 0; p < 4; ++p) {
                             const float4 a = sm.aabb[p * sm.n_cap + i];

@@ -528,11 +528,15 @@ pk_diversity_staged_kernel(const float* __restrict__ pop, const float* __restric
     pk_diversity_problem<CPL, VEC, false>(pop, ref, Nr, n, ntf, blockIdx.x, Cs, Cs + ((n * n + 3) & ~3), out);
 }
 
-// The matrix in the warp's own slab of a caller's scratch (slab floats apart),
-// which stays in L2: many more problems in flight than shared memory holds.
-// Warps take problems from a counter, so unequal problems even out.  128 x 8
-// pairs of 100 trees: 2.11 ms with rows generated in the steps, 2.29 staged in
-// shared memory, 1.43 from the scratch (16 warps per SM; 8: 1.86, 24: 1.42).
+// The matrix in the warp's own slab of a caller's scratch (slab floats apart):
+// many more problems in flight than shared memory holds.  Up to 115 trees all
+// slabs stay in L2; beyond, part of the rows come from HBM.  Warps take problems
+// from a counter, so unequal problems even out.  128 x 8 pairs of 100 trees: 2.11
+// ms with rows generated in the steps, 2.29 staged in shared memory, 1.43 from the
+// scratch (16 warps per SM; 8: 1.86, 24: 1.42).  Out of L2 it is still the faster
+// form, rows against scratch: 128 trees 3.30 / 2.48 ms, 200 (379 MB) 12.6 / 8.3,
+// 256 (621 MB) 23.4 / 12.2, and 8 warps per SM instead of 16 are slower (200
+// trees, 64 x 8 pairs: 6.4 ms against 4.6).
 template <int CPL, bool VEC>
 __global__ void __launch_bounds__(32 * PK_LAP_WARPS, 1)
 pk_diversity_work_kernel(const float* __restrict__ pop, const float* __restrict__ ref, int Nr, int n, int ntf,
@@ -623,8 +627,9 @@ extern "C" int pk_diversity_matrix(const float* pop, const float* ref, int Np, i
 
 // Scratch of pk_diversity_matrix_work: a header for the problem counter and one
 // matrix slab per warp.  As many warps per SM, between 16 and 32, as keep the
-// slabs within the 126 MB L2 (n <= 78: 32; 96: 20; from 108: 16), and no more
-// than there are problems.
+// slabs within the 126 MB L2 (n <= 81: 32; 82: 28; 96 to 103: 20; from 104: 16),
+// and no more than there are problems.  From 116 trees the 16 no longer fit: with
+// 148 SMs 155 MB at 128 trees, 379 at 200, 621 at 256.
 #define PK_DIV_HEADER 32   // floats; keeps the slabs 128-byte aligned
 static size_t pk_div_slab(int n) { return ((size_t)n * n + 31) & ~(size_t)31; }
 

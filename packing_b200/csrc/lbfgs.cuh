@@ -264,7 +264,9 @@ __global__ void pk_lbfgs_direction_kernel(PkLbfgsState<F> s, int n_iter, F lr, F
 }
 
 // Phase 2 (:631): x += t d for every system (inactive ones too, as the
-// reference does while any system is active).
+// reference does while any system is active).  For callers of the C interface that
+// run the loop phase by phase; lbfgs itself steps in pk_lbfgs_step_if_kernel or
+// in the line search.
 template <typename F>
 __global__ void pk_lbfgs_step_kernel(F* x, const F* d, const F* t, int M, int N)
 {
@@ -773,9 +775,10 @@ __device__ void pk_relax_instance(int e, const float* __restrict__ xyt_in, const
 // loads even.  Instances are indexed 0 .. E-1 whatever part of the order a
 // launch covers.
 // WIDE: for a batch of at most 512 threads per SM, whose time is that of its
-// slowest CTA: 128 registers instead of 80, so nothing spills (48 x 200 legalisation
-// iterations 25 -> 21 us each, 8 x 50 trees 10 % less; 4096 x 200, where the
-// third CTA per SM is worth as much, 1 % more).
+// slowest CTA: 128 registers instead of 80, so next to nothing spills (area 20
+// bytes of stores instead of 226, the symmetric builds 4 to 20, the others none;
+// 48 x 200 legalisation iterations 25 -> 21 us each, 8 x 50 trees 10 % less; 4096
+// x 200, where the third CTA per SM is worth as much, 1 % more).
 template <int MODE, bool PERSISTENT, bool SYM, bool WIDE = false>
 __global__ void __launch_bounds__(256, WIDE ? 2 : 3) pk_relax_kernel(const float* __restrict__ xyt_in, const float* __restrict__ h_in,
                                 const int* __restrict__ offsets, const int* __restrict__ order, int count, int E,
