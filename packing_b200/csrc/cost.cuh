@@ -1408,10 +1408,11 @@ __device__ double pk_eval_instance(const float* X, int ng, const float* H, const
 
 // The size classes of an order that one launch covers: position b of the order
 // belongs to the first class whose end lies beyond it (all ends 0: no classes).
-// A build of its own reads them (CLASSES; 2000 packings of 5 to 200 trees, LUT:
-// 39 -> 42 us): read by every launch they cost the six forked ones of a large
-// batch 18 of 111 us, whose parameters together then no longer fit the SM's
-// constant cache.
+// A parameter of a build of its own (Bounds): read by every launch they cost the
+// six forked ones of a large batch 18 of 111 us, whose parameters together then no
+// longer fit the SM's constant cache, and unread they cost a 64 x 20 call 0.4 of 14
+// us.  Applied to the result: before the evaluation their registers made the LUT
+// build spill (2000 packings of 5 to 200 trees 38.5 -> 42 us).
 #define PK_MAX_BOUNDS 8
 struct PkClassBounds { unsigned c[PK_MAX_BOUNDS]; };   // end << 11 | n_max
 
@@ -1419,25 +1420,20 @@ struct PkClassBounds { unsigned c[PK_MAX_BOUNDS]; };   // end << 11 | n_max
 // mode has no clipper: it fits 64 registers without spilling, so four CTAs of
 // 256 threads share an SM and one CTA's broad phase overlaps the others'
 // gathers (4096 x n = 200: 0.201 -> 0.183 ms, the same bits).
-template <int MODE, bool SYM, bool CLASSES>
+template <int MODE, bool SYM, typename... Bounds>
 __global__ void __launch_bounds__(256, MODE == PK_PAIR_LUT ? 4 : 3) pk_cost_kernel(const float* __restrict__ xyt, const int* __restrict__ offsets,
                                const int* __restrict__ order, int E,
                                int n_max, const float* __restrict__ h, PkCostSpec spec,
                                float* __restrict__ cost, float* __restrict__ grad,
-                               float* __restrict__ grad_h, int cap_near, int cap_items, const PkClassBounds cls)
+                               float* __restrict__ grad_h, int cap_near, int cap_items, const Bounds... cls)
 {
     extern __shared__ __align__(16) unsigned char pk_smem[];
     const int e = order ? order[blockIdx.x] : blockIdx.x;
-    int most = n_max;
-    if (CLASSES)
-#pragma unroll
-        for (int c = PK_MAX_BOUNDS - 1; c >= 0; --c)
-            if (blockIdx.x < (cls.c[c] >> 11)) most = cls.c[c] & 2047;
 
     if (e < 0 || e >= E) return;
     const int base = offsets ? offsets[e] : e * n_max;
     const int n = offsets ? offsets[e + 1] - base : n_max;
-    if (n < 0 || n > most) {
+    if (n < 0 || n > n_max) {
         if (threadIdx.x == 0) cost[e] = __int_as_float(0x7fc00000);   // NaN marks a bad offset
         return;
     }
@@ -1447,7 +1443,17 @@ __global__ void __launch_bounds__(256, MODE == PK_PAIR_LUT ? 4 : 3) pk_cost_kern
     const double tot = pk_eval_instance<MODE, SYM>(xyt + (size_t)base * 3, n, h ? h + 3 * e : nullptr, spec,
                                               grad ? grad + (size_t)base * 3 : nullptr,
                                               grad_h ? grad_h + 3 * e : nullptr, sm);
-    if (threadIdx.x == 0) cost[e] = (float)tot;
+    if (threadIdx.x == 0) {
+        float c = (float)tot;
+        if constexpr (sizeof...(Bounds) == 1) {
+            int most = n_max;
+#pragma unroll
+            for (int k = PK_MAX_BOUNDS - 1; k >= 0; --k)
+                if (blockIdx.x < ((cls.c[k] >> 11), ...)) most = ((int)(cls.c[k] & 2047), ...);
+            if (n > most) c = __int_as_float(0x7fc00000);
+        }
+        cost[e] = c;
+    }
 }
 
 // Multiprocessors of the current device (0 on error), asked once per device.
@@ -1554,22 +1560,22 @@ static int pk_launch_cost(const float* xyt, const int* offsets, const int* order
     PkCostLaunch L;
     const int rc = pk_cost_args(xyt, order, count, E, n_max, h, spec, threads, cost, &L);
     if (rc || L.T == 0) return rc;
-    const PkClassBounds cls = classes ? *classes : PkClassBounds{};
     cudaError_t err = cudaSuccess;
     switch (spec->pair_mode) {
-#define PK_CASE2(M, S, C, SLOT)                                                                     \
+#define PK_CASE2(SLOT, KERNEL, ...)                                                                 \
     {                                                                                               \
-        err = pk_set_smem((const void*)pk_cost_kernel<M, S, C>, SLOT, L.smem);                      \
+        err = pk_set_smem((const void*)KERNEL, SLOT, L.smem);                                       \
         if (err == cudaSuccess)                                                                     \
-            pk_cost_kernel<M, S, C><<<count, L.T, L.smem, st>>>(xyt, offsets, order, E, n_max, h, *spec, cost, grad, \
-                                                                grad_h, L.cap_near, L.cap_items, cls); \
+            KERNEL<<<count, L.T, L.smem, st>>>(xyt, offsets, order, E, n_max, h, *spec, cost, grad, grad_h, L.cap_near, \
+                                               __VA_ARGS__);                                        \
     }
 #define PK_CASE(M)                                                                                  \
     case M:                                                                                         \
-        if (classes && spec->symmetry > 1) PK_CASE2(M, true, true, 44 + M)                          \
-        else if (classes) PK_CASE2(M, false, true, 40 + M)                                          \
-        else if (spec->symmetry > 1) PK_CASE2(M, true, false, 28 + M)                               \
-        else PK_CASE2(M, false, false, M)                                                           \
+        if (classes && spec->symmetry > 1)                                                          \
+            PK_CASE2(44 + M, (pk_cost_kernel<M, true, PkClassBounds>), L.cap_items, *classes)       \
+        else if (classes) PK_CASE2(40 + M, (pk_cost_kernel<M, false, PkClassBounds>), L.cap_items, *classes) \
+        else if (spec->symmetry > 1) PK_CASE2(28 + M, (pk_cost_kernel<M, true>), L.cap_items)       \
+        else PK_CASE2(M, (pk_cost_kernel<M, false>), L.cap_items)                                   \
         if (err == cudaSuccess) err = cudaGetLastError();                                           \
         break;
         PK_CASE(PK_PAIR_NONE)
