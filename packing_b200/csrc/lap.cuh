@@ -93,20 +93,20 @@ __device__ __forceinline__ bool pk_hungarian_warp(int N, RowFn rowfn, int (&cm)[
     }
     if (PREFETCH) rowfn(0, c);
     for (int i = 0; i < N; ++i) {
-        unsigned used = invalid, closed = invalid;   // in the tree; not to be chosen
+        unsigned used = invalid;
         float ui = 0.f, urow = 0.f;
         int cur_row = i, cur_col = -1;
 #pragma unroll
         for (int k = 0; k < CPL; ++k) { minv[k] = 1e30f; p[k] = -1; }
         for (;;) {   // each turn adds a column to the tree, so at most N turns
             if (!PREFETCH) rowfn(cur_row, c);
-            // the lane's smallest slack: selects, no branches, pairs before
-            // pairs of pairs; the left one keeps a tie
+            // the lane's smallest slack: no branches, pairs before pairs of pairs;
+            // the left one keeps a tie, and a NaN loses on either side
             float sl[CPL], su[CPL];
             unsigned ss[CPL];   // column << 16 | row matched to it (0xffff: none)
 #pragma unroll
             for (int k = 0; k < CPL; ++k) {
-                const bool open = !((closed >> k) & 1u);
+                const bool open = !((used >> k) & 1u);
                 const float red = (c[k] - urow) - v[k];
                 const bool better = open && red < minv[k];
                 minv[k] = better ? red : minv[k];
@@ -119,13 +119,14 @@ __device__ __forceinline__ bool pk_hungarian_warp(int N, RowFn rowfn, int (&cm)[
             for (int o = 1; o < CPL; o <<= 1)
 #pragma unroll
                 for (int k = 0; k + o < CPL; k += 2 * o) {
-                    const bool right = sl[k + o] < sl[k];
-                    sl[k] = right ? sl[k + o] : sl[k];
+                    const float m = fminf(sl[k], sl[k + o]);
+                    const bool right = m != sl[k];
+                    sl[k] = m;
                     su[k] = right ? su[k + o] : su[k];
                     ss[k] = right ? ss[k + o] : ss[k];
                 }
-            // open slacks are never NaN: a NaN cost fails the '<' above and leaves minv
-            // untouched, and what becomes NaN below is closed
+            // A NaN cost fails the '<' above and leaves minv untouched; a slack becomes
+            // NaN when another of -inf is taken before it, and nothing chooses it then.
             const float delta = pk_redux_min(sl[0]);
             if (!(delta < 1e30f)) return false;   // no finite slack: infeasible input
             const unsigned sel = __reduce_min_sync(PK_FULL_MASK, sl[0] == delta ? ss[0] : 0xffffffffu);
@@ -147,13 +148,7 @@ __device__ __forceinline__ bool pk_hungarian_warp(int N, RowFn rowfn, int (&cm)[
             }
             ui += delta;
             if (free_col) break;
-            const unsigned taken = lane == owner ? 1u << pk_lap_slot<VEC>(cur_col) : 0u;
-            used |= taken;
-            closed |= taken;
-            if (delta == -INFINITY) {   // of several -inf slacks the others are NaN now: no '<' finds them
-#pragma unroll
-                for (int k = 0; k < CPL; ++k) closed |= minv[k] != minv[k] ? 1u << k : 0u;
-            }
+            used |= lane == owner ? 1u << pk_lap_slot<VEC>(cur_col) : 0u;
         }
         // flip the alternating path (lap_batch.py:157-163): every column on it
         // takes the row (and that row's dual) of its parent column, the first
