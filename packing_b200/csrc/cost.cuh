@@ -1631,7 +1631,7 @@ extern "C" int pk_cost_classes(const float* xyt, const int* offsets, const int* 
     // packing the CTA of the largest one.  It is faster while the GPU takes the
     // batch in a few waves of such CTAs; by (E / resident CTAs), one launch
     // against forked, in us:
-    //   LUT, 5 to 200 trees:  3.4  38 / 52,  5.1  58 / 55;  5 to 900:  3.4  54 / 62,  6.8  95 / 75,  14  184 / 128
+    //   LUT, 5 to 200 trees:  3.4  40 / 52,  5.1  58 / 55;  5 to 900:  3.4  54 / 62,  6.8  95 / 75,  14  184 / 128
     //   area, 5 to 200: 1.1  30 / 43,  4.5  75 / 72;  5 to 900: 3.4  95 / 114,  6.8  155 / 138,  14  305 / 230
     //   separation, 5 to 200:  4.5  85 / 88;  2000 of 10 trees and one of 900, LUT:  14  80 / 58
     PkClassBounds bounds = {};
